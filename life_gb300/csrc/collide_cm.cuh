@@ -1,6 +1,8 @@
 // Central-moments collision in FP64 (De Rosis 2019), the reference's
 // CENTRAL_MOMENTS branch of GridClass::streamCollide.
 #pragma once
+#include <cstring>
+
 #include "lbm_device.cuh"
 
 namespace life {
@@ -8,7 +10,7 @@ namespace life {
 // Inverse central-moment transform (De Rosis 2019), term order as in the
 // reference (src/Grid.cpp:109-223); FP64 parity depends on that order.
 template <bool UNF>
-__device__ __forceinline__ void collide_cm(const double f[9], double rho, double ux, double uy, double Fx, double Fy,
+__host__ __device__ __forceinline__ void collide_cm(const double f[9], double rho, double ux, double uy, double Fx, double Fy,
                            double omega, double cs, double fs[9]) {
     // the two sums start at their first term rather than at +0 (see
     // moment_sums: equal up to the sign of a zero, which pos_zero restores)
@@ -145,6 +147,159 @@ __device__ __forceinline__ void collide_cm(const double f[9], double rho, double
         a = a + (0.25 * k8);
         fs[8] = a;
     }
+}
+
+// ---- one population of the central-moment collision ----------------------
+//
+// collide_cm's expressions with their power-of-two coefficients taken out:
+// scaling by a power of two commutes with round-to-nearest while nothing
+// leaves the normal range, so (0.25 a + 0.25 b) k is 0.25 ((a + b) k), and
+// every moment k enters as (poly) (scale k), the scaled moment formed once.
+// Without the factors each polynomial is at most four terms, and the terms
+// of all nine populations are the same few products with a sign, so ONE
+// instruction stream serves any population: a warp whose lanes hold the nine
+// populations of a site runs 20 FP64 instructions (36 with a force) where
+// the nine written-out polynomials take about 220 (320). The sums keep the
+// reference's order. cm_factored_ok() tells whether the values are in the
+// range where the scalings are exact; otherwise the written-out form runs.
+struct CmSite {
+    double ux, uy;              // velocity
+    double X2, Y2, XY, W;       // ux^2, uy^2, ux uy, 2 ux uy
+    double X2Y2, uxY2, X2uy;
+    double k0, k3, k4, k5, k8;  // moments after relaxation (k1, k2, k6, k7: force)
+    double k1, k2, k6, k7;
+};
+
+// x with its sign flipped when the integer c is negative / multiplied by 2^e
+// (the exponent field moved by e; x zero or well inside the normal range).
+__host__ __device__ __forceinline__ double bits_double(unsigned long long u) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)u);
+#else
+    double d;
+    std::memcpy(&d, &u, sizeof d);
+    return d;
+#endif
+}
+__host__ __device__ __forceinline__ double sgn_c(int c, double x) {
+    return bits_double(div_bits(x) ^ ((unsigned long long)((unsigned)c & 0x80000000u) << 32));
+}
+__host__ __device__ __forceinline__ double scale2(double x, int e) {
+    const unsigned long long u = div_bits(x);
+    return (u << 1) == 0ull ? x : bits_double(u + ((unsigned long long)(long long)e << 52));
+}
+
+// Zero, or a magnitude in [2^lo, 2^hi).
+__host__ __device__ __forceinline__ bool exp_within(double x, int lo, int hi) {
+    const unsigned long long u = div_bits(x);
+    const int e = (int)(u >> 52) & 0x7ff;
+    return (u << 1) == 0ull || (e >= 1023 + lo && e < 1023 + hi);
+}
+// With |u| in [2^-60, 2^60) or zero, every product of the polynomials is zero
+// or above 2^-240, every non-zero sum of two of their terms above 2^-350 (a
+// difference of two doubles is zero or at least an ulp of the smaller), and
+// with the moments in [2^-300, 2^300) or zero no scaled product leaves the
+// normal range.
+__host__ __device__ __forceinline__ bool cm_factored_ok(const CmSite& c) {
+    return exp_within(c.ux, -60, 60) && exp_within(c.uy, -60, 60) && exp_within(c.k0, -300, 300) &&
+           exp_within(c.k4, -300, 300) && exp_within(c.k5, -300, 300) && exp_within(c.k1, -300, 300) &&
+           exp_within(c.k2, -300, 300);
+}
+
+template <bool UNF>
+__host__ __device__ __forceinline__ void cm_site(CmSite& c, double rho, double ux, double uy, double Fx, double Fy,
+                                                 double k4Pre, double k5Pre, double omega, double cs) {
+    c.ux = ux;
+    c.uy = uy;
+    c.X2 = LSQ(ux);
+    c.Y2 = LSQ(uy);
+    c.XY = ux * uy;
+    c.W = scale2(c.XY, 1);
+    c.X2Y2 = c.X2 * c.Y2;
+    c.uxY2 = ux * c.Y2;
+    c.X2uy = c.X2 * uy;
+    c.k0 = rho;
+    c.k3 = 2.0 * rho * LSQ(cs);
+    c.k4 = (1.0 - omega) * k4Pre;
+    c.k5 = (1.0 - omega) * k5Pre;
+    c.k8 = rho * LQU(cs);
+    c.k1 = UNF ? 0.0 : 0.5 * Fx;
+    c.k2 = UNF ? 0.0 : 0.5 * Fy;
+    c.k6 = UNF ? 0.0 : 0.5 * Fy * LSQ(cs);
+    c.k7 = UNF ? 0.0 : 0.5 * Fx * LSQ(cs);
+}
+
+// Post-collision population v (components cx, cy) of site c. `forced`: the
+// force moments enter (they are exact zeros otherwise).
+__host__ __device__ __forceinline__ double cm_population(int cx, int cy, const CmSite& c, bool forced) {
+    const bool rest = cx == 0 && cy == 0, xax = cx != 0 && cy == 0, yax = cx == 0 && cy != 0;
+    const bool diag = cx != 0 && cy != 0, up = cy > 0, same = cx == cy;
+    const int cc = cx * cy;
+    const double one = 1.0;
+    // powers of two taken out of the coefficients of k0, k3, k4, k5, k8
+    const int s0 = rest ? 0 : (diag ? -2 : -1), s3 = rest ? -1 : (diag ? -3 : -2);
+    const int s5 = rest ? 2 : (diag ? -1 : 0);
+    double a0, b0, c0, d0;
+    if (rest) { a0 = c.X2Y2; b0 = -c.X2; c0 = -c.Y2; d0 = one; }
+    else if (xax) { a0 = c.X2; b0 = -c.X2Y2; c0 = sgn_c(-cx, c.uxY2); d0 = sgn_c(cx, c.ux); }
+    else if (yax) { a0 = up ? c.Y2 : c.X2uy; b0 = up ? -c.X2uy : -c.X2Y2; c0 = up ? -c.X2Y2 : c.Y2; d0 = sgn_c(cy, c.uy); }
+    else { a0 = c.X2Y2; b0 = sgn_c(cy, c.X2uy); c0 = sgn_c(cx, c.uxY2); d0 = sgn_c(cc, c.XY); }
+    double a3, b3, c3, d3;
+    if (rest) { a3 = c.X2; b3 = c.Y2; c3 = -2.0; d3 = 0.0; }
+    else if (xax) { a3 = -c.X2; b3 = sgn_c(-cx, c.ux); c3 = -c.Y2; d3 = one; }
+    else if (yax) { a3 = -c.X2; b3 = -c.Y2; c3 = sgn_c(-cy, c.uy); d3 = one; }
+    else { a3 = c.X2; b3 = sgn_c(cx, c.ux); c3 = c.Y2; d3 = sgn_c(cy, c.uy); }
+    double a4, b4, c4, d4;
+    if (rest) { a4 = c.Y2; b4 = -c.X2; c4 = 0.0; d4 = 0.0; }
+    else if (xax) { a4 = c.X2; b4 = sgn_c(cx, c.ux); c4 = -c.Y2; d4 = one; }
+    else if (yax) { a4 = c.X2; b4 = -c.Y2; c4 = sgn_c(-cy, c.uy); d4 = -one; }
+    else { a4 = -c.X2; b4 = sgn_c(-cx, c.ux); c4 = c.Y2; d4 = sgn_c(cy, c.uy); }
+    double a5, b5, c5, d5;
+    if (rest) { a5 = c.XY; b5 = 0.0; c5 = 0.0; d5 = 0.0; }
+    else if (xax) { a5 = sgn_c(-cx, c.uy); b5 = -c.W; c5 = 0.0; d5 = 0.0; }
+    else if (yax) { a5 = sgn_c(-cy, c.ux); b5 = -c.W; c5 = 0.0; d5 = 0.0; }
+    else if (same) { a5 = up ? c.ux : c.W; b5 = up ? c.uy : -c.uy; c5 = up ? c.W : -c.ux; d5 = 0.5; }
+    else { a5 = up ? c.ux : c.uy; b5 = up ? -c.uy : -c.ux; c5 = c.W; d5 = -0.5; }
+    double a = (((a0 + b0) + c0) + d0) * scale2(c.k0, s0);
+    if (forced) {
+        double a1, b1, c1, d1, a2, b2, c2, d2;
+        int s1, s2;
+        const double Z = scale2(c.uxY2, 1), V = scale2(c.X2uy, 1);
+        if (rest) { a1 = c.uxY2; b1 = -c.ux; c1 = 0.0; d1 = 0.0; s1 = 1; }
+        else if (xax) { a1 = scale2(c.ux, 1); b1 = -Z; c1 = sgn_c(-cx, c.Y2); d1 = sgn_c(cx, one); s1 = -1; }
+        else if (yax) { a1 = -c.uxY2; b1 = sgn_c(-cy, c.XY); c1 = 0.0; d1 = 0.0; s1 = 0; }
+        else {
+            a1 = same ? c.uy : (up ? c.W : Z);
+            b1 = same ? sgn_c(cc * cy, c.W) : (up ? -c.uy : -c.W);
+            c1 = same || up ? Z : -c.uy;
+            d1 = same ? sgn_c(cy, c.Y2) : (up ? -c.Y2 : c.Y2);
+            s1 = -2;
+        }
+        if (rest) { a2 = c.X2uy; b2 = -c.uy; c2 = 0.0; d2 = 0.0; s2 = 1; }
+        else if (xax) { a2 = -c.X2uy; b2 = sgn_c(-cx, c.XY); c2 = 0.0; d2 = 0.0; s2 = 0; }
+        else if (yax) { a2 = scale2(c.uy, 1); b2 = -V; c2 = sgn_c(-cy, c.X2); d2 = sgn_c(cy, one); s2 = -1; }
+        else {
+            a2 = same ? c.ux : (up ? V : c.W);
+            b2 = same ? sgn_c(cy, c.W) : (up ? -c.W : -c.ux);
+            c2 = same || !up ? V : -c.ux;
+            d2 = same ? sgn_c(cy, c.X2) : (up ? c.X2 : -c.X2);
+            s2 = -2;
+        }
+        a = a + (((a1 + b1) + c1) + d1) * scale2(c.k1, s1);
+        a = a + (((a2 + b2) + c2) + d2) * scale2(c.k2, s2);
+    }
+    a = a + (((a3 + b3) + c3) + d3) * scale2(c.k3, s3);
+    a = a + (((a4 + b4) + c4) + d4) * scale2(c.k4, s3);
+    a = a + (((a5 + b5) + c5) + d5) * scale2(c.k5, s5);
+    if (forced) {
+        const double e6 = cy == 0 ? 0.0 : (diag ? sgn_c(cy, 0.5) : sgn_c(-cy, 0.5));
+        const double e7 = cx == 0 ? 0.0 : (diag ? sgn_c(cx, 0.5) : sgn_c(-cx, 0.5));
+        const double g6 = (rest || diag ? c.uy : -c.uy) + e6, g7 = (rest || diag ? c.ux : -c.ux) + e7;
+        a = a + g6 * scale2(c.k6, rest ? 1 : (diag ? -1 : 0));
+        a = a + g7 * scale2(c.k7, rest ? 1 : (diag ? -1 : 0));
+    }
+    const double k8 = scale2(c.k8, rest ? 0 : (diag ? -2 : -1));
+    return rest || diag ? a + k8 : a - k8;
 }
 
 }  // namespace life

@@ -315,7 +315,7 @@ __device__ __forceinline__ void collide_bgk(const double f[9], double rho, doubl
 
 // Central-moments collision (De Rosis 2019; src/Grid.cpp:106-233), in collide_cm.cuh.
 template <bool UNF = false>
-__device__ __forceinline__ void collide_cm(const double f[9], double rho, double ux, double uy, double Fx,
+__host__ __device__ __forceinline__ void collide_cm(const double f[9], double rho, double ux, double uy, double Fx,
                                            double Fy, double omega, double cs, double fs[9]);
 
 // force_xy_at in float for the FP32 kernels (values rounded on the host).

@@ -21,6 +21,7 @@
 #include "collide_cm.cuh"
 #include "lbm_device.cuh"
 #include "lbm_kernels.h"
+#include "lbm_lanes.cuh"
 
 namespace life {
 
@@ -162,11 +163,12 @@ __global__ void __launch_bounds__(256) k_interior_batch_f64(const BatchLatCase* 
     }
 }
 
-// Boundary-condition sites of one step, FP64 storage (perimeter_site,
-// lbm_device.cuh); the reduced-precision forms have theirs in lbm_lowp.cu.
+// Boundary-condition sites of one step, FP64 storage, three per warp
+// (lbm_lanes.cuh); the reduced-precision forms have theirs in lbm_lowp.cu.
 template <bool CM, class S>
-__global__ void k_perimeter(const typename S::T* __restrict__ A, typename S::T* __restrict__ B, LatDev L, int t) {
-    perimeter_site<CM, S>(A, B, L, step_t(L, t), blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(32) k_perimeter(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
+                                                  LatDev L, int t) {
+    lanes_perimeter<CM, S>(A, B, L, step_t(L, t), kLaneSites * (int)blockIdx.x);
 }
 
 // GridClass::convectiveSpeed (src/Grid.cpp:477-495): the mean outlet speed is
@@ -495,9 +497,9 @@ cudaError_t launch_perimeter(const void* A, void* B, const LatDev& L, int t, cud
     if (L.prec != LIFE_PREC_F64) return launch_perimeter_lowp(A, B, L, t, s);
     // one warp per block, spread over the SMs' FP64 units (as the
     // reduced-precision perimeter)
-    const int n = 2 * L.Nx + 2 * (L.Ny - 2);
-    if (L.cm) k_perimeter<true, StoreF64><<<(n + 31) / 32, 32, 0, s>>>((const double*)A, (double*)B, L, t);
-    else k_perimeter<false, StoreF64><<<(n + 31) / 32, 32, 0, s>>>((const double*)A, (double*)B, L, t);
+    const int n = 2 * L.Nx + 2 * (L.Ny - 2), g = (n + kLaneSites - 1) / kLaneSites;
+    if (L.cm) k_perimeter<true, StoreF64><<<g, 32, 0, s>>>((const double*)A, (double*)B, L, t);
+    else k_perimeter<false, StoreF64><<<g, 32, 0, s>>>((const double*)A, (double*)B, L, t);
     return cudaGetLastError();
 }
 

@@ -36,6 +36,7 @@
 #include <type_traits>
 
 #include "lbm_kernels.h"
+#include "lbm_lanes.cuh"
 #include "tma.cuh"
 
 namespace life {
@@ -401,11 +402,12 @@ cudaError_t launch_interior_lowp(const void* A, void* B, const LatDev& L, int t,
     return cudaGetLastError();
 }
 
-// Boundary-condition sites, reduced-precision storage (perimeter_site,
-// lbm_device.cuh; FP64 arithmetic, rounded as in lbm_f64.cu).
+// Boundary-condition sites, reduced-precision storage, three per warp
+// (lbm_lanes.cuh; FP64 arithmetic, rounded as in lbm_f64.cu).
 template <bool CM, class S>
-__global__ void k_perimeter_lowp(const typename S::T* __restrict__ A, typename S::T* __restrict__ B, LatDev L, int t) {
-    perimeter_site<CM, S>(A, B, L, step_t(L, t), blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(32) k_perimeter_lowp(const typename S::T* __restrict__ A,
+                                                       typename S::T* __restrict__ B, LatDev L, int t) {
+    lanes_perimeter<CM, S>(A, B, L, step_t(L, t), kLaneSites * (int)blockIdx.x);
 }
 
 // One warp per block: a boundary site is a long FP64 chain, and an SM's FP64
@@ -413,7 +415,7 @@ __global__ void k_perimeter_lowp(const typename S::T* __restrict__ A, typename S
 // rather than packed four warps to an SM.
 cudaError_t launch_perimeter_lowp(const void* A, void* B, const LatDev& L, int t, cudaStream_t s) {
     const int n = 2 * L.Nx + 2 * (L.Ny - 2);
-    const int g = (n + 31) / 32;
+    const int g = (n + kLaneSites - 1) / kLaneSites;
     if (L.prec == LIFE_PREC_F32) {
         if (L.cm) k_perimeter_lowp<true, StoreF32><<<g, 32, 0, s>>>((const float*)A, (float*)B, L, t);
         else k_perimeter_lowp<false, StoreF32><<<g, 32, 0, s>>>((const float*)A, (float*)B, L, t);
@@ -516,16 +518,6 @@ struct TmaShape {
 // Waits that gave up (never expected; the host turns a non-zero count into
 // LIFE_ERR_TIMEOUT).
 __device__ int g_tma_timeouts;
-
-__device__ __forceinline__ bool perimeter_ij(const LatDev& L, int q, int& i, int& j) {
-    const int Nx = L.Nx, Ny = L.Ny;
-    if (q < Nx) { i = q; j = 0; }
-    else if (q < 2 * Nx) { i = q - Nx; j = Ny - 1; }
-    else if (q < 2 * Nx + (Ny - 2)) { i = 0; j = q - 2 * Nx + 1; }
-    else if (q < 2 * Nx + 2 * (Ny - 2)) { i = Nx - 1; j = q - 2 * Nx - (Ny - 2) + 1; }
-    else return false;
-    return true;
-}
 
 template <bool CM, bool FORCED, class S>
 __device__ __forceinline__ void tma_tile_sites(const unsigned char* stage, typename S::T* __restrict__ B,
