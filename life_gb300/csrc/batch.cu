@@ -44,10 +44,13 @@ int ibm_apply(LifeCase* c, int t, const void* A, void* B, cudaStream_t s);
 
 namespace {
 
-__global__ void k_batch_advance(int* __restrict__ tnow, int n) {
+__global__ void k_batch_advance(int* __restrict__ tnow, int n, int steps) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) tnow[k] += 1;
+    if (k < n) tnow[k] += steps;
 }
+
+// Steps per graph launch of a small single case (see chain_steps).
+constexpr int kChain = 16;
 
 }  // namespace
 
@@ -70,6 +73,10 @@ struct LifeBatch {
     // relative to (t_base, cur_base) of each case
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
     int kernel_nodes[2] = {0, 0};
+    // kChain steps from an even parity in one graph (single small cases)
+    cudaGraphExec_t chain = nullptr;
+    int chain_nodes = 0;
+    long long launched = 0;  // kernel nodes launched so far
     std::vector<int> t_base, cur_base, rec_gen;
     std::vector<int> ring_end;  // step tables are valid for t < ring_end[k]
     std::string status_msg;
@@ -85,6 +92,8 @@ static void drop_graphs(LifeBatch* b) {
             cudaGraphExecDestroy(g);
             g = nullptr;
         }
+    if (b->chain) cudaGraphExecDestroy(b->chain);
+    b->chain = nullptr;
 }
 
 static void free_batch(LifeBatch* b) {
@@ -160,14 +169,15 @@ static bool fused_step(const LifeBatch* b) {
 // The interior launch of one batch step. `h`/`d`: the host and device copies
 // of the case table (the batch's own, or the scratch table of time_interior).
 static cudaError_t launch_batch_interior(LifeBatch* b, int phase, cudaStream_t s, const BatchLatCase* h = nullptr,
-                                         const BatchLatCase* d = nullptr) {
+                                         const BatchLatCase* d = nullptr, int t_off = 1) {
     if (!h) h = b->h_cases.data();
     if (!d) d = b->d_cases;
     if (b->cases.size() == 1) {
         // one case: its own interior kernel (one CTA row segment per block);
         // in the reduced-precision forms the launch also takes the perimeter
         const BatchLatCase& C = h[0];
-        const LatDev& L = C.L[phase];
+        LatDev L = C.L[phase];
+        L.t_off = t_off;
         const int t = b->cases[0]->t + 1 + phase;  // ignored: kernels read *L.t_dev + L.t_off
         if (b->prec == LIFE_PREC_F64) return launch_interior_f64((const double*)C.A[phase], (double*)C.B[phase], L, t, s);
         if (fused_step(b)) return launch_step_lowp(C.A[phase], C.B[phase], L, t, s);
@@ -178,12 +188,13 @@ static cudaError_t launch_batch_interior(LifeBatch* b, int phase, cudaStream_t s
     return launch_interior_batch_lowp(b->prec, d, b->d_tile_case, b->ntiles, b->tile_w, b->tile_h, b->grid, phase, s);
 }
 
-// Before a step from state t the step tables must hold t+1 and t+2; when they
-// do not, they are refilled for the next `n` steps (at most kStepChunk).
-static int refill_steps(LifeBatch* b, int n) {
+// Before `ahead` steps from state t the step tables must hold t+1..t+ahead+1;
+// when they do not, they are refilled for the next `n` steps (at most
+// kStepChunk, at least `ahead`).
+static int refill_steps(LifeBatch* b, int n, int ahead = 1) {
     for (size_t k = 0; k < b->cases.size(); k++) {
         LifeCase* c = b->cases[k];
-        if (c->t + 3 <= b->ring_end[k]) continue;
+        if (c->t + 2 + ahead <= b->ring_end[k]) continue;
         const int m = std::min(std::max(n, 1), kStepChunk) + 2;
         CK(cudaStreamSynchronize(b->stream));
         if (int rc = ensure_steps(c, c->t, m)) return rc;
@@ -192,61 +203,65 @@ static int refill_steps(LifeBatch* b, int n) {
     return LIFE_OK;
 }
 
-// Captures one batch step at the cases' current state and advances the host
-// view of every case by that step (t, buffer parity, IBM scratch parity).
+// Captures batch steps from the cases' current state and advances the host
+// view of every case by them (t, buffer parity, IBM scratch parity).
 // Per case, the convective outlet and the boundary perimeter run on the
 // case's side stream; the interior launch waits only for the outlets (the
 // perimeter and the interior both read P[cur] and write disjoint sites of
 // P[cur^1], so they overlap). The IBM forces (interpolation, or the FSI
 // subiteration loop) read only P[cur] and run beside the lattice step on the
 // case's aux stream after the outlet; the spread waits for all of them.
-static int capture_step(LifeBatch* b, int phase, cudaGraphExec_t* out, int* kernels) {
+static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* out, int* kernels) {
     cudaStream_t bs = b->stream;
     const int n = (int)b->cases.size();
     CK(cudaStreamBeginCapture(bs, cudaStreamCaptureModeThreadLocal));
     int rc = LIFE_OK;
-    cudaError_t e = cudaEventRecord(b->ev_fork, bs);
-    for (int k = 0; k < n && e == cudaSuccess && rc == LIFE_OK; k++) {
-        LifeCase* c = b->cases[k];
-        c->t_dev = b->d_tnow + k;
-        c->t_off = 1;
-        const int tt = c->t + 1;
-        const LatDev L = lattice_view(c, tt);
-        e = cudaStreamWaitEvent(c->side, b->ev_fork, 0);
-        // the outlet reads the outlet columns before the interior rewrites them
-        if (e == cudaSuccess && L.convective) e = launch_outlet(L, c->d_delU, c->side);
-        if (e == cudaSuccess) e = cudaEventRecord(c->ev_out, c->side);
-        if (e == cudaSuccess && L.convective) e = cudaStreamWaitEvent(bs, c->ev_out, 0);
-        const bool fused = fused_step(b);  // perimeter inside the interior launch
-        if (e == cudaSuccess && !fused) e = launch_perimeter(c->P[c->cur], c->P[c->cur ^ 1], L, tt, c->side);
-        if (e == cudaSuccess) e = cudaEventRecord(c->ev_join, c->side);
-        if (e == cudaSuccess && c->obj.hasIBM) {
-            e = cudaStreamWaitEvent(c->aux, c->ev_out, 0);
-            if (e == cudaSuccess) rc = ibm_forces(c, tt, c->P[c->cur], c->aux);
-            if (e == cudaSuccess && rc == LIFE_OK) e = cudaEventRecord(c->ev_aux, c->aux);
+    cudaError_t e = cudaSuccess;
+    for (int s = 0; s < steps && e == cudaSuccess && rc == LIFE_OK; s++) {
+        const int phase = (phase0 + s) & 1;
+        e = cudaEventRecord(b->ev_fork, bs);
+        for (int k = 0; k < n && e == cudaSuccess && rc == LIFE_OK; k++) {
+            LifeCase* c = b->cases[k];
+            c->t_dev = b->d_tnow + k;
+            c->t_off = 1 + s;
+            const int tt = c->t + 1;
+            const LatDev L = lattice_view(c, tt);
+            e = cudaStreamWaitEvent(c->side, b->ev_fork, 0);
+            // the outlet reads the outlet columns before the interior rewrites them
+            if (e == cudaSuccess && L.convective) e = launch_outlet(L, c->d_delU, c->side);
+            if (e == cudaSuccess) e = cudaEventRecord(c->ev_out, c->side);
+            if (e == cudaSuccess && L.convective) e = cudaStreamWaitEvent(bs, c->ev_out, 0);
+            const bool fused = fused_step(b);  // perimeter inside the interior launch
+            if (e == cudaSuccess && !fused) e = launch_perimeter(c->P[c->cur], c->P[c->cur ^ 1], L, tt, c->side);
+            if (e == cudaSuccess) e = cudaEventRecord(c->ev_join, c->side);
+            if (e == cudaSuccess && c->obj.hasIBM) {
+                e = cudaStreamWaitEvent(c->aux, c->ev_out, 0);
+                if (e == cudaSuccess) rc = ibm_forces(c, tt, c->P[c->cur], c->aux);
+                if (e == cudaSuccess && rc == LIFE_OK) e = cudaEventRecord(c->ev_aux, c->aux);
+            }
         }
-    }
-    if (e == cudaSuccess && rc == LIFE_OK) e = launch_batch_interior(b, phase, bs);
-    if (e == cudaSuccess) e = cudaEventRecord(b->ev_int, bs);
-    for (int k = 0; k < n && e == cudaSuccess && rc == LIFE_OK; k++) {
-        LifeCase* c = b->cases[k];
-        const int tt = c->t + 1;
-        const void* A = c->P[c->cur];
-        void* B = c->P[c->cur ^ 1];
-        if (c->stream != bs) e = cudaStreamWaitEvent(c->stream, b->ev_int, 0);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_join, 0);
-        if (e == cudaSuccess && c->obj.hasIBM) e = cudaStreamWaitEvent(c->stream, c->ev_aux, 0);
-        if (e == cudaSuccess && c->obj.hasIBM) rc = ibm_apply(c, tt, A, B, c->stream);
-        if (e == cudaSuccess && rc == LIFE_OK) e = launch_record(c, tt, c->stream);
-        if (c->stream != bs) {
-            if (e == cudaSuccess && rc == LIFE_OK) e = cudaEventRecord(c->ev_done, c->stream);
-            if (e == cudaSuccess && rc == LIFE_OK) e = cudaStreamWaitEvent(bs, c->ev_done, 0);
+        if (e == cudaSuccess && rc == LIFE_OK) e = launch_batch_interior(b, phase, bs, nullptr, nullptr, 1 + s);
+        if (e == cudaSuccess) e = cudaEventRecord(b->ev_int, bs);
+        for (int k = 0; k < n && e == cudaSuccess && rc == LIFE_OK; k++) {
+            LifeCase* c = b->cases[k];
+            const int tt = c->t + 1;
+            const void* A = c->P[c->cur];
+            void* B = c->P[c->cur ^ 1];
+            if (c->stream != bs) e = cudaStreamWaitEvent(c->stream, b->ev_int, 0);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_join, 0);
+            if (e == cudaSuccess && c->obj.hasIBM) e = cudaStreamWaitEvent(c->stream, c->ev_aux, 0);
+            if (e == cudaSuccess && c->obj.hasIBM) rc = ibm_apply(c, tt, A, B, c->stream);
+            if (e == cudaSuccess && rc == LIFE_OK) e = launch_record(c, tt, c->stream);
+            if (c->stream != bs) {
+                if (e == cudaSuccess && rc == LIFE_OK) e = cudaEventRecord(c->ev_done, c->stream);
+                if (e == cudaSuccess && rc == LIFE_OK) e = cudaStreamWaitEvent(bs, c->ev_done, 0);
+            }
+            c->cur ^= 1;
+            c->t = tt;
         }
-        c->cur ^= 1;
-        c->t = tt;
     }
     if (e == cudaSuccess && rc == LIFE_OK) {
-        k_batch_advance<<<(n + 127) / 128, 128, 0, bs>>>(b->d_tnow, n);
+        k_batch_advance<<<(n + 127) / 128, 128, 0, bs>>>(b->d_tnow, n, steps);
         e = cudaGetLastError();
     }
     for (LifeCase* c : b->cases) {
@@ -275,12 +290,26 @@ static int capture_step(LifeBatch* b, int phase, cudaGraphExec_t* out, int* kern
             cudaGraphNodeGetType(nd, &ty);
             if (ty == cudaGraphNodeTypeKernel) kn++;
         }
-        for (LifeCase* c : b->cases) kn += c->loop_body_kernels;
+        for (LifeCase* c : b->cases) kn += steps * c->loop_body_kernels;
         *kernels = kn;
     }
     if (g) cudaGraphDestroy(g);
     if (e != cudaSuccess) return cuda_fail(e, "batch step graph");
     return LIFE_OK;
+}
+
+// Undoes what captures did to the host view since the graphs' base state.
+static void rewind_host_view(LifeBatch* b) {
+    for (size_t k = 0; k < b->cases.size(); k++) {
+        LifeCase* c = b->cases[k];
+        const int adv = c->t - b->t_base[k];
+        c->t = b->t_base[k];
+        c->cur = b->cur_base[k];
+        if (adv & 1) {
+            std::swap(c->W.sites, c->W.sites_prev);
+            std::swap(c->W.nsites, c->W.nsites_prev);
+        }
+    }
 }
 
 static int build_graphs(LifeBatch* b) {
@@ -298,18 +327,8 @@ static int build_graphs(LifeBatch* b) {
         b->rec_gen[k] = b->cases[k]->rec_gen;
     }
     int rc = LIFE_OK;
-    for (int p = 0; p < 2 && rc == LIFE_OK; p++) rc = capture_step(b, p, &b->exec[p], &b->kernel_nodes[p]);
-    // the captures advanced the host view by up to two steps: undo
-    for (int k = 0; k < n; k++) {
-        LifeCase* c = b->cases[k];
-        const int adv = c->t - b->t_base[k];
-        c->t = b->t_base[k];
-        c->cur = b->cur_base[k];
-        if (adv & 1) {
-            std::swap(c->W.sites, c->W.sites_prev);
-            std::swap(c->W.nsites, c->W.nsites_prev);
-        }
-    }
+    for (int p = 0; p < 2 && rc == LIFE_OK; p++) rc = capture_steps(b, p, 1, &b->exec[p], &b->kernel_nodes[p]);
+    rewind_host_view(b);
     if (rc != LIFE_OK) drop_graphs(b);
     return rc;
 }
@@ -351,6 +370,33 @@ static int check_status(LifeBatch* b) {
     return LIFE_OK;
 }
 
+// Steps the next graph launch may take: kChain for a single case without
+// flexible bodies on a lattice below 2^22 sites, whose steps are so short that
+// the launch of each step's graph and its step-counter kernel show: 16 steps
+// in one graph against one took a 256^2 FP64 cavity from 28.9 to 24.0 us and a
+// 1501 x 703 FP32 channel from 28.3 to 23.9 us per step.
+// Larger lattices and flexible bodies step in 0.1 ms and more, and a batch of
+// several cases in about 1 ms. The chain is captured when a run is long enough
+// to repay it.
+static int chain_steps(LifeBatch* b, int left, int ph) {
+    if (b->cases.size() != 1 || left < kChain || ph != 0) return 1;
+    const LifeCase* c = b->cases[0];
+    if (c->obj.hasFlex || (long long)c->Nx * c->Ny >= (1LL << 22)) return 1;
+    if (!b->chain) {
+        if (left < 2 * kChain) return 1;
+        // captured from the base state, as the step graphs were
+        LifeCase* m = b->cases[0];
+        const int t = m->t, cur = m->cur;
+        m->t = b->t_base[0];
+        m->cur = b->cur_base[0];
+        const int rc = capture_steps(b, 0, kChain, &b->chain, &b->chain_nodes);
+        m->t = t;
+        m->cur = cur;
+        if (rc != LIFE_OK) return -rc;
+    }
+    return kChain;
+}
+
 static int run_batch(LifeBatch* b, int nsteps, cudaEvent_t start, cudaEvent_t stop, bool check = true) {
     if (graph_phase(b) < 0)
         if (int rc = build_graphs(b)) return rc;
@@ -362,18 +408,22 @@ static int run_batch(LifeBatch* b, int nsteps, cudaEvent_t start, cudaEvent_t st
         CK(cudaMemcpyAsync(b->d_tnow, tn.data(), sizeof(int) * n, cudaMemcpyHostToDevice, b->stream));
     }
     if (start) CK(cudaEventRecord(start, b->stream));
-    for (int s = 0; s < nsteps; s++) {
-        if (int rc = refill_steps(b, std::min(nsteps - s, kStepChunk))) return rc;
+    for (int s = 0; s < nsteps;) {
         const int ph = graph_phase(b);
-        CK(cudaGraphLaunch(b->exec[ph], b->stream));
+        const int m = chain_steps(b, nsteps - s, ph);
+        if (m < 0) return -m;
+        if (int rc = refill_steps(b, std::min(nsteps - s, kStepChunk), m)) return rc;
+        CK(cudaGraphLaunch(m > 1 ? b->chain : b->exec[ph], b->stream));
+        b->launched += m > 1 ? b->chain_nodes : b->kernel_nodes[ph];
         for (LifeCase* c : b->cases) {
-            c->t += 1;
-            c->cur ^= 1;
-            if (c->obj.hasIBM) {
+            c->t += m;
+            c->cur ^= m & 1;
+            if (c->obj.hasIBM && (m & 1)) {
                 std::swap(c->W.sites, c->W.sites_prev);
                 std::swap(c->W.nsites, c->W.nsites_prev);
             }
         }
+        s += m;
     }
     if (stop) CK(cudaEventRecord(stop, b->stream));
     return check ? check_status(b) : LIFE_OK;
@@ -460,7 +510,7 @@ int case_interior_ms(LifeCase* c, int reps, float* ms) {
     return life_batch_interior_ms(c->self_batch, reps, ms);
 }
 
-int case_kernels_per_step(LifeCase* c) { return c->self_batch ? c->self_batch->kernel_nodes[0] : 0; }
+long long case_kernels_launched(const LifeCase* c) { return c->self_batch ? c->self_batch->launched : 0; }
 int batch_steps(LifeBatch* b, int nsteps) { return life_batch_step(b, nsteps); }
 // Per-case device status after a failed batch run: the index of the first
 // failing case (or -1) and its code.

@@ -468,8 +468,9 @@ static int run_steps(LifeCase* c, int nsteps, StepTiming* tm) {
     const bool direct = !c->host_steps && !tm && nsteps < kDirectMaxSteps && !case_graphs_ready(c);
     if (!c->host_steps && !direct) {
         // the case's captured step graphs; the same kernels in the same order
+        const long long before = case_kernels_launched(c);
         if ((rc = case_graph_steps(c, nsteps, tm ? tm->start : nullptr, tm ? tm->stop : nullptr))) return rc;
-        if (tm) tm->launches = case_kernels_per_step(c) * nsteps;
+        if (tm) tm->launches = (int)(case_kernels_launched(c) - before);
         if (c->obj.hasFlex) {
             if ((rc = check_device_status(c))) return rc;
             if (c->status_code) {

@@ -127,8 +127,8 @@ bool case_graphs_ready(const LifeCase* c);
 bool case_fused_step(const LifeCase* c);
 // Mean device time of the case's interior kernel alone over reps launches.
 int case_interior_ms(LifeCase* c, int reps, float* ms);
-// Kernel nodes of one captured step of the case (0 before the first capture).
-int case_kernels_per_step(LifeCase* c);
+// Kernel nodes the case's step graphs have launched so far.
+long long case_kernels_launched(const LifeCase* c);
 void free_fem(LifeCase* c);
 // The recorder's kernel for the step ending at t (a no-op without a recorder);
 // inside a capture the step is read from c->t_dev.
