@@ -281,28 +281,66 @@ __device__ __forceinline__ bool export_fluid_lowp(const typename S::T* __restric
 }
 
 // Reference-layout export of the state after step t (what
-// GridClass::writeRestart dumps, src/Grid.cpp:1191-1222). The reference
-// layout is column-major in the device's terms (id = i*Ny + j), so a block
-// computes a 32 x 32 tile of sites with i fastest (the pulls read whole rows
-// of each population plane) and writes rho, u and force_ibm through shared
-// memory with j fastest (whole runs of the output); f, exported for restart
-// sets and parity checks, is written per site.
+// GridClass::writeRestart dumps, src/Grid.cpp:1191-1222). The first `pb` blocks
+// take the boundary-condition sites, three per warp (lbm_lanes.cuh), the
+// others the fluid sites: as one thread of a tile each, a wall site kept its
+// warp 28 us per row, four rows after one another, and the whole launch
+// waited for it (77 us for a 256^2 FP64 lattice, 26 us now). The reference layout is column-major in the
+// device's terms (id = i*Ny + j), so a block computes a 32 x 32 tile of sites
+// with i fastest (the pulls read whole rows of each population plane) and
+// writes rho, u and force_ibm through shared memory with j fastest (whole runs
+// of the output, which may be page-locked host memory); f, exported for
+// restart sets and parity checks, is written per site. Columns i0 <= i < i1
+// (their reference-layout rows are one contiguous range of the output).
 template <bool CM, class S>
 __global__ void __launch_bounds__(256) k_export(const typename S::T* __restrict__ P, LatDev L, int t,
                                                 double* __restrict__ rho_out, double* __restrict__ u_out,
                                                 double* __restrict__ f_out, double* __restrict__ fibm_out, int i0,
-                                                int i1) {
-    // columns i0 <= i < i1 (their reference-layout rows id = i*Ny + j are
-    // one contiguous range of the output)
+                                                int i1, int pb, int tiles_x) {
     __shared__ double s_rho[32][33];
     __shared__ double2 s_u[32][33], s_fi[32][33];
-    const int ib = i0 + blockIdx.x * 32, jb = blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
+    if ((int)blockIdx.x < pb) {
+        const SiteLane g = site_lane();
+        int i = 0, j = 0;
+        bool on = perimeter_ij(L, kLaneSites * (8 * (int)blockIdx.x + ty) + g.slot, i, j);
+        on = on && i >= i0 && i < i1 && site_type(L, i, j) != LIFE_FLUID;
+        if (!__any_sync(kAllLanes, on)) return;
+        double f, rho, ux, uy, Ix = 0.0, Iy = 0.0;
+        lanes_state<CM, S>(P, L, t, g, i, j, f, rho, ux, uy);
+        if (L.force_ibm) {
+            const size_t s = (size_t)j * L.pitch + i;
+            Ix = L.force_ibm[s];
+            Iy = L.force_ibm[L.S + s];
+            const bool ibm = Ix != 0.0 || Iy != 0.0;
+            if (__any_sync(kAllLanes, ibm)) {
+                double Fx, Fy, r, x, y;
+                force_xy_of(L, t, i, j, Fx, Fy);
+                lanes_macroscopic(g, f, Fx + Ix, Fy + Iy, r, x, y);
+                if (ibm) {
+                    rho = r;
+                    ux = x;
+                    uy = y;
+                }
+            }
+        }
+        if (!on || !g.store) return;
+        const size_t id = (size_t)i * L.Ny + j;
+        if (f_out) f_out[id * 9 + g.v] = f;
+        if (g.v == 0) {
+            if (rho_out) rho_out[id] = rho;
+            if (u_out) reinterpret_cast<double2*>(u_out)[id] = make_double2(ux, uy);
+            if (fibm_out) reinterpret_cast<double2*>(fibm_out)[id] = make_double2(Ix, Iy);
+        }
+        return;
+    }
+    const int b = (int)blockIdx.x - pb;
+    const int ib = i0 + b % tiles_x * 32, jb = b / tiles_x * 32;
     const int i = ib + tx;
 #pragma unroll 1
     for (int q = ty; q < 32; q += 8) {
         const int j = jb + q;
-        if (i >= i1 || j >= L.Ny) continue;
+        if (i >= i1 || j >= L.Ny || site_type(L, i, j) != LIFE_FLUID) continue;
         double f[9], rho, ux, uy;
         double Ix = 0.0, Iy = 0.0;
         if (export_fluid_lowp<S>(P, L, t, i, j, f_out == nullptr, rho, ux, uy)) {
@@ -311,17 +349,16 @@ __global__ void __launch_bounds__(256) k_export(const typename S::T* __restrict_
             s_fi[tx][q] = make_double2(0.0, 0.0);
             continue;
         }
-        site_state<CM, S>(P, L, t, i, j, f, rho, ux, uy);
+        double Fx, Fy;
+        gather<S>(P, L, i, j, f);
+        force_xy_of(L, t, i, j, Fx, Fy);
         if (L.force_ibm) {
             const size_t s = (size_t)j * L.pitch + i;
             Ix = L.force_ibm[s];
             Iy = L.force_ibm[L.S + s];
-            if (Ix != 0.0 || Iy != 0.0) {
-                double Fx, Fy;
-                force_xy_of(L, t, i, j, Fx, Fy);
-                macroscopic_ibm(f, Fx, Fy, Ix, Iy, rho, ux, uy);
-            }
         }
+        if (Ix != 0.0 || Iy != 0.0) macroscopic_ibm(f, Fx, Fy, Ix, Iy, rho, ux, uy);
+        else macroscopic(f, Fx, Fy, rho, ux, uy);
         s_rho[tx][q] = rho;
         s_u[tx][q] = make_double2(ux, uy);
         s_fi[tx][q] = make_double2(Ix, Iy);
@@ -335,7 +372,7 @@ __global__ void __launch_bounds__(256) k_export(const typename S::T* __restrict_
 #pragma unroll 1
     for (int r = ty; r < 32; r += 8) {
         const int io = ib + r, jo = jb + tx;
-        if (io >= i1 || jo >= L.Ny) continue;
+        if (io >= i1 || jo >= L.Ny || site_type(L, io, jo) != LIFE_FLUID) continue;
         const size_t id = (size_t)io * L.Ny + jo;
         if (rho_out) rho_out[id] = s_rho[r][tx];
         if (u_out) reinterpret_cast<double2*>(u_out)[id] = s_u[r][tx];
@@ -523,17 +560,22 @@ cudaError_t launch_export(const void* P, const LatDev& L, int t, bool initial, d
         return cudaGetLastError();
     }
     if (i1 <= i0) return cudaSuccess;
-    const dim3 g((i1 - i0 + 31) / 32, (L.Ny + 31) / 32), blk(32, 8);
+    const int tiles_x = (i1 - i0 + 31) / 32, pb = (2 * L.Nx + 2 * (L.Ny - 2) + 8 * kLaneSites - 1) / (8 * kLaneSites);
+    const int g = pb + tiles_x * ((L.Ny + 31) / 32);
+    const dim3 blk(32, 8);
+#define LIFE_EXPORT(CM, S) \
+    k_export<CM, S><<<g, blk, 0, s>>>((const typename S::T*)P, L, t, rho, u, f, fibm, i0, i1, pb, tiles_x)
     if (L.prec == LIFE_PREC_F64) {
-        if (L.cm) k_export<true, StoreF64><<<g, blk, 0, s>>>((const double*)P, L, t, rho, u, f, fibm, i0, i1);
-        else k_export<false, StoreF64><<<g, blk, 0, s>>>((const double*)P, L, t, rho, u, f, fibm, i0, i1);
+        if (L.cm) LIFE_EXPORT(true, StoreF64);
+        else LIFE_EXPORT(false, StoreF64);
     } else if (L.prec == LIFE_PREC_F32) {
-        if (L.cm) k_export<true, StoreF32><<<g, blk, 0, s>>>((const float*)P, L, t, rho, u, f, fibm, i0, i1);
-        else k_export<false, StoreF32><<<g, blk, 0, s>>>((const float*)P, L, t, rho, u, f, fibm, i0, i1);
+        if (L.cm) LIFE_EXPORT(true, StoreF32);
+        else LIFE_EXPORT(false, StoreF32);
     } else {
-        if (L.cm) k_export<true, StoreF16><<<g, blk, 0, s>>>((const __half*)P, L, t, rho, u, f, fibm, i0, i1);
-        else k_export<false, StoreF16><<<g, blk, 0, s>>>((const __half*)P, L, t, rho, u, f, fibm, i0, i1);
+        if (L.cm) LIFE_EXPORT(true, StoreF16);
+        else LIFE_EXPORT(false, StoreF16);
     }
+#undef LIFE_EXPORT
     return cudaGetLastError();
 }
 
