@@ -812,6 +812,205 @@ __device__ void band_solve_smem(double* Bd, int nn, int kl, int ku, int W, const
         }
 }
 
+// Dense LU and transposed solve (band_lu.h semantics) of a matrix whose
+// nonzeros are few but not in a narrow band, by one CTA: the epsilon system of
+// a closed line of markers (the first and the last are neighbours) or of
+// several bodies that touch. M(i, k) is at D[k * n + i]; rmask holds, for each
+// row, a bit per column that may be nonzero, cmask the same by column (nw
+// words each). Elimination step j visits only the rows with a bit in column j
+// and the columns with a bit in the pivot row, and spreads the bits as the
+// update fills entries in. Every other entry is an exact zero, whose products
+// leave the values they are added to unchanged, so each value is formed by the
+// same operations in the same order as in the dense loops. A step:
+//   phase 1  warp 0 lists column j's rows, picks the first maximal magnitude
+//            (each lane forms its candidate's reciprocal meanwhile); warp 1
+//            lists row j's columns; the last warp takes the forward
+//            substitution of step j-1 (y[k] -= U(j-1,k) y[j-1])
+//   swap     only where the pivot is not on the diagonal: whole rows, their
+//            masks, and row j's column list again
+//   phase 2  one thread per updated entry (its row's multiplier formed by
+//            each); the masks
+// b in y, the solution in y; rows and cols: 2n ints each. Needs 128 threads.
+// Returns false (uniformly) when a pivot is zero or not finite or the solution
+// is not finite: then zeros do matter, and the caller runs the dense loops.
+// One warp over all of the band (kl = ku = n) took 6.49 ms for the 132 markers
+// of a circle and its tail; this takes 0.32 ms, bound by the latencies of a
+// step (the lists, reciprocal, multiplier, product, difference).
+struct SparseLu {
+    double* D;
+    unsigned *rmask, *cmask;
+    double *y, *rcp;
+    int *piv, *rows, *cols;
+};
+
+// Set bits above `above` of an n-bit mask as an ascending list (one warp;
+// nw <= 32); returns the count on every lane.
+__device__ __forceinline__ int mask_list(const unsigned* mask, int nw, int above, int* out) {
+    const int lane = threadIdx.x & 31;
+    unsigned w = lane < nw ? mask[lane] : 0u;
+    const int first = above + 1 - 32 * lane;  // first wanted bit of this word
+    if (first >= 32) w = 0u;
+    else if (first > 0) w &= ~0u << first;
+    const int c = __popc(w);
+    int sum = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += x;
+    }
+    int at = sum - c;
+    while (w) {
+        out[at++] = 32 * lane + __ffs(w) - 1;
+        w &= w - 1;
+    }
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, sum, 31);
+}
+
+__device__ __forceinline__ bool finite_bits(double x) {
+    return ((unsigned)(__double_as_longlong(x) >> 32) & 0x7ff00000u) != 0x7ff00000u;
+}
+
+__device__ bool sparse_lu_solve(const SparseLu& S, int n, int nw) {
+    __shared__ int s_nr, s_nc[2], s_jp, s_bad, s_any;
+    __shared__ double s_r;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, last = (blockDim.x >> 5) - 1;
+    double* D = S.D;
+    if (tid == 0) { s_bad = 0; s_any = 0; }
+    __syncthreads();
+    for (int j = 0; j <= n; j++) {
+        const int pb = j & 1;
+        int *rows = S.rows + pb * n, *cols = S.cols + pb * n;
+        // phase 1
+        if (warp == 0 && j < n) {
+            const int nr = mask_list(S.cmask + (size_t)j * nw, nw, j, rows);  // below the diagonal
+            // candidates: the diagonal, then the listed rows
+            unsigned bh = 0, bl = 0;
+            int jp = -1;
+            double r = 0.0;
+            for (int q0 = 0; q0 <= nr; q0 += 32) {
+                const int q = q0 + lane;
+                const bool valid = q <= nr;
+                const int row = q == 0 ? j : (valid ? rows[q - 1] : j);
+                const double v = valid ? D[(size_t)j * n + row] : 0.0;
+                const double rc = __drcp_rn(v);
+                unsigned long long key = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+                if (key > 0x7ff0000000000000ull) key = q == 0 ? ~0ull : 0ull;
+                const unsigned kh = (unsigned)(key >> 32), klo = (unsigned)key;
+                const unsigned mh = __reduce_max_sync(0xffffffffu, valid ? kh : 0u);
+                const bool c1 = valid && kh == mh;
+                const unsigned ml = __reduce_max_sync(0xffffffffu, c1 ? klo : 0u);
+                const int src = __ffs(__ballot_sync(0xffffffffu, c1 && klo == ml)) - 1;
+                if (jp < 0 || mh > bh || (mh == bh && ml > bl)) {
+                    bh = mh;
+                    bl = ml;
+                    jp = __shfl_sync(0xffffffffu, row, src);
+                    r = __shfl_sync(0xffffffffu, rc, src);
+                }
+            }
+            if (lane == 0) {
+                s_nr = nr;
+                s_jp = jp;
+                s_r = r;
+                S.piv[j] = jp;
+                S.rcp[j] = r;
+                if ((bh | bl) == 0u || bh >= 0x7ff00000u) s_bad = 1;
+                if (jp != j) s_any = 1;
+            }
+        } else if (warp == 1 && j < n) {
+            const int nc = mask_list(S.rmask + (size_t)j * nw, nw, j, cols);
+            if (lane == 0) s_nc[pb] = nc;
+        } else if (warp == last && j > 0) {
+            const int k = j - 1, nc = s_nc[pb ^ 1];
+            const int* pc = S.cols + (pb ^ 1) * n;
+            const double yk = div_rn_recip(S.y[k], D[(size_t)k * n + k], S.rcp[k]);
+            __syncwarp();
+            if (lane == 0) S.y[k] = yk;
+            for (int q = lane; q < nc; q += 32) S.y[pc[q]] = S.y[pc[q]] - D[(size_t)pc[q] * n + k] * yk;
+        }
+        __syncthreads();
+        if (j == n || s_bad) break;
+        const int jp = s_jp, nr = s_nr;
+        if (jp != j) {
+            for (int k = tid; k < n; k += blockDim.x) {
+                const double a = D[(size_t)k * n + j], b = D[(size_t)k * n + jp];
+                D[(size_t)k * n + j] = b;
+                D[(size_t)k * n + jp] = a;
+                unsigned* m = S.cmask + (size_t)k * nw;
+                const unsigned bj = (m[j >> 5] >> (j & 31)) & 1u, bp = (m[jp >> 5] >> (jp & 31)) & 1u;
+                if (bj != bp) {
+                    m[j >> 5] ^= 1u << (j & 31);
+                    m[jp >> 5] ^= 1u << (jp & 31);
+                }
+            }
+            for (int w = tid; w < nw; w += blockDim.x) {
+                const unsigned a = S.rmask[(size_t)j * nw + w];
+                S.rmask[(size_t)j * nw + w] = S.rmask[(size_t)jp * nw + w];
+                S.rmask[(size_t)jp * nw + w] = a;
+            }
+            __syncthreads();
+            if (warp == 1) {
+                const int nc = mask_list(S.rmask + (size_t)j * nw, nw, j, cols);
+                if (lane == 0) s_nc[pb] = nc;
+            }
+            __syncthreads();
+        }
+        // phase 2
+        const int nc = s_nc[pb];
+        const double r = s_r;
+        for (int q = tid; q < nr * nc; q += blockDim.x) {
+            const int b = q / nr, i = rows[q - b * nr], k = cols[b];
+            const double l = D[(size_t)j * n + i] * r;
+            D[(size_t)k * n + i] = D[(size_t)k * n + i] - l * D[(size_t)k * n + j];
+        }
+        // the filled-in entries' bits: row masks by (row, word), column masks
+        // by (column, word); only columns above j and rows below the diagonal
+        for (int q = blockDim.x - 1 - tid; q < (nr + nc) * nw; q += blockDim.x) {
+            const int a = q / nw, w = q - a * nw;
+            const int first = j + 1 - 32 * w;
+            const unsigned keep = first >= 32 ? 0u : (first > 0 ? ~0u << first : ~0u);
+            if (a < nr) S.rmask[(size_t)rows[a] * nw + w] |= S.rmask[(size_t)j * nw + w] & keep;
+            else S.cmask[(size_t)cols[a - nr] * nw + w] |= S.cmask[(size_t)j * nw + w] & keep;
+        }
+        __syncthreads();
+        // the multipliers, now that no thread reads column j any more; what
+        // runs beside this (phase 1 of step j+1) reads neither
+        if (warp == 2)
+            for (int a = lane; a < nr; a += 32) D[(size_t)j * n + rows[a]] *= r;
+    }
+    if (s_bad) return false;  // (set before a barrier: the same on all threads)
+    // L^T x = y from the last row up: the products of a column's multipliers
+    // on lanes, subtracted in ascending row order; then the row interchanges
+    if (warp == 0) {
+        for (int i = n - 1; i >= 0; i--) {
+            const int c = mask_list(S.cmask + (size_t)i * nw, nw, i, S.rows);
+            double t = S.y[i];
+            for (int q0 = 0; q0 < c; q0 += 32) {
+                const int m = c - q0 < 32 ? c - q0 : 32;
+                double pr = 0.0;
+                if (lane < m) {
+                    const int k = S.rows[q0 + lane];
+                    pr = D[(size_t)i * n + k] * S.y[k];
+                }
+                for (int q = 0; q < m; q++) t = t - __shfl_sync(0xffffffffu, pr, q);
+            }
+            __syncwarp();
+            if (lane == 0) S.y[i] = t;
+            __syncwarp();
+        }
+        if (lane == 0 && s_any)
+            for (int i = n - 1; i >= 0; i--)
+                if (S.piv[i] != i) {
+                    const double t = S.y[i];
+                    S.y[i] = S.y[S.piv[i]];
+                    S.y[S.piv[i]] = t;
+                }
+    }
+    __syncthreads();
+    bool ok = true;
+    for (int i = tid; i < n; i += blockDim.x) ok = ok && finite_bits(S.y[i]);
+    return __syncthreads_and(ok) != 0;
+}
+
 // Epsilon system of a contiguous marker range [m0, m0+dim) (ObjectsClass::
 // computeEpsilon, src/Objects.cpp:264-311). Markers interact only when both
 // coordinates are within 3 lattice units (the support is +-1.5); those pairs
@@ -940,7 +1139,49 @@ __device__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int di
         __syncthreads();
         return true;
     }
-    // wide band: dense system in global scratch, same entries
+    // wide band with few nonzeros: sparse elimination on a dense matrix behind
+    // the entries in shared memory, or in the global scratch if it is too large
+    const int nw = (dim + 31) / 32;
+    if (nw <= 32 && nc + (nc + 1) / 2 + 1 <= cap) {
+        // the entries' keys to the end of their values
+        int* ck = reinterpret_cast<int*>(cval + nc);
+        for (int c = threadIdx.x; c < nc; c += blockDim.x) ck[c] = ckey[c];
+        __syncthreads();
+        ckey = ck;
+        double* at = cval + nc + (nc + 1) / 2;
+        SparseLu S;
+        S.y = at;
+        S.rcp = S.y + dim;
+        S.piv = reinterpret_cast<int*>(S.rcp + dim);
+        S.rows = S.piv + dim;
+        S.cols = S.rows + 2 * dim;
+        S.rmask = reinterpret_cast<unsigned*>(S.cols + 2 * dim);
+        S.cmask = S.rmask + (size_t)dim * nw;
+        const long long ints = 5LL * dim + 2LL * dim * nw;
+        const long long used = (at - sm) + 2LL * dim + (ints + 1) / 2;
+        if (used <= sm_doubles) {
+            S.D = used + (long long)dim * dim <= sm_doubles ? sm + used : A;
+            for (int q = threadIdx.x; q < dim * dim; q += blockDim.x) S.D[q] = 0.0;
+            for (int q = threadIdx.x; q < 2 * dim * nw; q += blockDim.x) S.rmask[q] = 0u;
+            for (int i = threadIdx.x; i < dim; i += blockDim.x) S.y[i] = 1.0;
+            __syncthreads();
+            for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+                const int pp = ckey[c];
+                if (pp < 0) continue;
+                const int k = pp / dim, i = pp % dim;  // A[k][i] is M(i, k)
+                S.D[pp] = cval[c];
+                atomicOr(&S.rmask[(size_t)i * nw + (k >> 5)], 1u << (k & 31));
+                atomicOr(&S.cmask[(size_t)k * nw + (i >> 5)], 1u << (i & 31));
+            }
+            __syncthreads();
+            if (sparse_lu_solve(S, dim, nw)) {
+                for (int i = threadIdx.x; i < dim; i += blockDim.x) M.eps[m0 + i] = S.y[i];
+                __syncthreads();
+                return true;
+            }
+        }
+    }
+    // dense system in global scratch, same entries
     for (long long q = threadIdx.x; q < (long long)dim * dim; q += blockDim.x) A[q] = 0.0;
     for (int i = threadIdx.x; i < dim; i += blockDim.x) bx[i] = 1.0;
     __syncthreads();
