@@ -6,10 +6,10 @@
 //                   (IBMNodeClass::interpolate + forceCalc,
 //                   reference src/IBMNode.cpp:26-58)
 //   k_ibm_clear     zero last step's IBM force at its support sites
-//   k_ibm_mark      list the 16x16 lattice tiles touched by any support
-//   k_ibm_spread    one CTA per touched tile: every site of the tile sums the
-//                   contributions of the markers that reach it in marker order
-//                   (the reference's ORDERED reduction, src/IBMNode.cpp:61-94)
+//   k_ibm_mark      list every site that some marker's support touches, once
+//   k_ibm_spread    three listed sites per warp: each sums the contributions
+//                   of the markers that reach it in marker order (the
+//                   reference's ORDERED reduction, src/IBMNode.cpp:61-94)
 //                   without atomics, applies the IBM velocity correction
 //                   (updateMacroscopic, src/IBMNode.cpp:97-136) and collides
 //                   the site again for the next step with the IBM force.
@@ -18,10 +18,9 @@
 #include "collide_cm.cuh"
 #include "ibm_kernels.h"
 #include "lbm_device.cuh"
+#include "lbm_lanes.cuh"
 
 namespace life {
-
-constexpr int TILE = 16;
 
 // One warp per marker: lane s reconstructs support site s, and every lane
 // then adds the nsupp terms in support order (the reference's loop), so the
@@ -75,21 +74,18 @@ __global__ void k_ibm_clear(IbmScratch W, LatDev L) {
     }
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < W.nbodies; b += gridDim.x * blockDim.x)
         W.body_box[b] = make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *W.nsites = 0;
-        *W.ntiles = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *W.nsites = 0;
 }
 
-__global__ void k_ibm_mark(MarkerDev M, IbmScratch W) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= M.n) return;
-    const int ns = M.nsupp[k];
-    for (int s = 0; s < ns; s++) {
-        const int tile = (M.sj[k * 9 + s] / TILE) * W.ntx + (M.si[k * 9 + s] / TILE);
-        if (atomicCAS(&W.tile_flag[tile], 0u, 1u) == 0u) W.tiles[atomicAdd(W.ntiles, 1)] = tile;
-    }
-    if (ns > 0) {
+// One thread per support entry: the first to set a site's bit lists the site.
+__global__ void k_ibm_mark(MarkerDev M, IbmScratch W, LatDev L) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = q / 9, e = q - 9 * k;
+    if (k >= M.n || e >= M.nsupp[k]) return;
+    const long long s = (long long)M.sj[q] * L.pitch + M.si[q];
+    const unsigned bit = 1u << (s & 31);
+    if (!(atomicOr(&W.site_flag[s >> 5], bit) & bit)) W.sites[atomicAdd(W.nsites, 1)] = s;
+    if (e == 0) {
         const int4 bb = M.bbox[k];
         int4* box = W.body_box + W.box_of[k];
         atomicMin(&box->x, bb.x);
@@ -99,127 +95,123 @@ __global__ void k_ibm_mark(MarkerDev M, IbmScratch W) {
     }
 }
 
+// One warp takes three listed sites, nine lanes each (lbm_lanes.cuh). The
+// lanes scan the bodies whose support box reaches one of the sites (in body
+// order) 32 markers at a time for all three sites; a marker that reaches a
+// site leaves its contribution in shared memory, and one lane per site and
+// component adds the chunk's contributions in marker order. The few hundred
+// sites of a body are one warp's work on each SM, not a few warps' on the SMs
+// that own their tiles: with one CTA per touched 16 x 16 tile and one thread
+// per site (a chain of 700-900 FP64 instructions of 64 cycles) the kernel took
+// 44 us for the 126 markers of the 1000 x 400 cylinder (central moments, FP32
+// storage), 26 us now; 41 us for a circle and its tail of 132 markers (BGK,
+// FP64), 13 us now.
+__device__ __forceinline__ bool box_has(const int4& b, int i, int j) {
+    return i >= b.x && i <= b.y && j >= b.z && j <= b.w;
+}
+
 template <bool CM, class S>
-__global__ void __launch_bounds__(256) k_ibm_spread(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
-                                                    LatDev L, int t, MarkerDev M, IbmScratch W) {
-    __shared__ int list[256];
-    __shared__ int warp_cnt[8];
-    // support tables and force factors of the compacted markers
-    __shared__ int s_ij[256][9];
-    __shared__ double s_d[256][9];
-    __shared__ double s_fx[256], s_fy[256];
-    __shared__ int s_ns[256];
-    // touched sites of the tile, compacted onto the first warps
-    __shared__ int s_tij[256];
-    __shared__ double s_tax[256], s_tay[256];
-    __shared__ int s_nt;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+__global__ void __launch_bounds__(32) k_ibm_spread(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
+                                                   LatDev L, int t, MarkerDev M, IbmScratch W) {
+    __shared__ double s_c[kLaneSites][2][32];
+    const int lane = threadIdx.x;
+    const SiteLane g = site_lane();
     t = step_t(L, t);
-    const int ntiles = *W.ntiles;
-    for (int q = blockIdx.x; q < ntiles; q += gridDim.x) {
-        const int tile = W.tiles[q];
-        const int ti0 = (tile % W.ntx) * TILE, tj0 = (tile / W.ntx) * TILE;
-        const int i = ti0 + (tid % TILE), j = tj0 + (tid / TILE);
-        double ax = 0.0, ay = 0.0;
-        bool touched = false;
-        // bodies in body order, markers of a body in marker order: the
-        // contributions to a site are summed in global marker order
-        for (int bi = 0; bi < W.nbodies; bi++) {
-          const int4 box = W.body_box[bi];
-          if (box.x > ti0 + TILE - 1 || box.y < ti0 || box.z > tj0 + TILE - 1 || box.w < tj0) continue;
-          const int kend = W.body_start[bi + 1];
-          for (int c0 = W.body_start[bi]; c0 < kend; c0 += 256) {
-            const int k = c0 + tid;
-            bool hit = false;
-            if (k < kend) {
-                const int4 bb = M.bbox[k];
-                hit = bb.x <= ti0 + TILE - 1 && bb.y >= ti0 && bb.z <= tj0 + TILE - 1 && bb.w >= tj0;
+    const int nsites = *W.nsites;
+    for (int q0 = kLaneSites * (int)blockIdx.x; q0 < nsites; q0 += kLaneSites * (int)gridDim.x) {
+        // this lane's site; a missing one repeats the first and is not stored
+        const bool on = q0 + g.slot < nsites;
+        const long long s = W.sites[on ? q0 + g.slot : q0];
+        const int j = (int)(s / L.pitch), i = (int)(s - (long long)j * L.pitch);
+        int is[kLaneSites], js[kLaneSites];
+#pragma unroll
+        for (int c = 0; c < kLaneSites; c++) {
+            is[c] = __shfl_sync(kAllLanes, i, 9 * c);
+            js[c] = __shfl_sync(kAllLanes, j, 9 * c);
+        }
+        // lanes 0 and 1 of a site sum the x and the y force
+        const int comp = g.v == 1 ? 1 : 0;
+        double acc = 0.0;
+        for (int b0 = 0; b0 < W.nbodies; b0 += 32) {
+            bool near = false;
+            if (b0 + lane < W.nbodies) {
+                const int4 box = W.body_box[b0 + lane];
+                near = box_has(box, is[0], js[0]) || box_has(box, is[1], js[1]) || box_has(box, is[2], js[2]);
             }
-            const unsigned bal = __ballot_sync(0xffffffffu, hit);
-            if (lane == 0) warp_cnt[warp] = __popc(bal);
-            __syncthreads();
-            int off = 0, cnt = 0;
-            for (int w = 0; w < 8; w++) {
-                if (w < warp) off += warp_cnt[w];
-                cnt += warp_cnt[w];
-            }
-            if (hit) {
-                // stage this marker's support (site packed as j*65536 + i)
-                const int r = off + __popc(bal & ((1u << lane) - 1u));
-                list[r] = k;
-                const int ns = M.nsupp[k];
-                s_ns[r] = ns;
-                for (int s = 0; s < 9; s++) {
-                    s_ij[r][s] = s < ns ? (M.sj[k * 9 + s] << 16) | M.si[k * 9 + s] : -1;
-                    s_d[r][s] = M.sd[k * 9 + s];
-                }
-                s_fx[r] = M.force[k * 2 + 0];
-                s_fy[r] = M.force[k * 2 + 1];
-            }
-            __syncthreads();
-            // Marker order within the chunk is preserved by the ordered compaction.
-            const int me = (j << 16) | i;
-            for (int r = 0; r < cnt; r++) {
-                const int ns = s_ns[r];
-                for (int s = 0; s < ns; s++)
-                    if (s_ij[r][s] == me) {
-                        const int m = list[r];
-                        const double d = s_d[r][s];
-                        const double e = M.eps[m], ds = M.ds[m];
-                        ax += s_fx[r] * e * ds * 1.0 * d;
-                        ay += s_fy[r] * e * ds * 1.0 * d;
-                        touched = true;
-                        break;
+            unsigned bodies = __ballot_sync(kAllLanes, near);
+            while (bodies) {
+                const int b = b0 + __ffs(bodies) - 1;
+                bodies &= bodies - 1;
+                const int kend = W.body_start[b + 1];
+                for (int k0 = W.body_start[b]; k0 < kend; k0 += 32) {
+                    const int k = k0 + lane;
+                    int at[kLaneSites];  // this marker's support entry at each site
+                    bool any = false;
+#pragma unroll
+                    for (int c = 0; c < kLaneSites; c++) at[c] = -1;
+                    if (k < kend) {
+                        const int4 bb = M.bbox[k];
+                        if (box_has(bb, is[0], js[0]) || box_has(bb, is[1], js[1]) || box_has(bb, is[2], js[2])) {
+                            const int ns = M.nsupp[k];
+#pragma unroll
+                            for (int e = 8; e >= 0; e--) {
+                                const int ei = M.si[k * 9 + e], ej = M.sj[k * 9 + e];
+#pragma unroll
+                                for (int c = 0; c < kLaneSites; c++)
+                                    if (e < ns && ei == is[c] && ej == js[c]) at[c] = e;
+                            }
+                            any = at[0] >= 0 || at[1] >= 0 || at[2] >= 0;
+                        }
                     }
+                    if (!__any_sync(kAllLanes, any)) continue;
+                    double gx = 0.0, gy = 0.0;
+                    if (any) {
+                        const double e = M.eps[k], ds = M.ds[k];
+                        gx = M.force[k * 2] * e * ds * 1.0;
+                        gy = M.force[k * 2 + 1] * e * ds * 1.0;
+                    }
+                    unsigned hits = 0;
+#pragma unroll
+                    for (int c = 0; c < kLaneSites; c++) {
+                        const unsigned h = __ballot_sync(kAllLanes, at[c] >= 0);
+                        if (c == g.slot) hits = h;
+                        if (at[c] >= 0) {
+                            const double d = M.sd[k * 9 + at[c]];
+                            s_c[c][0][lane] = gx * d;
+                            s_c[c][1][lane] = gy * d;
+                        }
+                    }
+                    __syncwarp();
+                    while (hits) {
+                        acc = acc + s_c[g.slot][comp][__ffs(hits) - 1];
+                        hits &= hits - 1;
+                    }
+                    __syncwarp();
+                }
             }
-            __syncthreads();
-          }
         }
-        if (tid == 0) {
-            W.tile_flag[tile] = 0u;
-            s_nt = 0;
-        }
-        __syncthreads();
-        {
-            const bool mine = touched && i < L.Nx && j < L.Ny;
-            const unsigned bal = __ballot_sync(0xffffffffu, mine);
-            int base = 0;
-            if (lane == 0 && bal) base = atomicAdd(&s_nt, __popc(bal));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (mine) {
-                const int r = base + __popc(bal & ((1u << lane) - 1u));
-                s_tij[r] = (j << 16) | i;
-                s_tax[r] = ax;
-                s_tay[r] = ay;
-            }
-        }
-        __syncthreads();
-        // the long FP64 chains (state, velocity correction, collision) on as
-        // few warps as there are touched sites
-        for (int r = tid; r < s_nt; r += blockDim.x) {
-            const int i = s_tij[r] & 0xffff, j = s_tij[r] >> 16;
-            const double ax = s_tax[r], ay = s_tay[r];
-            const long long s = (long long)j * L.pitch + i;
+        const double ax = lane_get(acc, g.base), ay = lane_get(acc, g.base + 1);
+        const bool store = on && g.store;
+        if (store && g.v == 0) {
             W.force_ibm[s] = ax;
             W.force_ibm[L.S + s] = ay;
-            W.sites[atomicAdd(W.nsites, 1)] = s;
-            double f[9], rho, ux, uy, Fx, Fy;
-            site_state<CM, S>(A, L, t, i, j, f, rho, ux, uy);
-            force_xy_of(L, t, i, j, Fx, Fy);
-            macroscopic_ibm(f, Fx, Fy, ax, ay, rho, ux, uy);
+            atomicAnd(&W.site_flag[s >> 5], ~(1u << (s & 31)));
+        }
+        double Fx, Fy, rho, ux, uy;
+        const double f = lanes_populations<CM, S>(A, L, t, g, i, j, Fx, Fy);
+        lanes_macroscopic(g, f, Fx + ax, Fy + ay, rho, ux, uy);
+        if (store && g.v == 0) {
             store_history(L, site_type(L, i, j), i, j, rho, ux, uy);
             if (L.convective && i >= L.Nx - 3) {
                 const int c = i - (L.Nx - 3);
                 L.outlet_u[((size_t)c * L.Ny + j) * 2 + 0] = ux;
                 L.outlet_u[((size_t)c * L.Ny + j) * 2 + 1] = uy;
             }
-            double Gx, Gy, fs[9];
-            force_xy_next(L, t + 1, rho, Gx, Gy);
-            collide<CM>(f, rho, ux, uy, Gx + ax, Gy + ay, L.omega, L.cs, fs);
-#pragma unroll
-            for (int v = 0; v < 9; v++) B[(size_t)v * L.S + s] = S::save(fs[v], v);
         }
-        __syncthreads();
+        double Gx, Gy;
+        force_xy_next(L, t + 1, rho, Gx, Gy);
+        const double fs = lanes_collide<CM>(g, f, rho, ux, uy, Gx + ax, Gy + ay, L.omega, L.cs);
+        if (store) B[(size_t)g.v * L.S + s] = S::save(fs, g.v);
     }
 }
 
@@ -289,22 +281,25 @@ cudaError_t launch_ibm_interp(const void* P, const LatDev& L, int t, const Marke
     return cudaGetLastError();
 }
 
+cudaError_t launch_ibm_clear(const LatDev& L, const IbmScratch& W, cudaStream_t s) {
+    k_ibm_clear<<<8, 256, 0, s>>>(W, L);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ibm_mark(const LatDev& L, const MarkerDev& M, const IbmScratch& W, cudaStream_t s) {
+    if (M.n == 0) return cudaSuccess;
+    k_ibm_mark<<<(9 * M.n + 127) / 128, 128, 0, s>>>(M, W, L);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_ibm_spread(const void* A, void* B, const LatDev& L, int t, const MarkerDev& M,
                               const IbmScratch& W, cudaStream_t s) {
-    k_ibm_clear<<<8, 256, 0, s>>>(W, L);
-    if (M.n > 0) {
-        k_ibm_mark<<<(M.n + 127) / 128, 128, 0, s>>>(M, W);
-        // four CTAs per SM of this device, at most one per tile
-        static int sms[64] = {0};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev >= 0 && dev < 64 && sms[dev] == 0) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-        const int nsm = (dev >= 0 && dev < 64 && sms[dev] > 0) ? sms[dev] : 1;
-        int grid = W.max_tiles < 4 * nsm ? W.max_tiles : 4 * nsm;
-        if (grid < 1) grid = 1;
-        TypedPtr<void> Ap{A}, Bp{B};
-        IBM_DISPATCH(k_ibm_spread, grid, 256, Ap, Bp, L, t, M, W);
-    }
+    if (M.n == 0) return cudaSuccess;
+    // a warp per three sites, nine sites per marker at most; beyond 4096
+    // blocks (about 27 per SM) a block takes further sites in turn
+    const int grid = 3 * M.n < 4096 ? 3 * M.n : 4096;
+    TypedPtr<void> Ap{A}, Bp{B};
+    IBM_DISPATCH(k_ibm_spread, grid, 32, Ap, Bp, L, t, M, W);
     return cudaGetLastError();
 }
 

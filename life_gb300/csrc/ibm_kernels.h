@@ -22,20 +22,17 @@ struct MarkerDev {
     int* body;      // [n] owning body
 };
 
-// Scratch of the tile-owner spread.
+// Scratch of the spread.
 struct IbmScratch {
     double* force_ibm;        // [2][S] dense IBM force of the current step
     long long* sites;         // support sites written this step
     long long* sites_prev;    // support sites of the previous step
     int* nsites;
     int* nsites_prev;
-    unsigned* tile_flag;      // [ntx*nty]
-    int* tiles;               // touched tiles
-    int* ntiles;
-    int ntx, nty, max_tiles;
+    unsigned* site_flag;      // [S / 32] a bit per site: listed this step (clear between steps)
     // Bodies as contiguous marker ranges [body_start[b], body_start[b+1])
     // and the bounding box of their support this step (imin, imax, jmin,
-    // jmax): a tile of the spread scans only the bodies whose box reaches it.
+    // jmax): a site of the spread scans only the bodies whose box reaches it.
     int nbodies;
     const int* body_start;    // [nbodies + 1]
     const int* box_of;        // [n] the range of each marker
@@ -50,6 +47,10 @@ cudaError_t launch_overlap_pairs(const double* pos, int nm, double Dx, int* coun
 // With t_dev, the step is read from device memory when the kernel runs.
 cudaError_t launch_ibm_interp(const void* P, const LatDev& L, int t, const MarkerDev& M, double velScale,
                               cudaStream_t s, const int* t_dev = nullptr);
+// A step's spread: clear (before mark), mark (after the last interpolation),
+// spread (after the lattice step). The first two touch no populations.
+cudaError_t launch_ibm_clear(const LatDev& L, const IbmScratch& W, cudaStream_t s);
+cudaError_t launch_ibm_mark(const LatDev& L, const MarkerDev& M, const IbmScratch& W, cudaStream_t s);
 cudaError_t launch_ibm_spread(const void* A, void* B, const LatDev& L, int t, const MarkerDev& M,
                               const IbmScratch& W, cudaStream_t s);
 

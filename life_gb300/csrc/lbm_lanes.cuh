@@ -177,14 +177,12 @@ __device__ __forceinline__ double lanes_regularised(const SiteLane& g, double f,
     return on ? reg : f;
 }
 
-// site_state() of the warp's three sites: this lane's population after the
-// boundary condition and the site's moments (equal on the site's lanes).
+// The first half of site_state() for the warp's three sites: this lane's
+// population after the boundary condition, and the step's force at the site.
 template <bool CM, class S>
-__device__ __forceinline__ void lanes_state(const typename S::T* __restrict__ P, const LatDev& L, int t,
-                                            const SiteLane& g, int i, int j, double& f, double& rho, double& ux,
-                                            double& uy) {
-    f = lanes_gather<S>(P, L, g, i, j);
-    double Fx, Fy;
+__device__ __forceinline__ double lanes_populations(const typename S::T* __restrict__ P, const LatDev& L, int t,
+                                                    const SiteLane& g, int i, int j, double& Fx, double& Fy) {
+    double f = lanes_gather<S>(P, L, g, i, j);
     force_xy_of(L, t, i, j, Fx, Fy);
     const int type = site_type(L, i, j);
     if (__any_sync(kAllLanes, type == LIFE_CONVECTIVE)) {
@@ -238,6 +236,17 @@ __device__ __forceinline__ void lanes_state(const typename S::T* __restrict__ P,
         }
         f = lanes_regularised<CM>(g, f, reg, type, nx, ny, nd, rn, u0, u1, L, r1, r2);
     }
+    return f;
+}
+
+// site_state() of the warp's three sites: this lane's population after the
+// boundary condition and the site's moments (equal on the site's lanes).
+template <bool CM, class S>
+__device__ __forceinline__ void lanes_state(const typename S::T* __restrict__ P, const LatDev& L, int t,
+                                            const SiteLane& g, int i, int j, double& f, double& rho, double& ux,
+                                            double& uy) {
+    double Fx, Fy;
+    f = lanes_populations<CM, S>(P, L, t, g, i, j, Fx, Fy);
     lanes_macroscopic(g, f, Fx, Fy, rho, ux, uy);
 }
 
