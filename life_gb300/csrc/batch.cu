@@ -205,12 +205,12 @@ static int refill_steps(LifeBatch* b, int n, int ahead = 1) {
 
 // Captures batch steps from the cases' current state and advances the host
 // view of every case by them (t, buffer parity, IBM scratch parity).
-// Per case, the convective outlet and the boundary perimeter run on the
-// case's side stream; the interior launch waits only for the outlets (the
-// perimeter and the interior both read P[cur] and write disjoint sites of
-// P[cur^1], so they overlap). The IBM forces (interpolation, or the FSI
-// subiteration loop) read only P[cur] and run beside the lattice step on the
-// case's aux stream after the outlet; the spread waits for all of them.
+// Per case, the boundary perimeter runs on the case's side stream beside the
+// interior launch (both read P[cur] and write disjoint sites of P[cur^1]). The
+// IBM forces (interpolation, or the FSI subiteration loop) read only P[cur]
+// and run beside the lattice step on the case's aux stream; the spread waits
+// for all of them. Where a kernel forms the convective outlet's speed term,
+// it comes before whatever reads it (LatDev::outlet_form).
 static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* out, int* kernels) {
     cudaStream_t bs = b->stream;
     const int n = (int)b->cases.size();
@@ -227,15 +227,16 @@ static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* o
             const int tt = c->t + 1;
             const LatDev L = lattice_view(c, tt);
             e = cudaStreamWaitEvent(c->side, b->ev_fork, 0);
-            // the outlet reads the outlet columns before the interior rewrites them
-            if (e == cudaSuccess && L.convective) e = launch_outlet(L, c->d_delU, c->side);
-            if (e == cudaSuccess) e = cudaEventRecord(c->ev_out, c->side);
-            if (e == cudaSuccess && L.convective) e = cudaStreamWaitEvent(bs, c->ev_out, 0);
             const bool fused = fused_step(b);  // perimeter inside the interior launch
+            if (L.convective && L.outlet_form == kOutletKernel) {
+                if (e == cudaSuccess) e = launch_outlet(L, c->d_delU, c->side);
+                if (e == cudaSuccess) e = cudaEventRecord(c->ev_out, c->side);
+                if (e == cudaSuccess && fused) e = cudaStreamWaitEvent(bs, c->ev_out, 0);
+            }
             if (e == cudaSuccess && !fused) e = launch_perimeter(c->P[c->cur], c->P[c->cur ^ 1], L, tt, c->side);
             if (e == cudaSuccess) e = cudaEventRecord(c->ev_join, c->side);
             if (e == cudaSuccess && c->obj.hasIBM) {
-                e = cudaStreamWaitEvent(c->aux, c->ev_out, 0);
+                e = cudaStreamWaitEvent(c->aux, L.outlet_form == kOutletKernel && L.convective ? c->ev_out : b->ev_fork, 0);
                 if (e == cudaSuccess) rc = ibm_forces(c, tt, c->P[c->cur], c->aux);
                 if (e == cudaSuccess && rc == LIFE_OK) e = cudaEventRecord(c->ev_aux, c->aux);
             }
@@ -308,6 +309,7 @@ static void rewind_host_view(LifeBatch* b) {
         if (adv & 1) {
             std::swap(c->W.sites, c->W.sites_prev);
             std::swap(c->W.nsites, c->W.nsites_prev);
+            std::swap(c->W.body_box, c->W.body_box_next);
         }
     }
 }
@@ -421,6 +423,7 @@ static int run_batch(LifeBatch* b, int nsteps, cudaEvent_t start, cudaEvent_t st
             if (c->obj.hasIBM && (m & 1)) {
                 std::swap(c->W.sites, c->W.sites_prev);
                 std::swap(c->W.nsites, c->W.nsites_prev);
+                std::swap(c->W.body_box, c->W.body_box_next);
             }
         }
         s += m;

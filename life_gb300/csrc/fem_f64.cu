@@ -1724,7 +1724,7 @@ cudaError_t launch_fsi_subiteration(const FsiDev& F, const MarkerDev& M, const v
     k_fsi_support<<<(F.nFlexMarkers + 3) / 4, 128, 0, s>>>(F, M);
     if (F.uni) k_fsi_epsilon_uni<<<1, 256, kEpsSmemDoubles * sizeof(double), s>>>(F, M);
     else k_fsi_epsilon_body<<<F.nFlex, 256, kEpsSmemDoubles * sizeof(double), s>>>(F, M);
-    cudaError_t e = launch_ibm_interp(P, L, t, M, velScale, s, cond ? &F.s->t : nullptr);
+    cudaError_t e = launch_ibm_interp(P, L, t, M, nullptr, velScale, s, cond ? &F.s->t : nullptr);
     if (e != cudaSuccess) return e;
     k_fem_dynamic<<<F.nFlex, 256, F.fem_smem, s>>>(F, M);
     k_fsi_residual<<<1, 32, 0, s>>>(F, cond ? *cond : cudaGraphConditionalHandle{}, cond ? 1 : 0);

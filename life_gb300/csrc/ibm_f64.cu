@@ -5,8 +5,9 @@
 //                   kernel computed them), then the direct force
 //                   (IBMNodeClass::interpolate + forceCalc,
 //                   reference src/IBMNode.cpp:26-58)
-//   k_ibm_clear     zero last step's IBM force at its support sites
-//   k_ibm_mark      list every site that some marker's support touches, once
+//   k_ibm_mark      list every site that some marker's support touches, once,
+//                   and zero last step's IBM force at its support sites (for
+//                   rigid markers the interpolation's warps do this)
 //   k_ibm_spread    three listed sites per warp: each sums the contributions
 //                   of the markers that reach it in marker order (the
 //                   reference's ORDERED reduction, src/IBMNode.cpp:61-94)
@@ -22,26 +23,72 @@
 
 namespace life {
 
+// Zero last step's IBM force at its support sites (thread q of `threads`).
+__device__ __forceinline__ void clear_force(const IbmScratch& W, const LatDev& L, int q, int threads) {
+    const int n = *W.nsites_prev;
+    for (; q < n; q += threads) {
+        const long long s = W.sites_prev[q];
+        W.force_ibm[s] = 0.0;
+        W.force_ibm[L.S + s] = 0.0;
+    }
+}
+
+// List the support site (i, j), if no other entry has, and widen the body's
+// support box by the marker's (once per marker: `first`).
+__device__ __forceinline__ void mark_site(const IbmScratch& W, const LatDev& L, int k, int i, int j, bool first,
+                                          const int4& bb) {
+    const long long s = (long long)j * L.pitch + i;
+    const unsigned bit = 1u << (s & 31);
+    if (!(atomicOr(&W.site_flag[s >> 5], bit) & bit)) W.sites[atomicAdd(W.nsites, 1)] = s;
+    if (first) {
+        int4* box = W.body_box + W.box_of[k];
+        atomicMin(&box->x, bb.x);
+        atomicMax(&box->y, bb.y);
+        atomicMin(&box->z, bb.z);
+        atomicMax(&box->w, bb.w);
+    }
+}
+
 // One warp per marker: lane s reconstructs support site s, and every lane
 // then adds the nsupp terms in support order (the reference's loop), so the
 // sums are formed exactly as in a sequential loop while the nine site states
-// are computed side by side.
-template <bool CM, class S>
+// are computed side by side. MARK: also the work of k_ibm_mark (the markers do
+// not move before the spread).
+template <bool CM, class S, bool MARK>
 __global__ void __launch_bounds__(128) k_ibm_interp(const typename S::T* __restrict__ P, LatDev L, int t, MarkerDev M,
-                                                    double velScale, const int* __restrict__ t_dev) {
+                                                    IbmScratch W, double velScale, const int* __restrict__ t_dev) {
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
+    if (MARK) clear_force(W, L, (int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(gridDim.x * blockDim.x));
     if (k >= M.n) return;  // uniform per warp
     t = t_dev ? *t_dev : step_t(L, t);  // inside a replayed graph the step comes from the device
     const int ns = M.nsupp[k];
-    double tr = 0.0, tx = 0.0, ty = 0.0;
+    const bool act = lane < ns;
     int i = 0, j = 0;
-    if (lane < ns) {
+    if (act) {
         i = M.si[k * 9 + lane];
         j = M.sj[k * 9 + lane];
+    }
+    const int imin = __reduce_min_sync(0xffffffffu, act ? i : (1 << 30));
+    const int imax = __reduce_max_sync(0xffffffffu, act ? i : -(1 << 30));
+    const int jmin = __reduce_min_sync(0xffffffffu, act ? j : (1 << 30));
+    const int jmax = __reduce_max_sync(0xffffffffu, act ? j : -(1 << 30));
+    const int4 bb = make_int4(imin, imax, jmin, jmax);
+    if (lane == 0) M.bbox[k] = bb;
+    if (MARK && act) mark_site(W, L, k, i, j, lane == 0, bb);
+    // support sites on a convective outlet: its speed term, formed here too
+    // (nothing of this step has to be finished before the interpolation)
+    double dU[2] = {0.0, 0.0};
+    const bool form = L.convective && L.outlet_form == kOutletSites;
+    if (form && imax == L.Nx - 1) {
+        const double uOut = lanes_outlet_mean<S::prec == LIFE_PREC_F64>(L);
+        if (act) outlet_term(L, uOut, j, dU[0], dU[1]);
+    }
+    double tr = 0.0, tx = 0.0, ty = 0.0;
+    if (act) {
         const double d = M.sd[k * 9 + lane];
         double f[9], rho, ux, uy;
-        site_state<CM, S>(P, L, t, i, j, f, rho, ux, uy);
+        site_state<CM, S>(P, L, t, i, j, f, rho, ux, uy, form ? dU : nullptr);
         tr = rho * d * 1.0 * 1.0;
         tx = rho * ux * d * 1.0 * 1.0;
         ty = rho * uy * d * 1.0 * 1.0;
@@ -52,47 +99,20 @@ __global__ void __launch_bounds__(128) k_ibm_interp(const typename S::T* __restr
         iMx += __shfl_sync(0xffffffffu, tx, q);
         iMy += __shfl_sync(0xffffffffu, ty, q);
     }
-    const bool act = lane < ns;
-    const int imin = __reduce_min_sync(0xffffffffu, act ? i : (1 << 30));
-    const int imax = __reduce_max_sync(0xffffffffu, act ? i : -(1 << 30));
-    const int jmin = __reduce_min_sync(0xffffffffu, act ? j : (1 << 30));
-    const int jmax = __reduce_max_sync(0xffffffffu, act ? j : -(1 << 30));
     if (lane == 0) {
         const double sc = velScale * iRho;
         M.force[k * 2 + 0] = 2.0 * (sc * M.vel[k * 2 + 0] - iMx);
         M.force[k * 2 + 1] = 2.0 * (sc * M.vel[k * 2 + 1] - iMy);
-        M.bbox[k] = make_int4(imin, imax, jmin, jmax);
     }
-}
-
-__global__ void k_ibm_clear(IbmScratch W, LatDev L) {
-    const int n = *W.nsites_prev;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        const long long s = W.sites_prev[q];
-        W.force_ibm[s] = 0.0;
-        W.force_ibm[L.S + s] = 0.0;
-    }
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < W.nbodies; b += gridDim.x * blockDim.x)
-        W.body_box[b] = make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *W.nsites = 0;
 }
 
 // One thread per support entry: the first to set a site's bit lists the site.
 __global__ void k_ibm_mark(MarkerDev M, IbmScratch W, LatDev L) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    clear_force(W, L, q, (int)(gridDim.x * blockDim.x));
     const int k = q / 9, e = q - 9 * k;
     if (k >= M.n || e >= M.nsupp[k]) return;
-    const long long s = (long long)M.sj[q] * L.pitch + M.si[q];
-    const unsigned bit = 1u << (s & 31);
-    if (!(atomicOr(&W.site_flag[s >> 5], bit) & bit)) W.sites[atomicAdd(W.nsites, 1)] = s;
-    if (e == 0) {
-        const int4 bb = M.bbox[k];
-        int4* box = W.body_box + W.box_of[k];
-        atomicMin(&box->x, bb.x);
-        atomicMax(&box->y, bb.y);
-        atomicMin(&box->z, bb.z);
-        atomicMax(&box->w, bb.w);
-    }
+    mark_site(W, L, k, M.si[q], M.sj[q], e == 0, M.bbox[k]);
 }
 
 // One warp takes three listed sites, nine lanes each (lbm_lanes.cuh). The
@@ -118,6 +138,12 @@ __global__ void __launch_bounds__(32) k_ibm_spread(const typename S::T* __restri
     const SiteLane g = site_lane();
     t = step_t(L, t);
     const int nsites = *W.nsites;
+    // the next step's list starts empty
+    if (blockIdx.x == 0) {
+        if (lane == 0) *W.nsites_prev = 0;
+        for (int b = lane; b < W.nbodies; b += 32)
+            W.body_box_next[b] = make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff);
+    }
     for (int q0 = kLaneSites * (int)blockIdx.x; q0 < nsites; q0 += kLaneSites * (int)gridDim.x) {
         // this lane's site; a missing one repeats the first and is not stored
         const bool on = q0 + g.slot < nsites;
@@ -272,17 +298,27 @@ struct TypedPtr {
     operator U*() const { return (U*)const_cast<void*>(p); }
 };
 
-cudaError_t launch_ibm_interp(const void* P, const LatDev& L, int t, const MarkerDev& M, double velScale,
-                              cudaStream_t s, const int* t_dev) {
+cudaError_t launch_ibm_interp(const void* P, const LatDev& L, int t, const MarkerDev& M, const IbmScratch* mark,
+                              double velScale, cudaStream_t s, const int* t_dev) {
     if (M.n == 0) return cudaSuccess;
     const int nb = (M.n + 3) / 4;  // one warp per marker
     TypedPtr<void> Pp{P};
-    IBM_DISPATCH(k_ibm_interp, nb, 128, Pp, L, t, M, velScale, t_dev);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_ibm_clear(const LatDev& L, const IbmScratch& W, cudaStream_t s) {
-    k_ibm_clear<<<8, 256, 0, s>>>(W, L);
+#define LIFE_INTERP(CM, S)                                                                              \
+    do {                                                                                                \
+        if (mark) k_ibm_interp<CM, S, true><<<nb, 128, 0, s>>>(Pp, L, t, M, *mark, velScale, t_dev);     \
+        else k_ibm_interp<CM, S, false><<<nb, 128, 0, s>>>(Pp, L, t, M, IbmScratch{}, velScale, t_dev);  \
+    } while (0)
+    if (L.prec == LIFE_PREC_F64) {
+        if (L.cm) LIFE_INTERP(true, StoreF64);
+        else LIFE_INTERP(false, StoreF64);
+    } else if (L.prec == LIFE_PREC_F32) {
+        if (L.cm) LIFE_INTERP(true, StoreF32);
+        else LIFE_INTERP(false, StoreF32);
+    } else {
+        if (L.cm) LIFE_INTERP(true, StoreF16);
+        else LIFE_INTERP(false, StoreF16);
+    }
+#undef LIFE_INTERP
     return cudaGetLastError();
 }
 

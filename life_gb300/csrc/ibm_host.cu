@@ -145,8 +145,10 @@ int upload_markers(LifeCase* c) {
         for (int k = start[r]; k < start[r + 1]; k++) box_of[k] = r;
     int *d_start = nullptr, *d_box_of = nullptr;
     if ((rc = alloc_t(c, &d_start, start.size())) || (rc = alloc_t(c, &d_box_of, box_of.size())) ||
-        (rc = alloc_t(c, &W.body_box, (size_t)W.nbodies)))
+        (rc = alloc_t(c, &W.body_box, (size_t)W.nbodies)) || (rc = alloc_t(c, &W.body_box_next, (size_t)W.nbodies)))
         return rc;
+    const std::vector<int4> empty((size_t)W.nbodies, make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff));
+    CK(cudaMemcpyAsync(W.body_box, empty.data(), sizeof(int4) * empty.size(), cudaMemcpyHostToDevice, c->stream));
     W.body_start = d_start;
     W.box_of = d_box_of;
     CK(cudaMemcpyAsync(d_start, start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice, c->stream));
@@ -165,21 +167,16 @@ int upload_markers(LifeCase* c) {
 // forces (interpolation and forceCalc, or the whole FSI subiteration loop)
 // read only the step's input populations A, so they can run beside the
 // lattice step; the spread writes the support sites of B and follows both.
-// The list of support sites belongs to the first part where the markers are
-// rigid. After a loop it comes with the spread: a kernel node behind a loop
+// Rigid markers' interpolation also lists the support sites. After a loop
+// the list comes with the spread: a kernel node behind a loop
 // node in its branch of the step graph keeps the loops of a batch's cases from
 // running side by side (64 cases, 27 with loops: 6.2 ms a step against 1.8).
 int ibm_forces(LifeCase* c, int t, const void* A, cudaStream_t s) {
     LatDev L = lattice_view(c, t);
-    cudaError_t e = launch_ibm_clear(L, c->W, s);
-    if (e != cudaSuccess) return cuda_fail(e, "ibm_clear");
-    c->ibm_launches += 1;
     if (c->obj.hasFlex) return fem_fsi_loop(c, t, A, L, s);
-    e = launch_ibm_interp(A, L, t, c->M, c->Dt / c->Dx, s);
+    cudaError_t e = launch_ibm_interp(A, L, t, c->M, &c->W, c->Dt / c->Dx, s);
     if (e != cudaSuccess) return cuda_fail(e, "ibm_interp");
-    e = launch_ibm_mark(L, c->M, c->W, s);
-    if (e != cudaSuccess) return cuda_fail(e, "ibm_mark");
-    c->ibm_launches += 2;
+    c->ibm_launches += 1;
     return LIFE_OK;
 }
 
@@ -196,6 +193,7 @@ int ibm_apply(LifeCase* c, int t, const void* A, void* B, cudaStream_t s) {
     c->ibm_launches += 1;
     std::swap(c->W.sites, c->W.sites_prev);
     std::swap(c->W.nsites, c->W.nsites_prev);
+    std::swap(c->W.body_box, c->W.body_box_next);
     return LIFE_OK;
 }
 

@@ -37,6 +37,7 @@ struct IbmScratch {
     const int* body_start;    // [nbodies + 1]
     const int* box_of;        // [n] the range of each marker
     int4* body_box;           // [nbodies]
+    int4* body_box_next;      // [nbodies] the other of two, reset by this step's spread
 };
 
 // Close marker pairs of removeOverlapMarkers (appended unordered, see
@@ -44,12 +45,12 @@ struct IbmScratch {
 cudaError_t launch_overlap_pairs(const double* pos, int nm, double Dx, int* count, int2* out, int cap,
                                  cudaStream_t s);
 // Population buffers are untyped; their element type follows L.prec.
-// With t_dev, the step is read from device memory when the kernel runs.
-cudaError_t launch_ibm_interp(const void* P, const LatDev& L, int t, const MarkerDev& M, double velScale,
-                              cudaStream_t s, const int* t_dev = nullptr);
-// A step's spread: clear (before mark), mark (after the last interpolation),
-// spread (after the lattice step). The first two touch no populations.
-cudaError_t launch_ibm_clear(const LatDev& L, const IbmScratch& W, cudaStream_t s);
+// With t_dev, the step is read from device memory when the kernel runs. With
+// `mark`, the launch also does the work of launch_ibm_mark.
+cudaError_t launch_ibm_interp(const void* P, const LatDev& L, int t, const MarkerDev& M, const IbmScratch* mark,
+                              double velScale, cudaStream_t s, const int* t_dev = nullptr);
+// The list of support sites (after the step's last interpolation; it touches
+// no populations), and the spread (after the list and the lattice step).
 cudaError_t launch_ibm_mark(const LatDev& L, const MarkerDev& M, const IbmScratch& W, cudaStream_t s);
 cudaError_t launch_ibm_spread(const void* A, void* B, const LatDev& L, int t, const MarkerDev& M,
                               const IbmScratch& W, cudaStream_t s);

@@ -457,13 +457,70 @@ __device__ __forceinline__ void regularised(double f[9], int type, int nx, int n
     }
 }
 
+constexpr int kOutletThreads = 256;  // of k_outlet_f64
+
+// The mean outlet speed of k_outlet_f64, formed by one warp with the same
+// additions in the same order: sequential over j for FP64 storage (32 values
+// loaded at a time), for the others the strided partial sums of its threads,
+// each warp's tree, and the warp sums in order.
+template <bool F64>
+__device__ __forceinline__ double lanes_outlet_mean(const LatDev& L) {
+    const int lane = (int)threadIdx.x & 31, Ny = L.Ny;
+    const double* u1 = L.outlet_u_prev + (size_t)2 * Ny * 2;  // column Nx-1
+    double acc = 0.0;
+    if (F64) {
+        double next = lane < Ny ? u1[lane * 2] : 0.0;
+        for (int j0 = 0; j0 < Ny; j0 += 32) {
+            const double x = next;
+            const int jn = j0 + 32 + lane, m = Ny - j0 < 32 ? Ny - j0 : 32;
+            if (jn < Ny) next = u1[jn * 2];
+            if (m == 32) {
+#pragma unroll
+                for (int q = 0; q < 32; q++) acc += __shfl_sync(0xffffffffu, x, q);
+            } else {
+                for (int q = 0; q < m; q++) acc += __shfl_sync(0xffffffffu, x, q);
+            }
+        }
+        return acc / (double)Ny;
+    }
+    // (the eight warps' sums side by side: their loads are in flight together)
+    constexpr int kWarps = kOutletThreads / 32;
+    double part[kWarps];
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) part[w] = 0.0;
+    for (int j0 = lane; j0 < Ny; j0 += kOutletThreads) {
+        double x[kWarps];
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) x[w] = j0 + 32 * w < Ny ? u1[(j0 + 32 * w) * 2] : 0.0;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) part[w] = j0 + 32 * w < Ny ? part[w] + x[w] : part[w];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) part[w] += __shfl_down_sync(0xffffffffu, part[w], o);
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) acc += __shfl_sync(0xffffffffu, part[w], 0);
+    return acc / (double)Ny;
+}
+
+// The outlet's speed term at row j from the mean (src/Grid.cpp:488-494).
+__device__ __forceinline__ void outlet_term(const LatDev& L, double uOut, int j, double& dU0, double& dU1) {
+    const double2* u = reinterpret_cast<const double2*>(L.outlet_u_prev) + j;
+    const double2 u3 = u[0], u2 = u[L.Ny], u1 = u[2 * L.Ny];  // columns Nx-3, Nx-2, Nx-1
+    dU0 = (-uOut / 2.0) * (3.0 * u1.x - 4.0 * u2.x + u3.x);
+    dU1 = (-uOut / 2.0) * (3.0 * u1.y - 4.0 * u2.y + u3.y);
+}
+
 // The reference state of step t at site (i,j): post-stream populations after
 // the boundary condition (GridClass::applyBCs, src/Grid.cpp:302-384;
 // convectiveBC :468-474) and the macroscopic moments (without the IBM
-// correction, which support sites receive afterwards).
+// correction, which support sites receive afterwards). dU: the outlet's speed
+// term at row j, where the caller forms it (otherwise it is read from delU).
 template <bool CM, class S>
 __device__ __forceinline__ void site_state(const typename S::T* __restrict__ P, const LatDev& L, int t, int i, int j,
-                                           double f[9], double& rho, double& ux, double& uy) {
+                                           double f[9], double& rho, double& ux, double& uy,
+                                           const double* dU = nullptr) {
     gather<S>(P, L, i, j, f);
     double Fx, Fy;
     force_xy_of(L, t, i, j, Fx, Fy);
@@ -471,7 +528,7 @@ __device__ __forceinline__ void site_state(const typename S::T* __restrict__ P, 
     if (type != LIFE_FLUID) {
         if (type == LIFE_CONVECTIVE) {
             const double* fp = L.outlet_f_prev + (size_t)j * 3;
-            const double dU0 = L.delU[j * 2 + 0], dU1 = L.delU[j * 2 + 1];
+            const double dU0 = dU ? dU[0] : L.delU[j * 2 + 0], dU1 = dU ? dU[1] : L.delU[j * 2 + 1];
             f[2] = fp[0] + 3.0 * wgt(2) * (dU0 * cx_of(2) + dU1 * cy_of(2));
             f[6] = fp[1] + 3.0 * wgt(6) * (dU0 * cx_of(6) + dU1 * cy_of(6));
             f[8] = fp[2] + 3.0 * wgt(8) * (dU0 * cx_of(8) + dU1 * cy_of(8));

@@ -173,13 +173,13 @@ __global__ void __launch_bounds__(32) k_perimeter(const typename S::T* __restric
 
 // GridClass::convectiveSpeed (src/Grid.cpp:477-495): the mean outlet speed is
 // a sequential sum over j, as in the reference.
-__global__ void k_outlet_f64(LatDev L, double* __restrict__ delU) {
+__global__ void __launch_bounds__(kOutletThreads) k_outlet_f64(LatDev L, double* __restrict__ delU) {
     __shared__ double uOut_s;
     __shared__ double col[1024];
     const int Ny = L.Ny;
-    const double* u1 = L.outlet_u + (size_t)2 * Ny * 2;  // column Nx-1
-    const double* u2 = L.outlet_u + (size_t)1 * Ny * 2;  // column Nx-2
-    const double* u3 = L.outlet_u;                       // column Nx-3
+    const double* u1 = L.outlet_u_prev + (size_t)2 * Ny * 2;  // column Nx-1
+    const double* u2 = L.outlet_u_prev + (size_t)1 * Ny * 2;  // column Nx-2
+    const double* u3 = L.outlet_u_prev;                       // column Nx-3
     if (L.prec != LIFE_PREC_F64) {
         // Reduced-precision forms (whose state is not the reference's bits):
         // a tree sum in a fixed order (strided per thread, then the warps,
@@ -541,7 +541,7 @@ cudaError_t launch_perimeter(const void* A, void* B, const LatDev& L, int t, cud
 }
 
 cudaError_t launch_outlet(const LatDev& L, double* delU, cudaStream_t s) {
-    k_outlet_f64<<<1, 256, 0, s>>>(L, delU);
+    k_outlet_f64<<<1, kOutletThreads, 0, s>>>(L, delU);
     return cudaGetLastError();
 }
 

@@ -179,17 +179,36 @@ __device__ __forceinline__ double lanes_regularised(const SiteLane& g, double f,
 
 // The first half of site_state() for the warp's three sites: this lane's
 // population after the boundary condition, and the step's force at the site.
-template <bool CM, class S>
+// STEP: called for a step (the outlet's speed term may have to be formed here,
+// LatDev::outlet_form), not for a state already reached.
+//
+// The outlet's mean used to be a kernel of its own that everything waited for:
+// 6 us of the 23 us step of a 1501 x 703 FP32 channel, 13-21 us with FP64
+// storage and 400 rows (a sum in order).
+template <bool CM, class S, bool STEP = false>
 __device__ __forceinline__ double lanes_populations(const typename S::T* __restrict__ P, const LatDev& L, int t,
                                                     const SiteLane& g, int i, int j, double& Fx, double& Fy) {
     double f = lanes_gather<S>(P, L, g, i, j);
     force_xy_of(L, t, i, j, Fx, Fy);
     const int type = site_type(L, i, j);
     if (__any_sync(kAllLanes, type == LIFE_CONVECTIVE)) {
+        double dU0 = 0.0, dU1 = 0.0;
+        if (STEP && L.outlet_form == kOutletSites) {
+            const double uOut = lanes_outlet_mean<S::prec == LIFE_PREC_F64>(L);
+            if (type == LIFE_CONVECTIVE) {
+                outlet_term(L, uOut, j, dU0, dU1);
+                if (g.store && g.v == 0) {
+                    L.delU[j * 2 + 0] = dU0;
+                    L.delU[j * 2 + 1] = dU1;
+                }
+            }
+        } else if (type == LIFE_CONVECTIVE) {
+            dU0 = L.delU[j * 2 + 0];
+            dU1 = L.delU[j * 2 + 1];
+        }
         if (type == LIFE_CONVECTIVE && g.cx < 0) {
             const int k = g.v == 2 ? 0 : (g.v == 6 ? 1 : 2);
-            f = L.outlet_f_prev[(size_t)j * 3 + k] +
-                3.0 * wgt(g.v) * (L.delU[j * 2 + 0] * (double)g.cx + L.delU[j * 2 + 1] * (double)g.cy);
+            f = L.outlet_f_prev[(size_t)j * 3 + k] + 3.0 * wgt(g.v) * (dU0 * (double)g.cx + dU1 * (double)g.cy);
         }
     }
     const bool reg = type != LIFE_FLUID && type != LIFE_CONVECTIVE;
@@ -241,12 +260,12 @@ __device__ __forceinline__ double lanes_populations(const typename S::T* __restr
 
 // site_state() of the warp's three sites: this lane's population after the
 // boundary condition and the site's moments (equal on the site's lanes).
-template <bool CM, class S>
+template <bool CM, class S, bool STEP = false>
 __device__ __forceinline__ void lanes_state(const typename S::T* __restrict__ P, const LatDev& L, int t,
                                             const SiteLane& g, int i, int j, double& f, double& rho, double& ux,
                                             double& uy) {
     double Fx, Fy;
-    f = lanes_populations<CM, S>(P, L, t, g, i, j, Fx, Fy);
+    f = lanes_populations<CM, S, STEP>(P, L, t, g, i, j, Fx, Fy);
     lanes_macroscopic(g, f, Fx, Fy, rho, ux, uy);
 }
 
@@ -324,7 +343,7 @@ __device__ __forceinline__ void lanes_perimeter(const typename S::T* __restrict_
     if (!__any_sync(kAllLanes, type != LIFE_FLUID)) return;
     const bool store = g.store && type != LIFE_FLUID;
     double f, rho, ux, uy;
-    lanes_state<CM, S>(A, L, t, g, i, j, f, rho, ux, uy);
+    lanes_state<CM, S, true>(A, L, t, g, i, j, f, rho, ux, uy);
     if (store && L.convective) {
         const int c = i - (L.Nx - 3);
         if (c >= 0 && g.v == 0) {

@@ -210,10 +210,14 @@ LatDev life::lattice_view(const LifeCase* c, int t) {
     L.steps = c->d_steps;
     L.u_in = c->d_u_in;
     L.rho_in = c->d_rho_in;
-    L.outlet_u = c->d_outlet_u;
+    L.outlet_u_prev = c->d_outlet_u[(t - 1) & 1];
+    L.outlet_u = c->d_outlet_u[t & 1];
     L.outlet_f_prev = c->d_outlet_f[(t - 1) & 1];
     L.outlet_f_next = c->d_outlet_f[t & 1];
     L.delU = c->d_delU;
+    // (the one-launch step kernels hold boundary sites one per thread, which
+    // read a finished delU)
+    L.outlet_form = case_fused_step(c) ? kOutletKernel : kOutletSites;
     L.force_ibm = c->W.force_ibm;
     L.t_dev = c->t_dev;
     L.t_off = c->t_off;
@@ -383,7 +387,8 @@ extern "C" int life_case_create(const LifeCaseParams* params, const LifeBodyDesc
     const size_t plane = (size_t)c->S;
     if ((rc = dev_alloc(c, &c->P[0], plane * 9 * c->elem)) || (rc = dev_alloc(c, &c->P[1], plane * 9 * c->elem)) ||
         (rc = dev_alloc_t(c, &c->d_u_in, (size_t)p.Ny * 2)) || (rc = dev_alloc_t(c, &c->d_rho_in, (size_t)p.Ny)) ||
-        (rc = dev_alloc_t(c, &c->d_outlet_u, (size_t)3 * p.Ny * 2)) ||
+        (rc = dev_alloc_t(c, &c->d_outlet_u[0], (size_t)3 * p.Ny * 2)) ||
+        (rc = dev_alloc_t(c, &c->d_outlet_u[1], (size_t)3 * p.Ny * 2)) ||
         (rc = dev_alloc_t(c, &c->d_outlet_f[0], (size_t)p.Ny * 3)) ||
         (rc = dev_alloc_t(c, &c->d_outlet_f[1], (size_t)p.Ny * 3)) ||
         (rc = dev_alloc_t(c, &c->d_delU, (size_t)p.Ny * 2)) || (rc = dev_alloc_t(c, &c->d_red, 4)) ||
@@ -494,7 +499,7 @@ static int run_steps(LifeCase* c, int nsteps, StepTiming* tm) {
         const void* A = c->P[c->cur];
         void* B = c->P[c->cur ^ 1];
         cudaError_t e;
-        if (conv) {
+        if (conv && L.outlet_form == kOutletKernel) {
             e = launch_outlet(L, c->d_delU, c->stream);
             if (e != cudaSuccess) return cuda_fail(e, "outlet");
             if (tm) tm->launches++;

@@ -70,7 +70,7 @@ struct LifeCase {
     double* d_rho_in = nullptr;
     life::StepScalars* d_steps = nullptr;
     int steps_cap = 0, steps_n = 0;
-    double* d_outlet_u = nullptr;
+    double* d_outlet_u[2] = {nullptr, nullptr};
     double* d_outlet_f[2] = {nullptr, nullptr};
     double* d_delU = nullptr;
     // densities after alternate steps (WOMERSLEY with gravity only) and the

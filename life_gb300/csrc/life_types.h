@@ -47,10 +47,12 @@ struct LatDev {
     // Convective outlet side state (reference GridClass::convectiveSpeed,
     // src/Grid.cpp:477-495, reads u of the previous step at the last three
     // columns; convectiveBC reads f_n[2,6,8] at the outlet column).
-    double* outlet_u;           // [3][Ny][2] final u of columns Nx-3, Nx-2, Nx-1
+    const double* outlet_u_prev;// [3][Ny][2] u of columns Nx-3, Nx-2, Nx-1 after the previous step
+    double* outlet_u;           // the same after the current step (two buffers alternating by parity)
     const double* outlet_f_prev;// [Ny][3] post-BC f[2,6,8] at Nx-1 of the previous step
     double* outlet_f_next;      // [Ny][3] written by the current step
-    const double* delU;         // [Ny][2] convective speed term of the current step
+    double* delU;               // [Ny][2] convective speed term of the current step
+    int outlet_form;            // who forms delU before the outlet column is stepped (kOutlet*)
     const double* force_ibm;    // [2][S] dense IBM force of the current step, or null
     // Inside a replayed graph the step index comes from device memory: when
     // t_dev is set, kernels use *t_dev + t_off instead of their t argument.
@@ -77,5 +79,9 @@ struct LatDev {
     // for the next step.
     int* tile_ctr;
 };
+
+// LatDev::outlet_form: a kernel before the step (k_outlet_f64), or the warps
+// that hold outlet sites (the perimeter's also store it).
+enum { kOutletKernel, kOutletSites };
 
 }  // namespace life
