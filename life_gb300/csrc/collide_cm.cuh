@@ -1,8 +1,7 @@
 // Central-moments collision in FP64 (De Rosis 2019), the reference's
 // CENTRAL_MOMENTS branch of GridClass::streamCollide.
 #pragma once
-#include <cstring>
-
+#include "int_f64.cuh"
 #include "lbm_device.cuh"
 
 namespace life {
@@ -172,15 +171,6 @@ struct CmSite {
 
 // x with its sign flipped when the integer c is negative / multiplied by 2^e
 // (the exponent field moved by e; x zero or well inside the normal range).
-__host__ __device__ __forceinline__ double bits_double(unsigned long long u) {
-#ifdef __CUDA_ARCH__
-    return __longlong_as_double((long long)u);
-#else
-    double d;
-    std::memcpy(&d, &u, sizeof d);
-    return d;
-#endif
-}
 __host__ __device__ __forceinline__ double sgn_c(int c, double x) {
     return bits_double(div_bits(x) ^ ((unsigned long long)((unsigned)c & 0x80000000u) << 32));
 }
@@ -300,6 +290,131 @@ __host__ __device__ __forceinline__ double cm_population(int cx, int cy, const C
     }
     const double k8 = scale2(c.k8, rest ? 0 : (diag ? -2 : -1));
     return rest || diag ? a + k8 : a - k8;
+}
+
+
+// ---- whole sites with the products on the integer units -------------------
+//
+// collide_bgk<UNF = true> and collide_cm<UNF = true> for a site whose values
+// lie in the range populations_in_range() and site_range_ok() test: the same
+// operations on the same operands. The products and the sums with a power of
+// two are formed by the integer units (int_f64.cuh), the other sums by the FP64
+// unit; for the central moments the power-of-two factors are taken out (as in
+// cm_population) and the partial sums that directions share, up to their sign,
+// formed once: 144 FP64 instructions a site where the written-out form takes
+// about 310. Measured (1536 x 1536, central moments): 1.36 -> 0.68 ms a step,
+// the FP64 unit busy 82 % of the time and the integer unit 53 %; with the
+// products on the FP64 unit as well the shared sums alone would leave 240.
+
+// The populations are in [2^-8, 1) and each velocity component is zero or in
+// [2^-60, 2^-3): then every product of the two collisions is zero or in the
+// normal range (cm_factored_ok's bounds), and what 1/2, 1 and 2 are added to
+// is smaller than they are (3 |ux + uy| < 3/4, |ux + uy + 2 ux uy| < 1/2).
+__host__ __device__ __forceinline__ bool populations_in_range(const double f[9]) {
+    unsigned worst = 0;
+#pragma unroll
+    for (int v = 0; v < 9; v++) {
+        const unsigned d = (unsigned)(div_bits(f[v]) >> 32) - ((1023u - 8u) << 20);
+        worst = d > worst ? d : worst;
+    }
+    return worst < (8u << 20);
+}
+__host__ __device__ __forceinline__ bool velocity_in_range(double u) {
+    const unsigned long long b = div_bits(u) << 1;
+    return b == 0ull || (unsigned)(b >> 53) - (1023u - 60u) < 57u;
+}
+__host__ __device__ __forceinline__ bool site_range_ok(double ux, double uy, double omega) {
+    const unsigned w = (unsigned)(div_bits(omega) >> 52);  // omega in [2^-50, 4)
+    return velocity_in_range(ux) && velocity_in_range(uy) && w - (1023u - 50u) < 52u;
+}
+
+__host__ __device__ __forceinline__ void collide_bgk_int(const double f[9], double rho, double ux, double uy,
+                                                         double omega, double fs[9]) {
+    const double px = mul_int(ux, 3.0), py = mul_int(uy, 3.0);
+    const double pa = mul_int(ux + uy, 3.0), pb = mul_int(ux - uy, 3.0);
+    const double d9 = mul_int<kZeroAny>(mul_int(ux, 9.0), uy);
+    const double X2 = mul_int(ux, ux), Y2 = mul_int(uy, uy);
+    constexpr double c0 = 0.0 - 1.0 / 3.0, c1 = 1.0 - 1.0 / 3.0;
+    const double x0 = mul_int(X2, c0), x1 = mul_int(X2, c1), y0 = mul_int(Y2, c0), y1 = mul_int(Y2, c1);
+    const double h00 = mul_int(x0 + y0, 4.5), h10 = mul_int(x1 + y0, 4.5);
+    const double h01 = mul_int(x0 + y1, 4.5), h11 = mul_int(x1 + y1, 4.5);
+    const double r0 = mul_int<kNonZero>(rho, 4.0 / 9.0), r1 = mul_int<kNonZero>(rho, 1.0 / 9.0);
+    const double r2 = mul_int<kNonZero>(rho, 1.0 / 36.0);
+    double feq[9];
+    feq[0] = mul_int<kNonZero>(add_pow2_int<0>(h00), r0);
+    feq[1] = mul_int<kNonZero>(add_pow2_int<0>(px) + h10, r1);
+    feq[2] = mul_int<kNonZero>(add_pow2_int<0>(-px) + h10, r1);
+    feq[3] = mul_int<kNonZero>(add_pow2_int<0>(py) + h01, r1);
+    feq[4] = mul_int<kNonZero>(add_pow2_int<0>(-py) + h01, r1);
+    feq[5] = mul_int<kNonZero>((add_pow2_int<0>(pa) + h11) + d9, r2);
+    feq[6] = mul_int<kNonZero>((add_pow2_int<0>(-pa) + h11) + d9, r2);
+    feq[7] = mul_int<kNonZero>((add_pow2_int<0>(pb) + h11) + -d9, r2);
+    feq[8] = mul_int<kNonZero>((add_pow2_int<0>(-pb) + h11) + -d9, r2);
+#pragma unroll
+    for (int v = 0; v < 9; v++) fs[v] = f[v] + mul_int(feq[v] - f[v], omega);
+}
+
+// om = 1 - omega, cs2 = cs^2, cs4 = cs^4 in the written-out form's operations.
+__host__ __device__ __forceinline__ void collide_cm_int(const double f[9], double rho, double ux, double uy,
+                                                        double om, double cs2, double cs4, double fs[9]) {
+    const double X2 = mul_int(ux, ux), Y2 = mul_int(uy, uy);
+    const double xm = add_pow2_int<0>(-ux), xq = add_pow2_int<0>(ux);
+    const double ym = add_pow2_int<0>(-uy), yq = add_pow2_int<0>(uy);
+    const double D = X2 - Y2;
+    double k4Pre, k5Pre;
+    {
+        // f (cx^2 - cy^2) and (f cx) cy with cx = c - ux: the components of
+        // c = 0 and -1 are -ux and -(1 + ux); signs go into the sums
+        const double sxm = mul_int<kNonZero>(xm, xm), sxq = mul_int<kNonZero>(xq, xq);
+        const double sym = mul_int<kNonZero>(ym, ym), syq = mul_int<kNonZero>(yq, yq);
+        k4Pre = mul_int(D, f[0]);
+        k4Pre = k4Pre + mul_int(sxm - Y2, f[1]);
+        k4Pre = k4Pre + mul_int(sxq - Y2, f[2]);
+        k4Pre = k4Pre + mul_int(X2 - sym, f[3]);
+        k4Pre = k4Pre + mul_int(X2 - syq, f[4]);
+        k4Pre = k4Pre + mul_int(sxm - sym, f[5]);
+        k4Pre = k4Pre + mul_int(sxq - syq, f[6]);
+        k4Pre = k4Pre + mul_int(sxm - syq, f[7]);
+        k4Pre = k4Pre + mul_int(sxq - sym, f[8]);
+        k5Pre = mul_int<kZeroAny>(mul_int(ux, f[0]), uy);
+        k5Pre = k5Pre - mul_int(uy, mul_int<kNonZero>(xm, f[1]));
+        k5Pre = k5Pre + mul_int(uy, mul_int<kNonZero>(xq, f[2]));
+        k5Pre = k5Pre - mul_int(mul_int(ux, f[3]), ym);
+        k5Pre = k5Pre + mul_int(mul_int(ux, f[4]), yq);
+        k5Pre = k5Pre + mul_int<kNonZero>(ym, mul_int<kNonZero>(xm, f[5]));
+        k5Pre = k5Pre + mul_int<kNonZero>(yq, mul_int<kNonZero>(xq, f[6]));
+        k5Pre = k5Pre - mul_int<kNonZero>(yq, mul_int<kNonZero>(xm, f[7]));
+        k5Pre = k5Pre - mul_int<kNonZero>(ym, mul_int<kNonZero>(xq, f[8]));
+    }
+    const double k4 = mul_int<kZeroAny>(om, pos_zero(k4Pre)), k5 = mul_int<kZeroAny>(om, pos_zero(k5Pre));
+    const double k3 = scale2_nz(mul_int<kNonZero>(rho, cs2), 1), k8 = mul_int<kNonZero>(rho, cs4);
+    const double XY = mul_int<kZeroAny>(ux, uy), W = scale2(XY, 1);
+    const double X2Y2 = mul_int<kZeroAny>(X2, Y2), uxY2 = mul_int<kZeroAny>(ux, Y2);
+    const double X2uy = mul_int<kZeroAny>(X2, uy);
+    const double A = X2 - X2Y2, Bq = X2uy - X2Y2, Sp = X2Y2 + X2uy;
+    const double S = X2 + Y2, Qp = X2 + ux, Qm = X2 - ux, QpY = Qp + Y2, QmY = Qm + Y2, Rp = Qp - Y2, Rm = Qm - Y2;
+    const double uyW = uy - W, dxy = ux - uy;
+    // population: (((p0 k0 + p3 k3) + p4 k4) + p5 k5) +- k8, the moments scaled
+    // by the powers of two of its class (Z3: whether p3 may be zero)
+#define LIFE_CM_POP(v, Z3, p0, p3, p4, p5, K0, K3, K4, K5, K8) \
+    fs[v] = (((mul_int(p0, K0) + mul_int<Z3>(p3, K3)) + mul_int<kZeroAny>(p4, K4)) + mul_int<kZeroAny>(p5, K5)) + (K8)
+    LIFE_CM_POP(0, kNonZero, add_pow2_int<0>(-A - Y2), -add_pow2_int<1>(-S), Y2 - X2, XY, rho, scale2_nz(k3, -1), scale2(k4, -1), scale2(k5, 2), k8);
+    {
+        const double K0 = scale2_nz(rho, -1), K3 = scale2_nz(k3, -2), K4 = scale2(k4, -2), K8 = -scale2_nz(k8, -1);
+        LIFE_CM_POP(1, kNonZero, (A - uxY2) + ux, add_pow2_int<0>(-QpY), add_pow2_int<0>(Rp), -(uy + W), K0, K3, K4, k5, K8);
+        LIFE_CM_POP(2, kNonZero, (A + uxY2) - ux, add_pow2_int<0>(-QmY), add_pow2_int<0>(Rm), uyW, K0, K3, K4, k5, K8);
+        LIFE_CM_POP(3, kNonZero, ((Y2 - X2uy) - X2Y2) + uy, add_pow2_int<0>(-(S + uy)), -add_pow2_int<0>(uy - D), -(ux + W), K0, K3, K4, k5, K8);
+        LIFE_CM_POP(4, kNonZero, (Bq + Y2) - uy, add_pow2_int<0>(-(S - uy)), -add_pow2_int<0>(-(D + uy)), ux - W, K0, K3, K4, k5, K8);
+    }
+    {
+        const double K0 = scale2_nz(rho, -2), K3 = scale2_nz(k3, -3), K4 = scale2(k4, -3), K5 = scale2(k5, -1);
+        const double K8 = scale2_nz(k8, -2);
+        LIFE_CM_POP(5, kZeroA, (Sp + uxY2) + XY, QpY + uy, uy - Rp, add_pow2_int<-1>((ux + uy) + W), K0, K3, K4, K5, K8);
+        LIFE_CM_POP(6, kZeroA, XY - (Bq + uxY2), QmY - uy, -(Rm + uy), add_pow2_int<-1>(-(uyW + ux)), K0, K3, K4, K5, K8);
+        LIFE_CM_POP(7, kZeroA, (uxY2 - Bq) - XY, QpY - uy, -(Rp + uy), -add_pow2_int<-1>(dxy - W), K0, K3, K4, K5, K8);
+        LIFE_CM_POP(8, kZeroA, (Sp - uxY2) - XY, QmY + uy, uy - Rm, -add_pow2_int<-1>(-(dxy + W)), K0, K3, K4, K5, K8);
+    }
+#undef LIFE_CM_POP
 }
 
 }  // namespace life

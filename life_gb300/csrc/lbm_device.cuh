@@ -30,7 +30,7 @@ __host__ __device__ constexpr int cy_of(int v) { return v == 3 || v == 5 || v ==
 __host__ __device__ constexpr int opp_of(int v) { return v == 0 ? 0 : (v % 2 == 1 ? v + 1 : v - 1); }
 
 // Lattice weights exactly as GridClass::GridClass builds them (4/9, 1/9, 1/36).
-__device__ __forceinline__ double wgt(int v) {
+__host__ __device__ __forceinline__ double wgt(int v) {
     return v == 0 ? 4.0 / 9.0 : (v < 5 ? 1.0 / 9.0 : 1.0 / 36.0);
 }
 
@@ -243,7 +243,7 @@ __device__ __forceinline__ void macroscopic_ibm(const double f[9], double Fx, do
 // GridClass::equilibrium (src/Grid.cpp:249-264): 2nd-order Hermite (BGK) or
 // the 4th-order product form used with central moments.
 // c . u without its zero-component products (c of a D2Q9 direction)
-__device__ __forceinline__ double cdot_d(int cx, int cy, double ux, double uy) {
+__host__ __device__ __forceinline__ double cdot_d(int cx, int cy, double ux, double uy) {
     if (cx == 0) return cy == 0 ? 0.0 : cy * uy;
     return cy == 0 ? cx * ux : cx * ux + cy * uy;
 }
@@ -265,7 +265,7 @@ __device__ __forceinline__ double equilibrium(int v, double rho, double ux, doub
 }
 
 // GridClass::latticeForce (src/Grid.cpp:267-279), Guo forcing for BGK.
-__device__ __forceinline__ double lattice_force(int v, double ux, double uy, double Fx, double Fy) {
+__host__ __device__ __forceinline__ double lattice_force(int v, double ux, double uy, double Fx, double Fy) {
     const int cx = cx_of(v), cy = cy_of(v);
     const double cu = cdot_d(cx, cy, ux, uy);
     const double tx = cx == 0 ? -ux : (cx - ux) + cx * 3.0 * cu;
@@ -284,7 +284,7 @@ __device__ __forceinline__ double lattice_force(int v, double ux, double uy, dou
 // zero of either sign gives 1); the diagonal term 9 cx cy ux uy is
 // (9 ux) uy or its negative.
 template <bool UNF = false>
-__device__ __forceinline__ void collide_bgk(const double f[9], double rho, double ux, double uy, double Fx,
+__host__ __device__ __forceinline__ void collide_bgk(const double f[9], double rho, double ux, double uy, double Fx,
                                             double Fy, double omega, double fs[9]) {
     const bool forced = !UNF && (Fx != 0.0 || Fy != 0.0);
     const double px = 3.0 * ux, py = 3.0 * uy;

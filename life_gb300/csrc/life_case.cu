@@ -196,6 +196,9 @@ LatDev life::lattice_view(const LifeCase* c, int t) {
     L.has_ibm = c->obj.hasIBM;
     L.omega = c->p.omega;
     L.cs = c->cs;
+    L.om1 = 1.0 - c->p.omega;
+    L.cs2 = c->cs * c->cs;
+    L.cs4 = c->cs * c->cs * c->cs * c->cs;
     const double w[3] = {4.0 / 9.0, 1.0 / 9.0, 1.0 / 36.0};
     for (int k = 0; k < 3; k++) L.wreg[k] = w[k] / (2.0 * (c->cs * c->cs * c->cs * c->cs));
     L.Fx0 = c->Fx0;

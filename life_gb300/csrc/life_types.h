@@ -33,6 +33,7 @@ struct LatDev {
     int convective;       // right wall is a convective outlet
     int has_ibm;
     double omega, cs;
+    double om1, cs2, cs4; // 1 - omega, cs cs, ((cs cs) cs) cs
     double wreg[3];       // w / (2 cs^4) of the three weights (regularised condition)
     double Fx0, Fy0;      // constant force_xy (reference src/Grid.cpp:1035-1045)
     // the same values rounded to float once, on the host (FP32 kernels read
