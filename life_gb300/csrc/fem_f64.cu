@@ -41,11 +41,17 @@ __device__ __forceinline__ double shift_angle_d(double a) {
     return a - kPI;
 }
 
+// diracDelta (inc/Utils.h:220-232): beyond 1/2 (5 - 3 a - sqrt(1 - 3 (1-a)^2)) / 6,
+// else (1 + sqrt(1 - 3 a^2)) / 3. Lanes differ in the branch, so both take one
+// root and one quotient (-3 x + 1 and 1 - 3 x round alike).
 __device__ __forceinline__ double dirac_d(double dist) {
-    double a = fabs(dist);
+    const double a = fabs(dist);
     if (a > 1.5) return 0.0;
-    if (a > 0.5) return (5.0 - 3.0 * a - sqrt(-3.0 * DSQ(1.0 - a) + 1.0)) / 6.0;
-    return (1.0 + sqrt(1.0 - 3.0 * DSQ(a))) / 3.0;
+    const bool outer = a > 0.5;
+    const double t = outer ? 1.0 - a : a;
+    const double root = sqrt(1.0 - 3.0 * DSQ(t));
+    const double num = (outer ? 5.0 - 3.0 * a : 1.0) + (outer ? -root : root);
+    return num / (outer ? 6.0 : 3.0);
 }
 
 // Element rotation T = diag(R, R), R = [[c, s, 0], [-s, c, 0], [0, 0, 1]]
@@ -60,33 +66,70 @@ __device__ __forceinline__ double tval(int i, int j, double c, double s) {
     return b == 0 ? -s : c;
 }
 
-// out = T^T A T with the reference's summation order over non-zero terms.
+// Structurally non-zero entries of the local element matrices, bit 6 i + j: the
+// mass and linear stiffness matrices couple the axial displacements {0, 3} and
+// the bending ones {1, 2, 4, 5} separately; the geometric stiffness couples the
+// displacements {0, 1, 3, 4} without the axial pairs.
+__host__ __device__ constexpr unsigned long long pattern(bool geometric) {
+    unsigned long long m = 0;
+    for (int i = 0; i < 6; i++)
+        for (int j = 0; j < 6; j++) {
+            const bool nz = geometric ? i % 3 != 2 && j % 3 != 2 && (i % 3 == 1 || j % 3 == 1) : (i % 3 == 0) == (j % 3 == 0);
+            if (nz) m |= 1ull << (6 * i + j);
+        }
+    return m;
+}
+// +0 + x (which is x but for the sign of a zero), without the FP64 unit
+__device__ __forceinline__ double from_zero(double x) {
+    return (unsigned long long)__double_as_longlong(x) == 0x8000000000000000ull ? 0.0 : x;
+}
+
+// out = T^T A T with the reference's summation order over non-zero terms of T
+// and of A (pattern MASK); the other terms are exact zeros.
+template <unsigned long long MASK>
 __device__ __forceinline__ void tt_a_t(const double* A, double c, double s, double* out) {
     double R1[36];
+    bool full[36];
 #pragma unroll
     for (int i = 0; i < 6; i++)
 #pragma unroll
         for (int j = 0; j < 6; j++) {
             double acc = 0.0;
+            bool any = false;
 #pragma unroll
             for (int k = 0; k < 6; k++)
-                if (tnz(k, i)) acc += tval(k, i, c, s) * A[k * 6 + j];
+                if (tnz(k, i) && ((MASK >> (6 * k + j)) & 1)) {
+                    const double x = tval(k, i, c, s) * A[k * 6 + j];
+                    acc = any ? acc + x : from_zero(x);
+                    any = true;
+                }
             R1[i * 6 + j] = acc;
+            full[i * 6 + j] = any;
         }
 #pragma unroll
     for (int i = 0; i < 6; i++)
 #pragma unroll
         for (int j = 0; j < 6; j++) {
             double acc = 0.0;
+            bool any = false;
 #pragma unroll
             for (int k = 0; k < 6; k++)
-                if (tnz(k, j)) acc += R1[i * 6 + k] * tval(k, j, c, s);
+                if (tnz(k, j) && full[i * 6 + k]) {
+                    const double x = R1[i * 6 + k] * tval(k, j, c, s);
+                    acc = any ? acc + x : from_zero(x);
+                    any = true;
+                }
             out[i * 6 + j] = acc;
         }
 }
 
-// FEMBodyClass::updateFEMValues (src/FEMBody.cpp:198-223)
-__device__ void update_fem_values(FemBodyDev& B) {
+// FEMBodyClass::updateFEMValues (src/FEMBody.cpp:198-223). The CTA's last warp
+// runs `side` while the others evaluate the elements.
+struct NoSideTask {
+    __device__ void operator()() const {}
+};
+template <class Side = NoSideTask>
+__device__ __forceinline__ void update_fem_values(FemBodyDev& B, Side side = Side{}) {
     const double* U = vec(B, V_U);
     for (int n = threadIdx.x; n < B.nNodes; n += blockDim.x) {
         double* nd = B.node + n * 6;
@@ -95,7 +138,9 @@ __device__ void update_fem_values(FemBodyDev& B) {
         nd[5] = nd[4] + U[n * 3 + 2];
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < B.nEl; e += blockDim.x) {
+    const int workers = (int)blockDim.x - 32;
+    if ((int)threadIdx.x >= workers) side();
+    for (int e = threadIdx.x; e < B.nEl && (int)threadIdx.x < workers; e += workers) {
         const double* n0 = B.node + e * 6;
         const double* n1 = B.node + (e + 1) * 6;
         const double ev0 = n1[2] - n0[2], ev1 = n1[3] - n0[3];
@@ -486,7 +531,9 @@ __global__ void k_selftest_division(long long n, unsigned long long seed, unsign
         const int span = (w & 7) == 0 ? 2000 : 80;
         const long long xa = (long long)(1023 + (long long)((w >> 8) % span) - span / 2);
         const long long xb = (long long)(1023 + (long long)((w >> 24) % span) - span / 2);
-        const unsigned long long ba = (u & 0x800fffffffffffffull) | ((unsigned long long)(xa < 1 ? 1 : (xa > 2046 ? 2046 : xa)) << 52);
+        // one pair in 16 has equal or almost equal significands (a quotient at 1)
+        const unsigned long long ua = ((w >> 50) & 15) == 0 ? (u & 0x8000000000000000ull) | ((v + ((w >> 54) & 7) - 3) & 0xfffffffffffffull) : u;
+        const unsigned long long ba = (ua & 0x800fffffffffffffull) | ((unsigned long long)(xa < 1 ? 1 : (xa > 2046 ? 2046 : xa)) << 52);
         const unsigned long long bb = (v & 0x800fffffffffffffull) | ((unsigned long long)(xb < 1 ? 1 : (xb > 2046 ? 2046 : xb)) << 52);
         // one numerator in 64 is a signed zero (the velocity of a site at rest)
         const double a = ((w >> 40) & 63) == 0 ? __longlong_as_double((long long)(u & 0x8000000000000000ull))
@@ -495,6 +542,13 @@ __global__ void k_selftest_division(long long n, unsigned long long seed, unsign
         const double ref = a / b;
         const double got = div_rn_recip(a, b, __drcp_rn(b));
         if (__double_as_longlong(ref) != __double_as_longlong(got) && !(ref != ref && got != got)) atomicAdd(bad, 1ull);
+        // the integer reciprocal and quotient, where they decide
+        unsigned long long X;
+        if (recip64(b, X)) {
+            double r, i;
+            if (recip_round(b, X, r) && __double_as_longlong(r) != __double_as_longlong(__drcp_rn(b))) atomicAdd(bad, 1ull);
+            if (quotient_round(a, b, X, i) && __double_as_longlong(i) != __double_as_longlong(ref)) atomicAdd(bad, 1ull);
+        }
     }
 }
 
@@ -516,21 +570,198 @@ __device__ __forceinline__ int pick_pivot(double v, bool valid, int lane) {
     return __ffs(__ballot_sync(0xffffffffu, c1 && klo == ml)) - 1;
 }
 
+// Rows k0..k0+m-1 (m <= 32) of the forward substitution by one warp: y_k =
+// t_k / U(k,k), and every row r in (k, k+w] subtracts U(k,r) y_k; lane r & 31
+// holds t of row r. The reciprocals of the diagonal, a row per lane, come first;
+// rcp[k] = RN(1 / U(k,k)). (The loads of a row stand before the chain of the
+// row above it.)
+__device__ __forceinline__ void forward_rows(double* Bd, int nn, int kl, int W, int w, int k0, int m, int lane,
+                                             const double* rcp, double* y, double& t) {
+    const double mine = lane < m ? bd(Bd, W, kl, k0 + lane, k0 + lane) : 0.0;
+    unsigned long long mX;
+    const bool mok = recip64(mine, mX);
+    auto upper = [&](int k) {
+        const int rr = k + 1 + ((lane - k - 1) & 31);
+        return rr <= k + w && rr < nn ? bd(Bd, W, kl, k, rr) : 0.0;
+    };
+    double u = upper(k0);
+    for (int q = 0; q < m; q++) {
+        const int k = k0 + q, owner = k & 31, rr = k + 1 + ((lane - k - 1) & 31);
+        const double ukk = __shfl_sync(0xffffffffu, mine, q), uk = u;
+        const unsigned long long X = __shfl_sync(0xffffffffu, mX, q);
+        const bool ok = __shfl_sync(0xffffffffu, mok, q);
+        const double tn = k + 32 < nn ? y[k + 32] : 0.0;
+        if (q + 1 < m) u = upper(k + 1);
+        const double tk = __shfl_sync(0xffffffffu, t, owner);
+        double yk;
+        if (!(quotient_round(tk, ukk, X, yk) && ok)) yk = div_rn_recip(tk, ukk, rcp[k]);
+        if (lane == owner) {
+            y[k] = yk;
+            t = tn;
+        }
+        if (rr <= k + w && rr < nn) t = t - uk * yk;
+    }
+}
+
+// Band LU and forward substitution for kl, ku <= 5 (the beams' systems, and the
+// epsilon system of markers about a lattice unit apart): warp 0 factors with
+// the whole active window in registers, warp 1 runs the forward substitution
+// eight rows behind. The window of column j is rows j..j+5 and columns j..j+5:
+// v0 = M(j, j); lane (i, k), i and k in 1..5, holds a = M(j+i, j), A = M(j+i, j+k)
+// and the pivot row's uA = M(j, j+k). A column is one chain: the reciprocal of
+// the diagonal (integer steps) with the pivot test beside it, multiplier,
+// product and difference, and the broadcast of the next diagonal; the rest of
+// the window moves up by shuffles, and its last row and column, which no step
+// has touched, come from shared memory, in the shadow of the next reciprocal.
+// One warp issues an instruction every few cycles, so what counts beside the
+// chain is the number of instructions: every address is a lane's constant plus
+// a row stride, every bound a lane's last column.
+//
+// An interchange (another candidate is larger) exchanges two rows of the window
+// and takes a second reciprocal. The pivot row then reaches columns j+6..j+10:
+// these columns join the window (uB, Bx) until six columns after the last
+// interchange, when no remaining row has a changed entry that far right.
+// Entries beyond the band or the matrix are zeros, whose products change
+// nothing. The pipeline over four warps and shared memory below took 1290
+// cycles a column, this takes 630: the reciprocal about 200, multiplier,
+// product and difference 195, the pivot test, the stores and the shuffles the
+// rest. k_fem_dynamic of the 1200 x 400 filament: 1.19 -> 0.76 million cycles.
+__device__ __forceinline__ double band_entry(const double* Bd, int nn, int kl, int ku, int W, int r, int c) {
+    return r < nn && c < nn && c - r <= ku && r - c <= kl ? Bd[r * W + c - r + kl] : 0.0;
+}
+__device__ __forceinline__ unsigned long long magnitude_key(double v, unsigned long long nan) {
+    const unsigned long long key = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    return key > 0x7ff0000000000000ull ? nan : key;
+}
+constexpr int kForwardRows = 8;  // rows warp 1 takes at a time
+
+__device__ void band_lu_window(double* Bd, int nn, int kl, int ku, int W, int* piv, double* y, double* rcp) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {
+        const bool on = lane < 25;
+        const int i = on ? 1 + lane / 5 : 5, k = on ? 1 + lane % 5 : 5;
+        double v0 = band_entry(Bd, nn, kl, ku, W, 0, 0), a = band_entry(Bd, nn, kl, ku, W, i, 0);
+        double uA = band_entry(Bd, nn, kl, ku, W, 0, k), A = band_entry(Bd, nn, kl, ku, W, i, k);
+        double uB = 0.0, Bx = 0.0;
+        // what enters window j+1: M(j+1+i, j+1+k) on the lanes i = 5 or k = 5,
+        // M(j+1, j+6) on k = 5, M(j+6, j+1) on i = 5, as offsets from row j of
+        // the band; loaded while j < the lane's limit (0: never)
+        const int oA = (1 + i) * W + k - i + kl, oU = W + 5 + kl, oL = 6 * W + kl - 5;
+        const int far = i > k ? i : k;
+        const int nA = (i == 5 || k == 5) && k - i <= ku && i - k <= kl ? nn - 1 - far : 0;
+        const int nU = k == 5 && ku >= 5 ? nn - 6 : 0, nL = i == 5 && kl >= 5 ? nn - 6 : 0;
+        // stores of column j: the multiplier (lanes k = 1), U's row (lanes i = 1)
+        const int sL = i * W + kl - i, sU = kl + k;
+        const int mL = on && k == 1 && i <= kl ? nn - i : 0, mU = on && i == 1 && k <= kl + ku ? nn - k : 0;
+        double* row = Bd;  // row j
+        int last = -100;   // column of the last interchange
+        for (int j = 0; j < nn; j++, row += W) {
+            unsigned long long X;
+            double r;
+            bool ok = recip64(v0, X);
+            ok &= recip_round(v0, X, r);
+            const double eA = j < nA ? row[oA] : 0.0, eU = j < nU ? row[oU] : 0.0, eL = j < nL ? row[oL] : 0.0;
+            int src = 0;
+            // magnitudes by their high words first (a NaN on the diagonal stays)
+            const unsigned ha = (unsigned)__double2hiint(a) & 0x7fffffffu;
+            if (__any_sync(0xffffffffu, ha >= ((unsigned)__double2hiint(v0) & 0x7fffffffu))) {
+                // the first maximal magnitude: a NaN on the diagonal wins,
+                // others never do
+                const bool cand = on && k == 1;
+                const unsigned long long ka = magnitude_key(a, 0ull);
+                if (__any_sync(0xffffffffu, cand && ka > magnitude_key(v0, ~0ull))) {
+                    const unsigned kh = cand ? (unsigned)(ka >> 32) : 0u;
+                    const unsigned mh = __reduce_max_sync(0xffffffffu, kh);
+                    const bool c1 = cand && kh == mh;
+                    const unsigned ml = __reduce_max_sync(0xffffffffu, c1 ? (unsigned)ka : 0u);
+                    // lane (src, 1)
+                    const int from = __ffs(__ballot_sync(0xffffffffu, c1 && (unsigned)ka == ml)) - 1;
+                    src = 1 + from / 5;
+                    if (j - last >= 6) {  // the far columns join
+                        uB = 0.0;
+                        Bx = band_entry(Bd, nn, kl, ku, W, j + i, j + k + 5);
+                    }
+                    last = j;
+                    const double pv = __shfl_sync(0xffffffffu, a, from);
+                    const double rA = __shfl_sync(0xffffffffu, A, from + k - 1);
+                    const double rB = __shfl_sync(0xffffffffu, Bx, from + k - 1);
+                    if (i == src) {
+                        A = uA;
+                        Bx = uB;
+                        a = v0;
+                    }
+                    uA = rA;
+                    uB = rB;
+                    v0 = pv;
+                    ok = recip64(v0, X);
+                    ok &= recip_round(v0, X, r);
+                }
+            }
+            double scale = r;
+            if (!ok) {
+                r = __drcp_rn(v0);
+                // a zero pivot does not scale the column
+                scale = ((unsigned long long)__double_as_longlong(v0) << 1) != 0ull ? r : 1.0;
+            }
+            const double L = a * scale;
+            // x + L * (-u), written as the identical x - L * u
+            A = A - L * uA;
+            if (j < mL) row[sL] = L;
+            if (j < mU) row[sU] = uA;
+            if (lane == 0) {
+                row[kl] = v0;
+                piv[j] = j + src;
+                rcp[j] = r;  // RN(1 / U(j,j)) for the forward solve
+            }
+            const bool far_in = j - last < 6;
+            if (far_in) {
+                Bx = Bx - L * uB;
+                if (on && i == 1 && k + 5 <= kl + ku && j + k + 5 < nn) row[sU + 5] = uB;
+            }
+            if (j % kForwardRows == kForwardRows - 1 || j == nn - 1) named_bar(1, 64);
+            // the window of column j+1
+            v0 = __shfl_sync(0xffffffffu, A, 0);
+            const double fa = __shfl_sync(0xffffffffu, A, 5 * i), fA = __shfl_down_sync(0xffffffffu, A, 6);
+            const double pA = __shfl_sync(0xffffffffu, A, k);
+            a = i < 5 ? fa : eL;
+            uA = k < 5 ? pA : eU;
+            A = i < 5 && k < 5 ? fA : eA;
+            if (far_in) {
+                const double fB0 = __shfl_sync(0xffffffffu, Bx, 5 * i), fB = __shfl_down_sync(0xffffffffu, Bx, 6);
+                const double pB0 = __shfl_sync(0xffffffffu, Bx, 0), pB = __shfl_sync(0xffffffffu, Bx, k);
+                if (k == 5) {
+                    uA = pB0;
+                    if (i < 5) A = fB0;
+                }
+                uB = k < 5 ? pB : 0.0;
+                Bx = i == 5 ? band_entry(Bd, nn, kl, ku, W, j + 6, j + 6 + k) : (k < 5 ? fB : 0.0);
+            }
+        }
+    } else if (warp == 1) {
+        double t = lane < nn ? y[lane] : 0.0;
+        for (int k0 = 0; k0 < nn; k0 += kForwardRows) {
+            named_bar(1, 64);
+            const int m = nn - k0 < kForwardRows ? nn - k0 : kForwardRows;
+            forward_rows(Bd, nn, kl, W, kl + ku, k0, m, lane, rcp, y, t);
+        }
+        __syncwarp();
+    }
+}
+
 // Band LU of M and the forward half of the transposed solve (U^T y = b, y in
-// place), pipelined over warps 0-3 of the CTA; kl <= 31 and kl + ku <= 31.
+// place) by warps 0-3 of the CTA; kl <= 31 and kl + ku <= 31. Bands of up to
+// five go to band_lu_window; wider ones are pipelined.
 // The operations are those of band_factor_smem followed by the row-ordered
 // forward substitution; only who does them, and when, differs. The critical
 // path is warp 0's chain per column: reciprocal of the pivot, multipliers,
 // update of the next column's candidates. Everything else runs beside it:
-//   warp 0: step j's row swap, the scaling and the step-j update of column
-//           j+1, barrier 1, then the reciprocals of column j+1's candidates
-//           (each lane its own; the pivot's is kept, the same correctly
-//           rounded 1/pivot as a division after the choice). Column j+1's
-//           candidates are already in its registers (the rows it just
-//           updated, plus one row no earlier step touched);
-//   warp 3: after barrier 1, the choice of column j+1's pivot from the same
-//           candidates, which are final in shared memory by then, handed to
-//           warp 0 in s_src through barrier 2;
+//   warp 0: the reciprocals of column j's candidates (each lane its own; the
+//           pivot's is kept, the same correctly rounded 1/pivot as a division
+//           after the choice) from integer steps, the choice of the pivot
+//           between them, barrier 2, the row swap, the scaling and the step-j
+//           update of column j+1, barrier 1. Column j+1's candidates are then
+//           already in its registers (the rows it just updated, plus one row
+//           no earlier step touched);
 //   warps 1, 3: after barrier 1, the step-j update of columns j+2..kmax,
 //           split between them, then barrier 2 (which warp 0 waits on before
 //           the swap of step j+1, the first thing to touch those rows again);
@@ -543,8 +774,9 @@ __device__ __forceinline__ int pick_pivot(double v, bool valid, int lane) {
 // and barrier 2 after every step but the last; warp 2 calls barrier 1 nn
 // times. The k-th calls pair up, so every barrier completes. Needs at least
 // 128 threads; with fewer, warp 0 does everything.
+// (With the reciprocal in FP64, and the pivot chosen by warp 3 and handed over
+// through barrier 2, a column took 1271 cycles.)
 __device__ void band_lu_forward(double* Bd, int nn, int kl, int ku, int W, int* piv, double* y, double* rcp) {
-    __shared__ int s_src;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (blockDim.x < 128) {
         if (warp == 0) {
@@ -559,68 +791,64 @@ __device__ void band_lu_forward(double* Bd, int nn, int kl, int ku, int W, int* 
         }
         return;
     }
+    if (kl <= 5 && ku <= 5) {
+        band_lu_window(Bd, nn, kl, ku, W, piv, y, rcp);
+        return;
+    }
     if (warp == 0) {
-        // lane l holds the pivot candidate M(j+l, j) and its reciprocal
-        const int imax0 = kl < nn - 1 ? kl : nn - 1;
-        double v = lane <= imax0 ? bd(Bd, W, kl, lane, 0) : 0.0;
-        double rc = __drcp_rn(v);
-        int src = pick_pivot(v, lane <= imax0, lane);
+        // lane l holds the pivot candidate M(j+l, j)
+        double v = lane <= (kl < nn - 1 ? kl : nn - 1) ? bd(Bd, W, kl, lane, 0) : 0.0;
         for (int j = 0; j < nn; j++) {
             const int imax = j + kl < nn - 1 ? j + kl : nn - 1;
             const int kmax = j + kl + ku < nn - 1 ? j + kl + ku : nn - 1;
-            if (j > 0) {
-                named_bar(2, 96);
-                src = s_src;
-            }
+            const bool row = j + lane <= imax, early = j + 1 <= kmax;
+            // the candidates' reciprocals, and the choice among them meanwhile
+            unsigned long long X;
+            double rc;
+            bool ok = recip64(v, X);
+            ok &= recip_round(v, X, rc);
+            const int src = pick_pivot(v, row, lane);
+            // the row that enters column j+1's candidates: no step has touched it
+            const double entering =
+                lane == kl && j + 1 + kl < nn ? bd(Bd, W, kl, j + 1 + kl, j + 1) : 0.0;
+            if (j > 0) named_bar(2, 96);
+            double x = row && early ? bd(Bd, W, kl, j + lane, j + 1) : 0.0;
             const int jp = j + src;
-            const double pv = __shfl_sync(0xffffffffu, v, src);
-            const double v0 = __shfl_sync(0xffffffffu, v, 0);
-            if (lane == 0) piv[j] = jp;
+            const double pv = __shfl_sync(0xffffffffu, v, src), v0 = __shfl_sync(0xffffffffu, v, 0);
+            const double u1 = __shfl_sync(0xffffffffu, x, src), x0 = __shfl_sync(0xffffffffu, x, 0);
+            double r = __shfl_sync(0xffffffffu, rc, src);
+            if (!__shfl_sync(0xffffffffu, ok, src)) r = __drcp_rn(pv);
             // pivot != 0 (NaN counts as non-zero), tested on the bits
             const bool nz = ((unsigned long long)__double_as_longlong(pv) << 1) != 0ull;
-            const bool swapped = nz && jp != j;
-            const int c = j + lane;
-            double rj = 0.0, rp = 0.0;
-            if (c <= kmax) {
-                rj = bd(Bd, W, kl, j, c);
-                rp = bd(Bd, W, kl, jp, c);
-            }
-            const bool mrow = lane >= 1 && j + lane <= imax;  // multiplier row i = j + lane
-            const bool early = j + 1 <= kmax;
-            double x = 0.0;
-            if (mrow && early) x = bd(Bd, W, kl, j + lane, j + 1);
-            const double oj1 = __shfl_sync(0xffffffffu, rj, 1);  // old M(j, j+1)
-            const double op1 = __shfl_sync(0xffffffffu, rp, 1);  // old M(jp, j+1)
-            const double r = __shfl_sync(0xffffffffu, rc, src);
-            if (lane == 0) rcp[j] = r;  // RN(1 / U(j,j)) for the forward solve
-            // post-swap values
-            const double a = (swapped && j + lane == jp) ? v0 : v;
-            const double u1 = swapped ? op1 : oj1;
-            if (swapped && j + lane == jp) x = oj1;
+            const bool swapped = nz && src != 0;
+            // values after the swap (which a zero pivot does not make)
+            const double a = swapped && lane == src ? v0 : v;
+            if (swapped && lane == src) x = x0;
             const double L = nz ? a * r : a;
-            double nx = 0.0;
             // x + L * (-u1), written as the identical x - L * u1
-            if (mrow && early) nx = x - L * u1;
-            if (swapped && c <= kmax) {
-                bd(Bd, W, kl, j, c) = rp;
-                if (c >= j + 2) bd(Bd, W, kl, jp, c) = rj;
+            const bool mrow = lane >= 1 && row;  // multiplier row i = j + lane
+            const double nx = mrow && early ? x - L * (swapped ? u1 : x0) : 0.0;
+            if (swapped) {
+                const int c = j + lane;
+                if (c <= kmax) {
+                    const double rj = bd(Bd, W, kl, j, c), rp = bd(Bd, W, kl, jp, c);
+                    bd(Bd, W, kl, j, c) = rp;
+                    if (c >= j + 2) bd(Bd, W, kl, jp, c) = rj;
+                }
+                __syncwarp();
+            }
+            if (lane == 0) {
+                piv[j] = jp;
+                rcp[j] = r;  // RN(1 / U(j,j)) for the forward solve
             }
             if (mrow) {
                 bd(Bd, W, kl, j + lane, j) = L;
                 if (early) bd(Bd, W, kl, j + lane, j + 1) = nx;
             }
             named_bar(1, 128);
-            // column j+1's candidates: rows j+1..imax were just updated (lane
-            // l+1 holds row j+1+l); row j+1+kl, if it exists, is untouched
-            if (j + 1 < nn) {
-                const int imax1 = j + 1 + kl < nn - 1 ? j + 1 + kl : nn - 1;
-                const int row = j + 1 + lane;
-                double nv = __shfl_down_sync(0xffffffffu, nx, 1);
-                if (row > imax1) nv = 0.0;
-                else if (row > imax) nv = bd(Bd, W, kl, row, j + 1);
-                v = nv;
-                rc = __drcp_rn(v);
-            }
+            // column j+1's candidates: lane l+1 holds the updated row j+1+l
+            v = __shfl_down_sync(0xffffffffu, nx, 1);
+            if (lane == kl) v = entering;
         }
     } else if (warp == 1 || warp == 3) {
         // entry q of the kl x (kl+ku-1) block of a full step, kept in registers
@@ -632,15 +860,6 @@ __device__ void band_lu_forward(double* Bd, int nn, int kl, int ku, int W, int* 
             const int imax = j + kl < nn - 1 ? j + kl : nn - 1;
             const int kmax = j + kl + ku < nn - 1 ? j + kl + ku : nn - 1;
             const int rows = imax - j, cols = kmax - j - 1;
-            if (warp == 3 && j + 1 < nn) {
-                // column j+1's pivot: rows j+1..imax hold warp 0's updated
-                // values, row j+1+kl its untouched one
-                const int imax1 = j + 1 + kl < nn - 1 ? j + 1 + kl : nn - 1;
-                const int row = j + 1 + lane;
-                const double cv = row <= imax1 ? bd(Bd, W, kl, row, j + 1) : 0.0;
-                const int sp = pick_pivot(cv, row <= imax1, lane);
-                if (lane == 0) s_src = sp;
-            }
             if (rows == kl && cols == fc && rows * cols <= 128) {
                 // bd(i,k) + bd(i,j) * (-bd(j,k)), written as the identical
                 // bd(i,k) - bd(i,j) * bd(j,k)
@@ -665,15 +884,7 @@ __device__ void band_lu_forward(double* Bd, int nn, int kl, int ku, int W, int* 
         double t = lane < nn ? y[lane] : 0.0;
         for (int k = 0; k < nn; k++) {
             named_bar(1, 128);
-            const int owner = k & 31;
-            const double tk = __shfl_sync(0xffffffffu, t, owner);
-            const double yk = div_rn_recip(tk, bd(Bd, W, kl, k, k), rcp[k]);
-            if (lane == owner) {
-                y[k] = yk;
-                t = k + 32 < nn ? y[k + 32] : 0.0;
-            }
-            const int rr = k + 1 + ((lane - k - 1) & 31);
-            if (rr <= k + w && rr < nn) t = t - bd(Bd, W, kl, k, rr) * yk;
+            forward_rows(Bd, nn, kl, W, w, k, 1, lane, rcp, y, t);
         }
         __syncwarp();
     }
@@ -686,87 +897,178 @@ __device__ void band_forward_only(const double* Bd_, int nn, int kl, int ku, int
     double* Bd = const_cast<double*>(Bd_);
     const int lane = threadIdx.x & 31, w = kl + ku;
     double t = lane < nn ? y[lane] : 0.0;
-    for (int k = 0; k < nn; k++) {
-        const int owner = k & 31;
-        const double tk = __shfl_sync(0xffffffffu, t, owner);
-        const double yk = div_rn_recip(tk, bd(Bd, W, kl, k, k), rcp[k]);
-        if (lane == owner) {
-            y[k] = yk;
-            t = k + 32 < nn ? y[k + 32] : 0.0;
-        }
-        const int rr = k + 1 + ((lane - k - 1) & 31);
-        if (rr <= k + w && rr < nn) t = t - bd(Bd, W, kl, k, rr) * yk;
-    }
+    for (int k0 = 0; k0 < nn; k0 += 32) forward_rows(Bd, nn, kl, W, w, k0, nn - k0 < 32 ? nn - k0 : 32, lane, rcp, y, t);
     __syncwarp();
 }
 
-// Backward half of the transposed solve (L^T), one warp, after
-// band_lu_forward: lane l forms the product of the multiplier stored in band
-// row i+1+l with y at its final row Fp[i+1+l] (Fp: nn ints of scratch) and
-// puts it at its rank among those rows; lane 0 subtracts them in ascending
-// final row, the order of the dense solve. Then the row interchanges.
+// The products pr of lanes 0..m-1 subtracted from acc in lane order.
+__device__ __forceinline__ double subtract_lanes(double acc, double pr, int m) {
+    if (m == 5) {
+#pragma unroll
+        for (int q = 0; q < 5; q++) acc = acc - __shfl_sync(0xffffffffu, pr, q);
+    } else {
+        for (int q = 0; q < m; q++) acc = acc - __shfl_sync(0xffffffffu, pr, q);
+    }
+    return acc;
+}
+
+// Backward half of the transposed solve (L^T) after band_lu_forward, warps 0
+// and 1 of the CTA: row i subtracts the products of the multipliers stored in
+// band rows i+1..i+kl with y at their final rows, in ascending final row (the
+// order of the dense solve); then the row interchanges. The chain of a row is
+// one product and up to kl differences: its operands are loaded a row ahead,
+// and the newest y stays in a register. With interchanges warp 1 follows the
+// final rows (the swaps, from the last back) and leaves every row's terms in
+// order in Fp, a chunk of rows ahead of warp 0. 590 -> 478 cycles a row (kl = 5)
+// without interchanges; the chain alone is 415.
 __device__ void band_solve_back(const double* Bd_, int nn, int kl, int W, const int* piv, int* Fp, double* y) {
     double* Bd = const_cast<double*>(Bd_);
     __shared__ double s_prod[32];
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     bool any = false;
     for (int i0 = 0; i0 < nn; i0 += 32) {
         const int i = i0 + lane;
         any |= __any_sync(0xffffffffu, i < nn && piv[i] != i);
     }
     if (!any) {
-        // No interchange: every multiplier stays in its row, the final rows
-        // are i+1..i+kl in ascending order, and lane l's product is the l-th
-        // term. The newest value y[i+1] is lane 0's running sum of the
-        // previous row.
-        double ti = 0.0;
-        for (int i = nn - 1; i >= 0; i--) {
-            const int m = (i + kl < nn - 1 ? i + kl : nn - 1) - i;
-            const bool act = lane < m;
-            double yv = 0.0, bv = 0.0;
-            if (act) {
-                bv = bd(Bd, W, kl, i + 1 + lane, i);
-                yv = lane == 0 ? ti : y[i + 1 + lane];
+        // every multiplier stays in its row: lane l's product is the l-th term
+        if (warp != 0) return;
+        double yw = 0.0, bv = 0.0, yi = y[nn - 1];  // lane l: y[i+1+l] and its multiplier
+        int i = nn - 1;
+        // the last kl rows have fewer terms
+        for (; i >= 0 && i + kl > nn - 1; i--) {
+            const double pr = bv * yw, yc = yi;
+            if (i > 0) {
+                yi = y[i - 1];
+                bv = lane < kl && i + lane < nn ? bd(Bd, W, kl, i + lane, i - 1) : 0.0;
             }
-            const double pr = bv * yv;
-            double acc = y[i];
-            for (int q = 0; q < m; q++) acc = acc - __shfl_sync(0xffffffffu, pr, q);
-            ti = acc;
-            if (lane == 0) y[i] = ti;
-            __syncwarp();
+            const double acc = subtract_lanes(yc, pr, nn - 1 - i);
+            const double up = __shfl_up_sync(0xffffffffu, yw, 1);
+            yw = lane == 0 ? acc : up;
+            if (lane == 0) y[i] = acc;
         }
+        // M(i+1+lane, i) is a lane's constant away from row i
+        const double* at = Bd + (i + lane) * W + kl - 1 - lane;  // of row i-1
+        const bool mine = lane < kl;
+        if (kl == 5) {
+            for (; i >= 0; i--, at -= W) {
+                const double pr = bv * yw;
+                double acc = yi;
+                if (i > 0) {
+                    yi = y[i - 1];
+                    if (mine) bv = *at;
+                }
+                const double up = __shfl_up_sync(0xffffffffu, yw, 1);
+#pragma unroll
+                for (int q = 0; q < 5; q++) acc = acc - __shfl_sync(0xffffffffu, pr, q);
+                yw = lane == 0 ? acc : up;
+                if (lane == 0) y[i] = acc;
+            }
+        } else {
+            for (; i >= 0; i--, at -= W) {
+                const double pr = bv * yw;
+                double acc = yi;
+                if (i > 0) {
+                    yi = y[i - 1];
+                    if (mine) bv = *at;
+                }
+                const double up = __shfl_up_sync(0xffffffffu, yw, 1);
+                for (int q = 0; q < kl; q++) acc = acc - __shfl_sync(0xffffffffu, pr, q);
+                yw = lane == 0 ? acc : up;
+                if (lane == 0) y[i] = acc;
+            }
+        }
+        __syncwarp();
         return;
     }
-    for (int r = lane; r < nn; r += 32) Fp[r] = r;
-    __syncwarp();
-    for (int i = nn - 1; i >= 0; i--) {
-        const int rmax = i + kl < nn - 1 ? i + kl : nn - 1;
-        const int m = rmax - i;
-        const bool act = lane < m;
-        const int fk = act ? Fp[i + 1 + lane] : 0x7fffffff;
-        int rank = 0;
-        for (int q = 0; q < m; q++) rank += __shfl_sync(0xffffffffu, fk, q) < fk ? 1 : 0;
-        if (act) s_prod[rank] = bd(Bd, W, kl, i + 1 + lane, i) * y[fk];
+    const int chunk = kl > 0 ? (nn / (2 * kl) < 32 ? nn / (2 * kl) : 32) : 0;
+    if (kl > 8 || chunk < 1) {
+        if (warp != 0) return;
+        for (int r = lane; r < nn; r += 32) Fp[r] = r;
         __syncwarp();
-        if (lane == 0) {
-            double ti = y[i];
-            for (int q = 0; q < m; q++) ti = ti - s_prod[q];
-            y[i] = ti;
-            const int p = piv[i];
-            const int tmp = Fp[i];
-            Fp[i] = Fp[p];
-            Fp[p] = tmp;
+        for (int i = nn - 1; i >= 0; i--) {
+            const int rmax = i + kl < nn - 1 ? i + kl : nn - 1;
+            const int m = rmax - i;
+            const bool act = lane < m;
+            const int fk = act ? Fp[i + 1 + lane] : 0x7fffffff;
+            int rank = 0;
+            for (int q = 0; q < m; q++) rank += __shfl_sync(0xffffffffu, fk, q) < fk ? 1 : 0;
+            if (act) s_prod[rank] = bd(Bd, W, kl, i + 1 + lane, i) * y[fk];
+            __syncwarp();
+            if (lane == 0) {
+                double ti = y[i];
+                for (int q = 0; q < m; q++) ti = ti - s_prod[q];
+                y[i] = ti;
+                const int p = piv[i];
+                const int tmp = Fp[i];
+                Fp[i] = Fp[p];
+                Fp[p] = tmp;
+            }
+            __syncwarp();
         }
+    } else {
+        // terms of row i: Fp[half][(rows into the chunk) * kl + rank], the band
+        // row's offset from i+1 in the high half and the final row in the low
+        const int nch = (nn + chunk - 1) / chunk;
+        int F = 0;                            // warp 1: final row of band row i+1+lane
+        double ti = 0.0, bv = 0.0, yv = 0.0;  // warp 0
+        int fk = -1;
+        for (int c = 0; c <= nch; c++) {
+            if (warp == 1 && c < nch) {
+                int* out = Fp + (c & 1) * chunk * kl;
+                for (int q = 0; q < chunk; q++) {
+                    const int i = nn - 1 - (c * chunk + q);
+                    if (i < 0) break;
+                    const int p = piv[i], m = (i + kl < nn - 1 ? i + kl : nn - 1) - i;
+                    int rank = 0;
+                    for (int e = 0; e < m; e++) rank += __shfl_sync(0xffffffffu, F, e) < F ? 1 : 0;
+                    if (lane < m) out[q * kl + rank] = (lane << 16) | F;
+                    // the swap of step i: rows i (still its own) and p
+                    const int l = p - i - 1, fp = __shfl_sync(0xffffffffu, F, l >= 0 ? l : 0);
+                    if (lane == l) F = i;
+                    const int up = __shfl_up_sync(0xffffffffu, F, 1);
+                    F = lane == 0 ? (l >= 0 ? fp : i) : up;
+                }
+            } else if (warp == 0 && c > 0) {
+                const int* in = Fp + ((c - 1) & 1) * chunk * kl;
+                const int i1 = nn - 1 - (c - 1) * chunk;  // the chunk's first row
+                auto load = [&](int i) {
+                    fk = -1;
+                    bv = yv = 0.0;
+                    if (lane < (i + kl < nn - 1 ? i + kl : nn - 1) - i) {
+                        const int e = in[(i1 - i) * kl + lane];
+                        fk = e & 0xffff;
+                        bv = bd(Bd, W, kl, i + 1 + (e >> 16), i);
+                        yv = y[fk];  // (the newest row is in ti)
+                    }
+                };
+                load(i1);
+                for (int i = i1; i >= 0 && i > i1 - chunk; i--) {
+                    const int m = (i + kl < nn - 1 ? i + kl : nn - 1) - i;
+                    const double pr = bv * (fk == i + 1 ? ti : yv), yc = y[i];
+                    if (i > 0 && i - 1 > i1 - chunk) load(i - 1);
+                    ti = subtract_lanes(yc, pr, m);
+                    __syncwarp();
+                    if (lane == 0) y[i] = ti;
+                    __syncwarp();
+                }
+            }
+            named_bar(3, 64);
+        }
+        if (warp != 0) return;
+    }
+    for (int i0 = ((nn - 1) / 32) * 32; i0 >= 0; i0 -= 32) {
+        unsigned swaps = __ballot_sync(0xffffffffu, i0 + lane < nn && piv[i0 + lane] != i0 + lane);
+        if (lane == 0)
+            while (swaps) {
+                const int i = i0 + 31 - __clz(swaps), p = piv[i];
+                swaps &= ~(1u << (i - i0));
+                const double tt = y[i];
+                y[i] = y[p];
+                y[p] = tt;
+            }
         __syncwarp();
     }
-    if (lane == 0)
-        for (int i = nn - 1; i >= 0; i--)
-            if (piv[i] != i) {
-                const double tt = y[i];
-                y[i] = y[piv[i]];
-                y[piv[i]] = tt;
-            }
-    __syncwarp();
 }
 
 // Transposed solve M^T x = y in place (one lane, any band); Fp is nn ints of
@@ -1041,7 +1343,7 @@ __device__ __forceinline__ double eps_entry(const MarkerDev& M, int ki, int kj, 
 //                exact 0.0 the direct evaluation gives.
 //   c0[2*dim]    (ints)
 //   cand[cap]    pairs that pass a conservative prefilter (|dx| and |dy|
-//                below 3*Dx*(1 + 2^-40)), then their matrix entries
+//                below about 3*Dx), then their matrix entries
 //   band / y / pivots / final rows of the banded LU
 // Entries use the same operations and operands as eps_entry, so they are
 // identical. Returns false (uniformly) when the marker set does not fit; the
@@ -1077,15 +1379,28 @@ __device__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int di
     if (threadIdx.x == 0) { s_kl = 0; s_ku = 0; s_nc = 0; }
     for (int q = threadIdx.x; q < 2 * dim; q += blockDim.x) xy[q] = M.pos[m0 * 2 + q];
     __syncthreads();
+    // s = pos / Dx of every coordinate, and s in FP32 for the prefilter, at the
+    // entries' place until those are formed
+    const bool room = cap >= 3 * dim;
+    double* sc = cval;
+    float* sf = reinterpret_cast<float*>(cval + 2 * dim);
+    if (room) {
+        for (int q = threadIdx.x; q < 2 * dim; q += blockDim.x) {
+            sc[q] = xy[q] / Dx;
+            sf[q] = (float)sc[q];
+        }
+        __syncthreads();
+    }
     for (int q = threadIdx.x; q < 10 * dim; q += blockDim.x) {
         const int k = q / 10, a = (q % 10) / 5, o = q % 5;
-        const double sc = xy[2 * k + a] / Dx;
-        const int base = (int)floor(sc) - 2;
+        const double sk = room ? sc[2 * k + a] : xy[2 * k + a] / Dx;
+        const int base = (int)floor(sk) - 2;
         if (o == 0) c0[2 * k + a] = base;
-        ph[q] = dirac_d(fabs(sc - (base + o)));
+        ph[q] = dirac_d(fabs(sk - (base + o)));
     }
-    // prefilter + compaction, whole warps per iteration
-    const double lim = 3.0 * Dx * (1.0 + 0x1p-40);
+    // prefilter + compaction, whole warps per iteration (in FP32 with a margin
+    // well above its rounding, so that no pair of the exact test is lost)
+    const double lim = 3.0 * Dx * (1.0 + 0x1p-40), sure = 3.0 * Dx * (1.0 - 0x1p-40);
     const int lane = threadIdx.x & 31;
     const int total = dim * dim;
     for (int p0 = threadIdx.x & ~31; p0 < total; p0 += blockDim.x) {
@@ -1093,7 +1408,13 @@ __device__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int di
         bool c = false;
         if (pp < total) {
             const int i = pp / dim, j = pp % dim;
-            c = fabs(xy[2 * i] - xy[2 * j]) < lim && fabs(xy[2 * i + 1] - xy[2 * j + 1]) < lim;
+            if (room) {
+                const float xi = sf[2 * i], yi = sf[2 * i + 1], xj = sf[2 * j], yj = sf[2 * j + 1];
+                c = fabsf(xi - xj) < fmaf(0x1p-21f, fabsf(xi) + fabsf(xj), 3.001f) &&
+                    fabsf(yi - yj) < fmaf(0x1p-21f, fabsf(yi) + fabsf(yj), 3.001f);
+            } else {
+                c = fabs(xy[2 * i] - xy[2 * j]) < lim && fabs(xy[2 * i + 1] - xy[2 * j + 1]) < lim;
+            }
         }
         const unsigned bal = __ballot_sync(0xffffffffu, c);
         int base = 0;
@@ -1108,7 +1429,9 @@ __device__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int di
     for (int c = threadIdx.x; c < nc; c += blockDim.x) {
         const int pp = ckey[c];
         const int i = pp / dim, j = pp % dim;
-        if (fabs(xy[2 * i] - xy[2 * j]) / Dx < 3.0 && fabs(xy[2 * i + 1] - xy[2 * j + 1]) / Dx < 3.0) {
+        // (well below 3 Dx the quotient is below 3; only at the edge is it formed)
+        const double ax = fabs(xy[2 * i] - xy[2 * j]), ay = fabs(xy[2 * i + 1] - xy[2 * j + 1]);
+        if ((ax < sure || ax / Dx < 3.0) && (ay < sure || ay / Dx < 3.0)) {
             cval[c] = eps_entry_tab(M, m0 + i, j, ph, c0, M.ds[m0 + j]);
             if (j > i) atomicMax(&s_kl, j - i);
             else if (i > j) atomicMax(&s_ku, i - j);
@@ -1133,7 +1456,7 @@ __device__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int di
         __syncthreads();
         if (threadIdx.x < 128) band_lu_forward(Bd, dim, kl, ku, W, sp, y, reinterpret_cast<double*>(fp + dim));
         __syncthreads();
-        if (threadIdx.x < 32) band_solve_back(Bd, dim, kl, W, sp, fp, y);
+        if (threadIdx.x < 64) band_solve_back(Bd, dim, kl, W, sp, fp, y);
         __syncthreads();
         for (int i = threadIdx.x; i < dim; i += blockDim.x) M.eps[m0 + i] = y[i];
         __syncthreads();
@@ -1238,7 +1561,7 @@ __device__ void epsilon_range(const FsiDev& F, const MarkerDev& M, int m0, int d
         if (kl + ku < 32) {
             if (threadIdx.x < 128) band_lu_forward(Bd, dim, kl, ku, W, sp, y, reinterpret_cast<double*>(fp + dim));
             __syncthreads();
-            if (threadIdx.x < 32) band_solve_back(Bd, dim, kl, W, sp, fp, y);
+            if (threadIdx.x < 64) band_solve_back(Bd, dim, kl, W, sp, fp, y);
         } else if (threadIdx.x < 32) {
             band_factor_smem(Bd, dim, kl, ku, W, sp);
             if (threadIdx.x == 0) band_solve_smem(Bd, dim, kl, ku, W, sp, fp, y);
@@ -1420,50 +1743,60 @@ __global__ void __launch_bounds__(256) k_fem_dynamic(FsiDev F, MarkerDev M) {
             __syncthreads();
             if (threadIdx.x < 32) band_forward_only(sBd, nn, 5, 5, KW, sY, sRcp);
             __syncthreads();
-            if (threadIdx.x < 32) band_solve_back(sBd, nn, 5, KW, sPiv, sFp, sY);
+            if (threadIdx.x < 64) band_solve_back(sBd, nn, 5, KW, sPiv, sFp, sY);
             __syncthreads();
         } else {
-            // buildGlobalMatrices (src/FEMBody.cpp:90-109)
-            for (int e = threadIdx.x; e < B.nEl; e += blockDim.x) {
+            // buildGlobalMatrices (src/FEMBody.cpp:90-109): the stiffness and
+            // the internal force of an element on one half of the threads, its
+            // mass matrix on the other
+            for (int q = threadIdx.x & 127; q < B.nEl; q += 128) {
+                const int e = q;
                 const double* el = B.el + (size_t)e * EL_STRIDE;
-                const double L = el[EL_L], L0 = el[EL_L0], E = el[EL_E], A = el[EL_A], I = el[EL_I];
-                const double c = el[EL_COS], s = el[EL_SIN], ang = el[EL_ANG];
+                const double c = el[EL_COS], s = el[EL_SIN];
+                double* sc = B.elscr + (size_t)e * ES_STRIDE;
+                if (threadIdx.x >= 128) {
+                    tt_a_t<pattern(false)>(el + EL_M, c, s, sc + ES_M);
+                    continue;
+                }
+                const double L = el[EL_L], L0 = el[EL_L0], E = el[EL_E], A = el[EL_A], I = el[EL_I], ang = el[EL_ANG];
                 const double u = (DSQ(L) - DSQ(L0)) / (L + L0);
                 const double th1 = shift_angle_d(B.node[e * 6 + 5] - ang);
                 const double th2 = shift_angle_d(B.node[(e + 1) * 6 + 5] - ang);
                 const double F0 = (E * A / L0) * u;
-                const double M1 = (2 * E * I / L0) * (2.0 * th1 + th2);
-                const double M2 = (2 * E * I / L0) * (th1 + 2.0 * th2);
+                const double bend = 2 * E * I / L0;
+                const double M1 = bend * (2.0 * th1 + th2);
+                const double M2 = bend * (th1 + 2.0 * th2);
+                const double shear = (1.0 / L0) * (M1 + M2);
                 double Fl[6];
                 Fl[0] = -F0;
-                Fl[1] = (1.0 / L0) * (M1 + M2);
+                Fl[1] = shear;
                 Fl[2] = M1;
                 Fl[3] = F0;
-                Fl[4] = -(1.0 / L0) * (M1 + M2);
+                Fl[4] = -shear;
                 Fl[5] = M2;
-                double* sc = B.elscr + (size_t)e * ES_STRIDE;
                 tt_vec(Fl, c, s, sc + ES_F);
-                tt_a_t(el + EL_M, c, s, sc + ES_M);
                 double G[36], G2[36], KNL[36];
-                tt_a_t(el + EL_KL, c, s, G);
-                const double Fa = -Fl[0], V0 = Fl[4];
-    #pragma unroll
-                for (int q = 0; q < 36; q++) KNL[q] = 0.0;
-                KNL[0 * 6 + 1] = -V0 / L0;
-                KNL[0 * 6 + 4] = V0 / L0;
-                KNL[1 * 6 + 0] = -V0 / L0;
-                KNL[1 * 6 + 1] = Fa / L0;
-                KNL[1 * 6 + 3] = V0 / L0;
-                KNL[1 * 6 + 4] = -Fa / L0;
-                KNL[3 * 6 + 1] = V0 / L0;
-                KNL[3 * 6 + 4] = -V0 / L0;
-                KNL[4 * 6 + 0] = V0 / L0;
-                KNL[4 * 6 + 1] = -Fa / L0;
-                KNL[4 * 6 + 3] = -V0 / L0;
-                KNL[4 * 6 + 4] = Fa / L0;
-                tt_a_t(KNL, c, s, G2);
-    #pragma unroll
-                for (int q = 0; q < 36; q++) sc[ES_K + q] = G[q] + G2[q];
+                tt_a_t<pattern(false)>(el + EL_KL, c, s, G);
+                const double v = Fl[4] / L0, f = -Fl[0] / L0;
+#pragma unroll
+                for (int q6 = 0; q6 < 36; q6++) KNL[q6] = 0.0;
+                KNL[0 * 6 + 1] = -v;
+                KNL[0 * 6 + 4] = v;
+                KNL[1 * 6 + 0] = -v;
+                KNL[1 * 6 + 1] = f;
+                KNL[1 * 6 + 3] = v;
+                KNL[1 * 6 + 4] = -f;
+                KNL[3 * 6 + 1] = v;
+                KNL[3 * 6 + 4] = -v;
+                KNL[4 * 6 + 0] = v;
+                KNL[4 * 6 + 1] = -f;
+                KNL[4 * 6 + 3] = -v;
+                KNL[4 * 6 + 4] = f;
+                tt_a_t<pattern(true)>(KNL, c, s, G2);
+                // (the geometric part has no rotations: rows and columns 2, 5)
+#pragma unroll
+                for (int q6 = 0; q6 < 36; q6++)
+                    sc[ES_K + q6] = (q6 / 6) % 3 == 2 || q6 % 3 == 2 ? from_zero(G[q6]) : G[q6] + G2[q6];
             }
             __syncthreads();
             // Ordered assembly of M, K (band |r-c| <= 5) and F, then setNewmark
@@ -1529,7 +1862,7 @@ __global__ void __launch_bounds__(256) k_fem_dynamic(FsiDev F, MarkerDev M) {
                     cRcp[i] = sRcp[i];
                 }
             }
-            if (threadIdx.x < 32) band_solve_back(sBd, nn, 5, KW, sPiv, sFp, sY);
+            if (threadIdx.x < 64) band_solve_back(sBd, nn, 5, KW, sPiv, sFp, sY);
             __syncthreads();
         }
         {
@@ -1548,14 +1881,15 @@ __global__ void __launch_bounds__(256) k_fem_dynamic(FsiDev F, MarkerDev M) {
             const double* dU = vec(B, V_delU);
             for (int i = threadIdx.x; i < n; i += blockDim.x) sV[i] = dU[i] * dU[i];
         }
-        update_fem_values(B);
-        if (threadIdx.x == 0) {
-            double dd = 0.0;
-            for (int i = 0; i < n; i++) dd += sV[i];
-            s_res = sqrt(dd) / (F.ref_L * sqrt((double)n));
-            s_it++;
-        }
-        __syncthreads();
+        // (update_fem_values' first barrier stands between the squares and the sum)
+        update_fem_values(B, [&]() {
+            if ((threadIdx.x & 31) == 0) {
+                double dd = 0.0;
+                for (int i = 0; i < n; i++) dd += sV[i];
+                s_res = sqrt(dd) / (F.ref_L * sqrt((double)n));
+                s_it++;
+            }
+        });
     } while (s_res > 1e-10 && s_it < 20);
     finish_newmark(B, F);
     update_ibm(B, M);

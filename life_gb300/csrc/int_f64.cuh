@@ -120,7 +120,7 @@ __host__ __device__ __forceinline__ double add_pow2_int(double x) {
     const unsigned long long u = div_bits(x);
     const unsigned h = (unsigned)(u >> 32);
     const unsigned long long m = (((unsigned long long)((h & 0xfffffu) | 0x100000u) << 32) | (unsigned)u) << 10;
-    const unsigned d = (1023u + E) - ((h >> 20) & 0x7ffu);
+    const unsigned d = (unsigned)(1023 + E) - ((h >> 20) & 0x7ffu);
     unsigned long long a = shift_right(m, d);
     if (shift_left(a, d) != m) a |= 1;
     unsigned long long s = (1ull << 62) + ((int)h < 0 ? 0ull - a : a);
