@@ -1124,122 +1124,161 @@ __device__ void band_solve_smem(double* Bd, int nn, int kl, int ku, int W, const
 // update fills entries in. Every other entry is an exact zero, whose products
 // leave the values they are added to unchanged, so each value is formed by the
 // same operations in the same order as in the dense loops. A step:
-//   phase 1  warp 0 lists column j's rows, picks the first maximal magnitude
-//            (each lane forms its candidate's reciprocal meanwhile); warp 1
-//            lists row j's columns; the last warp takes the forward
-//            substitution of step j-1 (y[k] -= U(j-1,k) y[j-1])
+//   phase 1  warp 0 takes the first maximal magnitude of column j's rows (the
+//            diagonal's reciprocal is formed meanwhile) and the column's
+//            multipliers; the last warp the forward substitution of step j-1
+//            (y[k] -= U(j-1,k) y[j-1])
 //   swap     only where the pivot is not on the diagonal: whole rows, their
 //            masks, and row j's column list again
-//   phase 2  one thread per updated entry (its row's multiplier formed by
-//            each); the masks
-// b in y, the solution in y; rows and cols: 2n ints each. Needs 128 threads.
-// Returns false (uniformly) when a pivot is zero or not finite or the solution
-// is not finite: then zeros do matter, and the caller runs the dense loops.
+//   phase 2  one thread per updated entry, a 16 x 16 tile at a time; the masks;
+//            the last warp divides y[j] by the pivot, the two before it list
+//            the rows and columns of step j+1 (its masks with this step's bits,
+//            which others may be adding at the same time: the same bits)
+// b in y, the solution in y; rows and cols: 2n ints each, one after the other;
+// mult: n doubles. Needs 256 threads. Returns false (uniformly) when a pivot is
+// zero or not finite or the solution is not finite: then zeros do matter, and
+// the caller runs the dense loops.
 // One warp over all of the band (kl = ku = n) took 6.49 ms for the 132 markers
-// of a circle and its tail; this takes 0.32 ms, bound by the latencies of a
-// step (the lists, reciprocal, multiplier, product, difference).
+// of a circle and its tail; this takes 0.21 ms, bound by the latencies of a
+// step (reciprocal, multiplier, product, difference, two barriers).
 struct SparseLu {
     double* D;
     unsigned *rmask, *cmask;
-    double *y, *rcp;
+    double *y, *rcp, *mult;
     int *piv, *rows, *cols;
 };
 
-// Set bits above `above` of an n-bit mask as an ascending list (one warp;
-// nw <= 32); returns the count on every lane.
-__device__ __forceinline__ int mask_list(const unsigned* mask, int nw, int above, int* out) {
+// Set bits above `above` of lane-wise mask words (lane w holds word w; nw <= 32)
+// as an ascending list (one warp); returns the count on every lane.
+__device__ __forceinline__ int word_list(unsigned w, int above, int* out) {
     const int lane = threadIdx.x & 31;
-    unsigned w = lane < nw ? mask[lane] : 0u;
     const int first = above + 1 - 32 * lane;  // first wanted bit of this word
     if (first >= 32) w = 0u;
     else if (first > 0) w &= ~0u << first;
-    const int c = __popc(w);
-    int sum = c;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, sum, o);
-        if (lane >= o) sum += x;
-    }
-    int at = sum - c;
-    while (w) {
-        out[at++] = 32 * lane + __ffs(w) - 1;
-        w &= w - 1;
+    unsigned words = __ballot_sync(0xffffffffu, w != 0u);
+    int base = 0;
+    while (words) {
+        const int q = __ffs(words) - 1;
+        words &= words - 1;
+        const unsigned word = __shfl_sync(0xffffffffu, w, q);
+        if ((word >> lane) & 1u) out[base + __popc(word & ((1u << lane) - 1u))] = 32 * q + lane;
+        base += __popc(word);
     }
     __syncwarp();
-    return __shfl_sync(0xffffffffu, sum, 31);
+    return base;
+}
+__device__ __forceinline__ int mask_list(const unsigned* mask, int nw, int above, int* out) {
+    const int lane = threadIdx.x & 31;
+    return word_list(lane < nw ? mask[lane] : 0u, above, out);
 }
 
 __device__ __forceinline__ bool finite_bits(double x) {
     return ((unsigned)(__double_as_longlong(x) >> 32) & 0x7ff00000u) != 0x7ff00000u;
 }
 
-__device__ bool sparse_lu_solve(const SparseLu& S, int n, int nw) {
-    __shared__ int s_nr, s_nc[2], s_jp, s_bad, s_any;
-    __shared__ double s_r;
+__device__ __forceinline__ bool sparse_lu_solve(const SparseLu& S, int n, int nw) {
+    __shared__ int s_nr[2], s_nc[2], s_jp, s_bad, s_any, s_cnt[2][8];
+    __shared__ unsigned long long s_X;  // recip64 of the pivot (0: it does not apply)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, last = (blockDim.x >> 5) - 1;
     double* D = S.D;
     if (tid == 0) { s_bad = 0; s_any = 0; }
+    if (warp == last - 1) {
+        const int c = mask_list(S.cmask, nw, 0, S.rows);
+        if (lane == 0) s_nr[0] = c;
+    } else if (warp == last) {
+        const int c = mask_list(S.rmask, nw, 0, S.cols);
+        if (lane == 0) s_nc[0] = c;
+    }
     __syncthreads();
     for (int j = 0; j <= n; j++) {
         const int pb = j & 1;
-        int *rows = S.rows + pb * n, *cols = S.cols + pb * n;
+        int *rows = S.rows + pb * n, *cols = S.cols + pb * n;  // below / right of the diagonal
+        double* Dj = D + (size_t)j * n;
         // phase 1
         if (warp == 0 && j < n) {
-            const int nr = mask_list(S.cmask + (size_t)j * nw, nw, j, rows);  // below the diagonal
-            // candidates: the diagonal, then the listed rows
-            unsigned bh = 0, bl = 0;
-            int jp = -1;
-            double r = 0.0;
-            for (int q0 = 0; q0 <= nr; q0 += 32) {
-                const int q = q0 + lane;
-                const bool valid = q <= nr;
-                const int row = q == 0 ? j : (valid ? rows[q - 1] : j);
-                const double v = valid ? D[(size_t)j * n + row] : 0.0;
-                const double rc = __drcp_rn(v);
-                unsigned long long key = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-                if (key > 0x7ff0000000000000ull) key = q == 0 ? ~0ull : 0ull;
-                const unsigned kh = (unsigned)(key >> 32), klo = (unsigned)key;
-                const unsigned mh = __reduce_max_sync(0xffffffffu, valid ? kh : 0u);
-                const bool c1 = valid && kh == mh;
-                const unsigned ml = __reduce_max_sync(0xffffffffu, c1 ? klo : 0u);
-                const int src = __ffs(__ballot_sync(0xffffffffu, c1 && klo == ml)) - 1;
-                if (jp < 0 || mh > bh || (mh == bh && ml > bl)) {
-                    bh = mh;
-                    bl = ml;
-                    jp = __shfl_sync(0xffffffffu, row, src);
-                    r = __shfl_sync(0xffffffffu, rc, src);
+            const int nr = s_nr[pb];
+            // the first 32 candidates: the diagonal, then the listed rows
+            const int row = lane == 0 || lane > nr ? j : rows[lane - 1];
+            const double v = lane <= nr ? Dj[row] : 0.0;
+            const double v0 = __shfl_sync(0xffffffffu, v, 0);
+            int jp = j;
+            double pv = v0, r;
+            unsigned long long X;
+            bool ok = recip64(v0, X);
+            ok &= recip_round(v0, X, r);
+            // magnitudes by their high words first
+            const unsigned h0 = (unsigned)__double2hiint(v0) & 0x7fffffffu;
+            if (nr > 31 || __any_sync(0xffffffffu, lane > 0 && ((unsigned)__double2hiint(v) & 0x7fffffffu) >= h0)) {
+                // the first maximal magnitude: a NaN on the diagonal wins,
+                // others never do
+                unsigned long long best = magnitude_key(v0, ~0ull);
+                for (int q0 = 0; q0 < nr; q0 += 32) {
+                    const int i = q0 + lane < nr ? rows[q0 + lane] : -1;
+                    const double x = i >= 0 ? Dj[i] : 0.0;
+                    const unsigned long long key = i >= 0 ? magnitude_key(x, 0ull) : 0ull;
+                    const unsigned kh = (unsigned)(key >> 32), klo = (unsigned)key;
+                    const unsigned mh = __reduce_max_sync(0xffffffffu, kh);
+                    const bool c1 = i >= 0 && kh == mh;
+                    const unsigned ml = __reduce_max_sync(0xffffffffu, c1 ? klo : 0u);
+                    const unsigned long long top = ((unsigned long long)mh << 32) | ml;
+                    if (top > best) {
+                        best = top;
+                        const int src = __ffs(__ballot_sync(0xffffffffu, c1 && klo == ml)) - 1;
+                        jp = __shfl_sync(0xffffffffu, i, src);
+                        pv = __shfl_sync(0xffffffffu, x, src);
+                    }
+                }
+                if (jp != j) {
+                    ok = recip64(pv, X);
+                    ok &= recip_round(pv, X, r);
                 }
             }
+            if (!ok) {
+                r = __drcp_rn(pv);
+                X = 0ull;
+                if (lane == 0 && (pv == 0.0 || !finite_bits(pv))) s_bad = 1;
+            }
+            // the multipliers, as they stand after the interchange
+            if (lane > 0 && lane <= nr) {
+                const double m = (row == jp ? v0 : v) * r;
+                S.mult[lane - 1] = m;
+                Dj[row] = m;
+            }
+            for (int q = 31 + lane; q < nr; q += 32) {
+                const int i = rows[q];
+                const double m = (i == jp ? v0 : Dj[i]) * r;
+                S.mult[q] = m;
+                Dj[i] = m;
+            }
             if (lane == 0) {
-                s_nr = nr;
+                Dj[j] = pv;
                 s_jp = jp;
-                s_r = r;
                 S.piv[j] = jp;
+                s_X = X;
                 S.rcp[j] = r;
-                if ((bh | bl) == 0u || bh >= 0x7ff00000u) s_bad = 1;
                 if (jp != j) s_any = 1;
             }
-        } else if (warp == 1 && j < n) {
-            const int nc = mask_list(S.rmask + (size_t)j * nw, nw, j, cols);
-            if (lane == 0) s_nc[pb] = nc;
         } else if (warp == last && j > 0) {
             const int k = j - 1, nc = s_nc[pb ^ 1];
             const int* pc = S.cols + (pb ^ 1) * n;
-            const double yk = div_rn_recip(S.y[k], D[(size_t)k * n + k], S.rcp[k]);
-            __syncwarp();
-            if (lane == 0) S.y[k] = yk;
+            const double yk = S.y[k];
             for (int q = lane; q < nc; q += 32) S.y[pc[q]] = S.y[pc[q]] - D[(size_t)pc[q] * n + k] * yk;
         }
         __syncthreads();
         if (j == n || s_bad) break;
-        const int jp = s_jp, nr = s_nr;
+        const int jp = s_jp;
         if (jp != j) {
+            // (column j has its new values already)
             for (int k = tid; k < n; k += blockDim.x) {
-                const double a = D[(size_t)k * n + j], b = D[(size_t)k * n + jp];
-                D[(size_t)k * n + j] = b;
-                D[(size_t)k * n + jp] = a;
+                if (k != j) {
+                    const double a = D[(size_t)k * n + j], b = D[(size_t)k * n + jp];
+                    D[(size_t)k * n + j] = b;
+                    D[(size_t)k * n + jp] = a;
+                }
                 unsigned* m = S.cmask + (size_t)k * nw;
                 const unsigned bj = (m[j >> 5] >> (j & 31)) & 1u, bp = (m[jp >> 5] >> (jp & 31)) & 1u;
-                if (bj != bp) {
+                // (in column j both stay: the pivot and what was the diagonal)
+                if (bj != bp && k != j) {
                     m[j >> 5] ^= 1u << (j & 31);
                     m[jp >> 5] ^= 1u << (jp & 31);
                 }
@@ -1257,56 +1296,118 @@ __device__ bool sparse_lu_solve(const SparseLu& S, int n, int nw) {
             __syncthreads();
         }
         // phase 2
-        const int nc = s_nc[pb];
-        const double r = s_r;
-        for (int q = tid; q < nr * nc; q += blockDim.x) {
-            const int b = q / nr, i = rows[q - b * nr], k = cols[b];
-            const double l = D[(size_t)j * n + i] * r;
-            D[(size_t)k * n + i] = D[(size_t)k * n + i] - l * D[(size_t)k * n + j];
+        const int nr = s_nr[pb], nc = s_nc[pb];
+        if (warp == last) {
+            // (y[j] has its last term: phase 1 took step j-1's)
+            const double t = S.y[j], u = Dj[j];
+            const unsigned long long X = s_X;
+            double yk;
+            if (!quotient_round(t, u, X, yk) || X == 0ull) yk = div_rn_recip(t, u, S.rcp[j]);
+            if (lane == 0) S.y[j] = yk;
+        } else if (warp >= last - 2 && j + 1 < n) {
+            // column j+1 gains column j's rows if the pivot row reaches it, row
+            // j+1 the pivot row's columns if column j reaches it
+            const bool col = warp == last - 1;
+            const unsigned* own = (col ? S.cmask : S.rmask) + (size_t)(j + 1) * nw;
+            const unsigned* add = (col ? S.cmask : S.rmask) + (size_t)j * nw;
+            const unsigned reach = (col ? S.rmask : S.cmask)[(size_t)j * nw + ((j + 1) >> 5)] >> ((j + 1) & 31) & 1u;
+            unsigned w = 0u;
+            if (lane < nw) w = own[lane] | (reach ? add[lane] : 0u);
+            const int c = word_list(w, j + 1, (col ? S.rows : S.cols) + (pb ^ 1) * n);
+            if (lane == 0) (col ? s_nr : s_nc)[pb ^ 1] = c;
         }
-        // the filled-in entries' bits: row masks by (row, word), column masks
-        // by (column, word); only columns above j and rows below the diagonal
-        for (int q = blockDim.x - 1 - tid; q < (nr + nc) * nw; q += blockDim.x) {
-            const int a = q / nw, w = q - a * nw;
+        const int a0 = tid & 15, b0 = tid >> 4;
+        for (int b = b0; b < nc; b += 16) {
+            double* Dk = D + (size_t)cols[b] * n;
+            const double u = Dk[j];
+            for (int a = a0; a < nr; a += 16) {
+                const int i = rows[a];
+                Dk[i] = Dk[i] - S.mult[a] * u;
+            }
+        }
+        // the filled-in entries' bits; only columns above j and rows below the
+        // diagonal
+        // (by warps 1-4, which have no other task)
+        for (int w = b0 - 2; w >= 0 && b0 < 10 && w < nw; w += 8) {
             const int first = j + 1 - 32 * w;
             const unsigned keep = first >= 32 ? 0u : (first > 0 ? ~0u << first : ~0u);
-            if (a < nr) S.rmask[(size_t)rows[a] * nw + w] |= S.rmask[(size_t)j * nw + w] & keep;
-            else S.cmask[(size_t)cols[a - nr] * nw + w] |= S.cmask[(size_t)j * nw + w] & keep;
+            const unsigned rj = S.rmask[(size_t)j * nw + w] & keep, cj = S.cmask[(size_t)j * nw + w] & keep;
+            for (int a = a0; a < nr; a += 16) S.rmask[(size_t)rows[a] * nw + w] |= rj;
+            for (int b = a0; b < nc; b += 16) S.cmask[(size_t)cols[b] * nw + w] |= cj;
         }
         __syncthreads();
-        // the multipliers, now that no thread reads column j any more; what
-        // runs beside this (phase 1 of step j+1) reads neither
-        if (warp == 2)
-            for (int a = lane; a < nr; a += 32) D[(size_t)j * n + rows[a]] *= r;
     }
     if (s_bad) return false;  // (set before a barrier: the same on all threads)
-    // L^T x = y from the last row up: the products of a column's multipliers
-    // on lanes, subtracted in ascending row order; then the row interchanges
-    if (warp == 0) {
-        for (int i = n - 1; i >= 0; i--) {
-            const int c = mask_list(S.cmask + (size_t)i * nw, nw, i, S.rows);
-            double t = S.y[i];
-            for (int q0 = 0; q0 < c; q0 += 32) {
-                const int m = c - q0 < 32 ? c - q0 : 32;
-                double pr = 0.0;
-                if (lane < m) {
-                    const int k = S.rows[q0 + lane];
-                    pr = D[(size_t)i * n + k] * S.y[k];
-                }
-                for (int q = 0; q < m; q++) t = t - __shfl_sync(0xffffffffu, pr, q);
+    // L^T x = y from the last row up: the products of a column's multipliers on
+    // lanes, subtracted in ascending row order by warp 0; the other warps list
+    // the rows of the next `last` columns meanwhile (in rows and cols' place)
+    const int cap = 4 * n / (2 * last) < 32 ? 4 * n / (2 * last) : 32, groups = (n + last - 1) / last;
+    for (int g = 0; g <= groups; g++) {
+        if (warp > 0 && g < groups) {
+            const int i = n - 1 - (g * last + warp - 1);
+            if (i >= 0) {
+                const unsigned w = lane < nw ? S.cmask[(size_t)i * nw + lane] : 0u;
+                const int first = i + 1 - 32 * lane;
+                const int c = __reduce_add_sync(0xffffffffu, __popc(first >= 32 ? 0u : (first > 0 ? w & (~0u << first) : w)));
+                if (c <= cap) word_list(w, i, S.rows + ((g & 1) * last + warp - 1) * cap);
+                if (lane == 0) s_cnt[g & 1][warp] = c;
             }
-            __syncwarp();
-            if (lane == 0) S.y[i] = t;
-            __syncwarp();
-        }
-        if (lane == 0 && s_any)
-            for (int i = n - 1; i >= 0; i--)
-                if (S.piv[i] != i) {
-                    const double t = S.y[i];
-                    S.y[i] = S.y[S.piv[i]];
-                    S.y[S.piv[i]] = t;
+        } else if (warp == 0 && g > 0) {
+            const int i1 = n - 1 - (g - 1) * last;  // the group's first row
+            const int* lists = S.rows + ((g - 1) & 1) * last * cap;
+            const int rows_left = i1 + 1 < last ? i1 + 1 : last;
+            // a row's count and list two rows ahead, its operands one ahead
+            // (its newest term is in t)
+            int c = 0, c1 = 0, k = -1, k1 = -1;
+            double d = 0.0, yk = 0.0, yi = 0.0, t = 0.0;
+            auto list_of = [&](int p) {
+                c1 = p < rows_left ? s_cnt[(g - 1) & 1][p + 1] : 0;
+                k1 = lane < c1 && c1 <= cap ? lists[p * cap + lane] : -1;
+            };
+            auto load = [&](int p) {
+                c = c1;
+                k = k1;
+                d = yk = 0.0;
+                yi = S.y[i1 - p];
+                if (k >= 0) {
+                    d = D[(size_t)(i1 - p) * n + k];
+                    yk = S.y[k];
                 }
+                list_of(p + 1);
+            };
+            list_of(0);
+            load(0);
+            for (int p = 0; p < rows_left; p++) {
+                const int i = i1 - p, m = c;
+                const double pr = d * (p > 0 && k == i + 1 ? t : yk);
+                t = yi;
+                if (p + 1 < rows_left) load(p + 1);
+                if (m <= cap) {
+                    for (int q = 0; q < m; q++) t = t - __shfl_sync(0xffffffffu, pr, q);
+                } else {  // more rows than a list holds: every row below
+                    for (int q0 = i + 1; q0 < n; q0 += 32) {
+                        const int kk = q0 + lane, mm = n - q0 < 32 ? n - q0 : 32;
+                        const bool bit = kk < n && ((S.cmask[(size_t)i * nw + (kk >> 5)] >> (kk & 31)) & 1u);
+                        const unsigned some = __ballot_sync(0xffffffffu, bit);
+                        const double pq = bit ? D[(size_t)i * n + kk] * S.y[kk] : 0.0;
+                        for (int q = 0; q < mm; q++)
+                            if ((some >> q) & 1u) t = t - __shfl_sync(0xffffffffu, pq, q);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) S.y[i] = t;
+                __syncwarp();
+            }
+        }
+        __syncthreads();
     }
+    if (tid == 0 && s_any)
+        for (int i = n - 1; i >= 0; i--)
+            if (S.piv[i] != i) {
+                const double t = S.y[i];
+                S.y[i] = S.y[S.piv[i]];
+                S.y[S.piv[i]] = t;
+            }
     __syncthreads();
     bool ok = true;
     for (int i = tid; i < n; i += blockDim.x) ok = ok && finite_bits(S.y[i]);
@@ -1348,21 +1449,32 @@ __device__ __forceinline__ double eps_entry(const MarkerDev& M, int ki, int kj, 
 // Entries use the same operations and operands as eps_entry, so they are
 // identical. Returns false (uniformly) when the marker set does not fit; the
 // caller then runs the direct path.
-__device__ __forceinline__ double eps_entry_tab(const MarkerDev& M, int ki, int jl, const double* ph, const int* c0,
-                                                double dsj) {
+// (sd, si, sj: the marker's support; the nine loads of each go out together,
+// the sum is in order)
+__device__ __forceinline__ double eps_entry_tab(const double* sd, const int* si, const int* sj, int ns, int jl,
+                                                const double* ph, const int* c0, double dsj) {
+    int ei[9], ej[9];
+    double dv[9];
+#pragma unroll
+    for (int s = 0; s < 9; s++) {
+        ei[s] = si[s];
+        ej[s] = sj[s];
+        dv[s] = sd[s];
+    }
+    const int cx = c0[jl * 2], cy = c0[jl * 2 + 1];
     double acc = 0.0;
-    const int ns = M.nsupp[ki];
-    for (int s = 0; s < ns; s++) {
-        const double dvi = M.sd[ki * 9 + s];
-        const int ox = M.si[ki * 9 + s] - c0[jl * 2], oy = M.sj[ki * 9 + s] - c0[jl * 2 + 1];
+#pragma unroll
+    for (int s = 0; s < 9; s++) {
+        const int ox = ei[s] - cx, oy = ej[s] - cy;
         const double px = (ox >= 0 && ox < 5) ? ph[jl * 10 + ox] : 0.0;
         const double py = (oy >= 0 && oy < 5) ? ph[jl * 10 + 5 + oy] : 0.0;
-        acc += dvi * (px * py);
+        const double next = acc + dv[s] * (px * py);
+        acc = s < ns ? next : acc;
     }
     return acc * (1.0 * 1.0 * dsj);
 }
 
-__device__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int dim, double* A, double* bx, int* piv,
+__device__ __forceinline__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int dim, double* A, double* bx, int* piv,
                              int* lmax, double* sm, int sm_doubles) {
     __shared__ int s_kl, s_ku, s_nc;
     const long long fixed = 13LL * dim + 64;
@@ -1398,41 +1510,62 @@ __device__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int di
         if (o == 0) c0[2 * k + a] = base;
         ph[q] = dirac_d(fabs(sk - (base + o)));
     }
-    // prefilter + compaction, whole warps per iteration (in FP32 with a margin
-    // well above its rounding, so that no pair of the exact test is lost)
+    // prefilter + compaction, a row of pairs per warp (in FP32 with a margin well
+    // above its rounding, so that no pair of the exact test is lost)
     const double lim = 3.0 * Dx * (1.0 + 0x1p-40), sure = 3.0 * Dx * (1.0 - 0x1p-40);
     const int lane = threadIdx.x & 31;
-    const int total = dim * dim;
-    for (int p0 = threadIdx.x & ~31; p0 < total; p0 += blockDim.x) {
-        const int pp = p0 + lane;
-        bool c = false;
-        if (pp < total) {
-            const int i = pp / dim, j = pp % dim;
-            if (room) {
-                const float xi = sf[2 * i], yi = sf[2 * i + 1], xj = sf[2 * j], yj = sf[2 * j + 1];
-                c = fabsf(xi - xj) < fmaf(0x1p-21f, fabsf(xi) + fabsf(xj), 3.001f) &&
-                    fabsf(yi - yj) < fmaf(0x1p-21f, fabsf(yi) + fabsf(yj), 3.001f);
-            } else {
-                c = fabs(xy[2 * i] - xy[2 * j]) < lim && fabs(xy[2 * i + 1] - xy[2 * j + 1]) < lim;
+    for (int i = threadIdx.x >> 5; i < dim; i += blockDim.x >> 5) {
+        const float xi = room ? sf[2 * i] : 0.0f, yi = room ? sf[2 * i + 1] : 0.0f;
+#pragma unroll 2
+        for (int j0 = 0; j0 < dim; j0 += 32) {
+            const int j = j0 + lane;
+            bool c = false;
+            if (j < dim) {
+                if (room) {
+                    const float xj = sf[2 * j], yj = sf[2 * j + 1];
+                    c = fabsf(xi - xj) < fmaf(0x1p-21f, fabsf(xi) + fabsf(xj), 3.001f) &&
+                        fabsf(yi - yj) < fmaf(0x1p-21f, fabsf(yi) + fabsf(yj), 3.001f);
+                } else {
+                    c = fabs(xy[2 * i] - xy[2 * j]) < lim && fabs(xy[2 * i + 1] - xy[2 * j + 1]) < lim;
+                }
             }
+            const unsigned bal = __ballot_sync(0xffffffffu, c);
+            if (bal == 0u) continue;
+            int base = 0;
+            if (lane == 0) base = atomicAdd(&s_nc, __popc(bal));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            const int slot = base + __popc(bal & ((1u << lane) - 1u));
+            if (c && slot < cap) ckey[slot] = i * dim + j;
         }
-        const unsigned bal = __ballot_sync(0xffffffffu, c);
-        int base = 0;
-        if (lane == 0 && bal) base = atomicAdd(&s_nc, __popc(bal));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        const int slot = base + __popc(bal & ((1u << lane) - 1u));
-        if (c && slot < cap) ckey[slot] = pp;
     }
     __syncthreads();
     const int nc = s_nc;
     if (nc > cap) return false;
+    // the markers' supports, where the system will stand (a pair's entry reads
+    // all of one: from global memory 32 lanes touch 32 lines at a time)
+    const bool staged = 18LL * dim <= band_doubles;
+    const double* gd = M.sd + (size_t)m0 * 9;
+    const int *gi = M.si + (size_t)m0 * 9, *gj = M.sj + (size_t)m0 * 9;
+    if (staged) {
+        double* td = band;
+        int *ti = reinterpret_cast<int*>(band + 9 * dim), *tj = ti + 9 * dim;
+        for (int q = threadIdx.x; q < 9 * dim; q += blockDim.x) {
+            td[q] = gd[q];
+            ti[q] = gi[q];
+            tj[q] = gj[q];
+        }
+        gd = td;
+        gi = ti;
+        gj = tj;
+        __syncthreads();
+    }
     for (int c = threadIdx.x; c < nc; c += blockDim.x) {
         const int pp = ckey[c];
         const int i = pp / dim, j = pp % dim;
         // (well below 3 Dx the quotient is below 3; only at the edge is it formed)
         const double ax = fabs(xy[2 * i] - xy[2 * j]), ay = fabs(xy[2 * i + 1] - xy[2 * j + 1]);
         if ((ax < sure || ax / Dx < 3.0) && (ay < sure || ay / Dx < 3.0)) {
-            cval[c] = eps_entry_tab(M, m0 + i, j, ph, c0, M.ds[m0 + j]);
+            cval[c] = eps_entry_tab(gd + i * 9, gi + i * 9, gj + i * 9, M.nsupp[m0 + i], j, ph, c0, M.ds[m0 + j]);
             if (j > i) atomicMax(&s_kl, j - i);
             else if (i > j) atomicMax(&s_ku, i - j);
         } else {
@@ -1475,13 +1608,14 @@ __device__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int di
         SparseLu S;
         S.y = at;
         S.rcp = S.y + dim;
-        S.piv = reinterpret_cast<int*>(S.rcp + dim);
+        S.mult = S.rcp + dim;
+        S.piv = reinterpret_cast<int*>(S.mult + dim);
         S.rows = S.piv + dim;
         S.cols = S.rows + 2 * dim;
         S.rmask = reinterpret_cast<unsigned*>(S.cols + 2 * dim);
         S.cmask = S.rmask + (size_t)dim * nw;
         const long long ints = 5LL * dim + 2LL * dim * nw;
-        const long long used = (at - sm) + 2LL * dim + (ints + 1) / 2;
+        const long long used = (at - sm) + 3LL * dim + (ints + 1) / 2;
         if (used <= sm_doubles) {
             S.D = used + (long long)dim * dim <= sm_doubles ? sm + used : A;
             for (int q = threadIdx.x; q < dim * dim; q += blockDim.x) S.D[q] = 0.0;
@@ -1525,7 +1659,7 @@ __device__ bool epsilon_fast(const FsiDev& F, const MarkerDev& M, int m0, int di
 
 // Direct path (marker sets beyond the shared-memory plan): entries evaluated
 // pair by pair, band LU in `smem` when it fits, else the dense LU in A.
-__device__ void epsilon_range(const FsiDev& F, const MarkerDev& M, int m0, int dim, double* A, double* bx, int* piv,
+__device__ __forceinline__ void epsilon_range(const FsiDev& F, const MarkerDev& M, int m0, int dim, double* A, double* bx, int* piv,
                               int* lmax, double* smem = nullptr, int smem_doubles = 0) {
     if (epsilon_fast(F, M, m0, dim, A, bx, piv, lmax, smem, smem_doubles)) return;
     __shared__ int s_kl, s_ku;
@@ -1590,19 +1724,19 @@ __device__ void epsilon_range(const FsiDev& F, const MarkerDev& M, int m0, int d
 
 constexpr int kEpsSmemDoubles = 25000;  // 200000 bytes of dynamic shared memory (opt-in)
 
-__global__ void __launch_bounds__(256) k_fsi_epsilon_body(FsiDev F, MarkerDev M) {
+__global__ void __launch_bounds__(256, 1) k_fsi_epsilon_body(FsiDev F, MarkerDev M) {
     extern __shared__ double eps_smem[];
     FemBodyDev& B = F.bodies[blockIdx.x];
     epsilon_range(F, M, B.mbase, B.nMark, B.epsA, B.epsB, B.piv, B.lmax, eps_smem, kEpsSmemDoubles);
 }
 
-__global__ void __launch_bounds__(256) k_fsi_epsilon_uni(FsiDev F, MarkerDev M) {
+__global__ void __launch_bounds__(256, 1) k_fsi_epsilon_uni(FsiDev F, MarkerDev M) {
     extern __shared__ double eps_smem[];
     epsilon_range(F, M, 0, M.n, F.uniA, F.uniB, F.uniPiv, F.uniLmax, eps_smem, kEpsSmemDoubles);
 }
 
 // FEMBodyClass::dynamicFEM (src/FEMBody.cpp:26-68) for one body per CTA.
-__global__ void __launch_bounds__(256) k_fem_dynamic(FsiDev F, MarkerDev M) {
+__global__ void __launch_bounds__(256, 1) k_fem_dynamic(FsiDev F, MarkerDev M) {
     FemBodyDev& B = F.bodies[blockIdx.x];
     __shared__ double s_res;
     __shared__ int s_it;
@@ -1932,7 +2066,7 @@ __global__ void __launch_bounds__(256) k_fem_dynamic(FsiDev F, MarkerDev M) {
 
 // Standalone epsilon solve over n markers with caller-provided scratch
 // (A: n*n, b: n, piv, lmax: n).
-__global__ void __launch_bounds__(256) k_epsilon_markers(FsiDev F, MarkerDev M, int n, double* A, double* b, int* piv,
+__global__ void __launch_bounds__(256, 1) k_epsilon_markers(FsiDev F, MarkerDev M, int n, double* A, double* b, int* piv,
                                                          int* lmax) {
     extern __shared__ double eps_smem[];
     epsilon_range(F, M, 0, n, A, b, piv, lmax, eps_smem, kEpsSmemDoubles);
