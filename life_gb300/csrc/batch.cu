@@ -225,7 +225,8 @@ static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* o
             c->t_dev = b->d_tnow + k;
             c->t_off = 1 + s;
             const int tt = c->t + 1;
-            const LatDev L = lattice_view(c, tt);
+            LatDev L = lattice_view(c, tt);
+            L.crowded = n > 1;
             e = cudaStreamWaitEvent(c->side, b->ev_fork, 0);
             const bool fused = fused_step(b);  // perimeter inside the interior launch
             if (L.convective && L.outlet_form == kOutletKernel) {

@@ -328,91 +328,144 @@ __host__ __device__ __forceinline__ bool site_range_ok(double ux, double uy, dou
     return velocity_in_range(ux) && velocity_in_range(uy) && w - (1023u - 50u) < 52u;
 }
 
+// A product, or 1/2, 1 or 2 plus x, by the integer units or (INT = false) by the FP64
+// unit: the same values (but for the sign of a zero product). Where the FP64
+// unit is busy the integer form is free; on a lone warp, whose time is a chain,
+// an FP64 product is the shorter one.
+template <bool INT, int ZERO = kZeroA>
+__host__ __device__ __forceinline__ double prod(double a, double b) {
+    return INT ? mul_int<ZERO>(a, b) : a * b;
+}
+template <bool INT>
+__host__ __device__ __forceinline__ double half_plus(double x) {
+    return INT ? add_pow2_int<-1>(x) : 0.5 + x;
+}
+template <bool INT>
+__host__ __device__ __forceinline__ double one_plus(double x) {
+    return INT ? add_pow2_int<0>(x) : 1.0 + x;
+}
+template <bool INT>
+__host__ __device__ __forceinline__ double two_plus(double x) {
+    return INT ? add_pow2_int<1>(x) : 2.0 + x;
+}
+
+// equilibrium<false>() and equilibrium<true>() of all nine directions (rho in
+// [2^-5, 2^3), velocity_in_range), the products that directions share formed
+// once.
+template <bool INT = true>
+__host__ __device__ __forceinline__ void equilibria_bgk_int(double rho, double ux, double uy, double feq[9]) {
+    const double px = prod<INT>(ux, 3.0), py = prod<INT>(uy, 3.0);
+    const double pa = prod<INT>(ux + uy, 3.0), pb = prod<INT>(ux - uy, 3.0);
+    const double d9 = prod<INT, kZeroAny>(prod<INT>(ux, 9.0), uy);
+    const double X2 = prod<INT>(ux, ux), Y2 = prod<INT>(uy, uy);
+    constexpr double c0 = 0.0 - 1.0 / 3.0, c1 = 1.0 - 1.0 / 3.0;
+    const double x0 = prod<INT>(X2, c0), x1 = prod<INT>(X2, c1), y0 = prod<INT>(Y2, c0), y1 = prod<INT>(Y2, c1);
+    const double h00 = prod<INT>(x0 + y0, 4.5), h10 = prod<INT>(x1 + y0, 4.5);
+    const double h01 = prod<INT>(x0 + y1, 4.5), h11 = prod<INT>(x1 + y1, 4.5);
+    const double r0 = prod<INT, kNonZero>(rho, 4.0 / 9.0), r1 = prod<INT, kNonZero>(rho, 1.0 / 9.0);
+    const double r2 = prod<INT, kNonZero>(rho, 1.0 / 36.0);
+    feq[0] = prod<INT, kNonZero>(one_plus<INT>(h00), r0);
+    feq[1] = prod<INT, kNonZero>(one_plus<INT>(px) + h10, r1);
+    feq[2] = prod<INT, kNonZero>(one_plus<INT>(-px) + h10, r1);
+    feq[3] = prod<INT, kNonZero>(one_plus<INT>(py) + h01, r1);
+    feq[4] = prod<INT, kNonZero>(one_plus<INT>(-py) + h01, r1);
+    feq[5] = prod<INT, kNonZero>((one_plus<INT>(pa) + h11) + d9, r2);
+    feq[6] = prod<INT, kNonZero>((one_plus<INT>(-pa) + h11) + d9, r2);
+    feq[7] = prod<INT, kNonZero>((one_plus<INT>(pb) + h11) + -d9, r2);
+    feq[8] = prod<INT, kNonZero>((one_plus<INT>(-pb) + h11) + -d9, r2);
+}
+template <bool INT = true>
+__host__ __device__ __forceinline__ void equilibria_cm_int(double rho, double ux, double uy, double feq[9]) {
+    // per axis 2 - 3 u^2 and ((9 u^2 +- 6 u) - 3 u^2) + 2
+    const double X2 = prod<INT>(ux, ux), Y2 = prod<INT>(uy, uy);
+    const double x3 = prod<INT>(X2, 3.0), x9 = prod<INT>(X2, 9.0), x6 = prod<INT>(ux, 6.0);
+    const double y3 = prod<INT>(Y2, 3.0), y9 = prod<INT>(Y2, 9.0), y6 = prod<INT>(uy, 6.0);
+    const double ax = two_plus<INT>(-x3), axp = two_plus<INT>((x9 + x6) - x3), axm = two_plus<INT>((x9 - x6) - x3);
+    const double ay = two_plus<INT>(-y3), ayp = two_plus<INT>((y9 + y6) - y3), aym = two_plus<INT>((y9 - y6) - y3);
+    const double rq = scale2_nz(rho, -2);
+    const double r0 = prod<INT, kNonZero>(rq, 4.0 / 9.0), r1 = prod<INT, kNonZero>(rq, 1.0 / 9.0);
+    const double r2 = prod<INT, kNonZero>(rq, 1.0 / 36.0);
+    const double c = prod<INT, kNonZero>(r1, ax), p = prod<INT, kNonZero>(r2, axp), m = prod<INT, kNonZero>(r2, axm);
+    feq[0] = prod<INT, kNonZero>(prod<INT, kNonZero>(r0, ax), ay);
+    feq[1] = prod<INT, kNonZero>(prod<INT, kNonZero>(r1, axp), ay);
+    feq[2] = prod<INT, kNonZero>(prod<INT, kNonZero>(r1, axm), ay);
+    feq[3] = prod<INT, kNonZero>(c, ayp);
+    feq[4] = prod<INT, kNonZero>(c, aym);
+    feq[5] = prod<INT, kNonZero>(p, ayp);
+    feq[6] = prod<INT, kNonZero>(m, aym);
+    feq[7] = prod<INT, kNonZero>(p, aym);
+    feq[8] = prod<INT, kNonZero>(m, ayp);
+}
+
+template <bool INT = true>
 __host__ __device__ __forceinline__ void collide_bgk_int(const double f[9], double rho, double ux, double uy,
                                                          double omega, double fs[9]) {
-    const double px = mul_int(ux, 3.0), py = mul_int(uy, 3.0);
-    const double pa = mul_int(ux + uy, 3.0), pb = mul_int(ux - uy, 3.0);
-    const double d9 = mul_int<kZeroAny>(mul_int(ux, 9.0), uy);
-    const double X2 = mul_int(ux, ux), Y2 = mul_int(uy, uy);
-    constexpr double c0 = 0.0 - 1.0 / 3.0, c1 = 1.0 - 1.0 / 3.0;
-    const double x0 = mul_int(X2, c0), x1 = mul_int(X2, c1), y0 = mul_int(Y2, c0), y1 = mul_int(Y2, c1);
-    const double h00 = mul_int(x0 + y0, 4.5), h10 = mul_int(x1 + y0, 4.5);
-    const double h01 = mul_int(x0 + y1, 4.5), h11 = mul_int(x1 + y1, 4.5);
-    const double r0 = mul_int<kNonZero>(rho, 4.0 / 9.0), r1 = mul_int<kNonZero>(rho, 1.0 / 9.0);
-    const double r2 = mul_int<kNonZero>(rho, 1.0 / 36.0);
     double feq[9];
-    feq[0] = mul_int<kNonZero>(add_pow2_int<0>(h00), r0);
-    feq[1] = mul_int<kNonZero>(add_pow2_int<0>(px) + h10, r1);
-    feq[2] = mul_int<kNonZero>(add_pow2_int<0>(-px) + h10, r1);
-    feq[3] = mul_int<kNonZero>(add_pow2_int<0>(py) + h01, r1);
-    feq[4] = mul_int<kNonZero>(add_pow2_int<0>(-py) + h01, r1);
-    feq[5] = mul_int<kNonZero>((add_pow2_int<0>(pa) + h11) + d9, r2);
-    feq[6] = mul_int<kNonZero>((add_pow2_int<0>(-pa) + h11) + d9, r2);
-    feq[7] = mul_int<kNonZero>((add_pow2_int<0>(pb) + h11) + -d9, r2);
-    feq[8] = mul_int<kNonZero>((add_pow2_int<0>(-pb) + h11) + -d9, r2);
+    equilibria_bgk_int<INT>(rho, ux, uy, feq);
 #pragma unroll
-    for (int v = 0; v < 9; v++) fs[v] = f[v] + mul_int(feq[v] - f[v], omega);
+    for (int v = 0; v < 9; v++) fs[v] = f[v] + prod<INT>(feq[v] - f[v], omega);
 }
 
 // om = 1 - omega, cs2 = cs^2, cs4 = cs^4 in the written-out form's operations.
+template <bool INT = true>
 __host__ __device__ __forceinline__ void collide_cm_int(const double f[9], double rho, double ux, double uy,
                                                         double om, double cs2, double cs4, double fs[9]) {
-    const double X2 = mul_int(ux, ux), Y2 = mul_int(uy, uy);
-    const double xm = add_pow2_int<0>(-ux), xq = add_pow2_int<0>(ux);
-    const double ym = add_pow2_int<0>(-uy), yq = add_pow2_int<0>(uy);
+    const double X2 = prod<INT>(ux, ux), Y2 = prod<INT>(uy, uy);
+    const double xm = one_plus<INT>(-ux), xq = one_plus<INT>(ux);
+    const double ym = one_plus<INT>(-uy), yq = one_plus<INT>(uy);
     const double D = X2 - Y2;
     double k4Pre, k5Pre;
     {
         // f (cx^2 - cy^2) and (f cx) cy with cx = c - ux: the components of
         // c = 0 and -1 are -ux and -(1 + ux); signs go into the sums
-        const double sxm = mul_int<kNonZero>(xm, xm), sxq = mul_int<kNonZero>(xq, xq);
-        const double sym = mul_int<kNonZero>(ym, ym), syq = mul_int<kNonZero>(yq, yq);
-        k4Pre = mul_int(D, f[0]);
-        k4Pre = k4Pre + mul_int(sxm - Y2, f[1]);
-        k4Pre = k4Pre + mul_int(sxq - Y2, f[2]);
-        k4Pre = k4Pre + mul_int(X2 - sym, f[3]);
-        k4Pre = k4Pre + mul_int(X2 - syq, f[4]);
-        k4Pre = k4Pre + mul_int(sxm - sym, f[5]);
-        k4Pre = k4Pre + mul_int(sxq - syq, f[6]);
-        k4Pre = k4Pre + mul_int(sxm - syq, f[7]);
-        k4Pre = k4Pre + mul_int(sxq - sym, f[8]);
-        k5Pre = mul_int<kZeroAny>(mul_int(ux, f[0]), uy);
-        k5Pre = k5Pre - mul_int(uy, mul_int<kNonZero>(xm, f[1]));
-        k5Pre = k5Pre + mul_int(uy, mul_int<kNonZero>(xq, f[2]));
-        k5Pre = k5Pre - mul_int(mul_int(ux, f[3]), ym);
-        k5Pre = k5Pre + mul_int(mul_int(ux, f[4]), yq);
-        k5Pre = k5Pre + mul_int<kNonZero>(ym, mul_int<kNonZero>(xm, f[5]));
-        k5Pre = k5Pre + mul_int<kNonZero>(yq, mul_int<kNonZero>(xq, f[6]));
-        k5Pre = k5Pre - mul_int<kNonZero>(yq, mul_int<kNonZero>(xm, f[7]));
-        k5Pre = k5Pre - mul_int<kNonZero>(ym, mul_int<kNonZero>(xq, f[8]));
+        const double sxm = prod<INT, kNonZero>(xm, xm), sxq = prod<INT, kNonZero>(xq, xq);
+        const double sym = prod<INT, kNonZero>(ym, ym), syq = prod<INT, kNonZero>(yq, yq);
+        k4Pre = prod<INT>(D, f[0]);
+        k4Pre = k4Pre + prod<INT>(sxm - Y2, f[1]);
+        k4Pre = k4Pre + prod<INT>(sxq - Y2, f[2]);
+        k4Pre = k4Pre + prod<INT>(X2 - sym, f[3]);
+        k4Pre = k4Pre + prod<INT>(X2 - syq, f[4]);
+        k4Pre = k4Pre + prod<INT>(sxm - sym, f[5]);
+        k4Pre = k4Pre + prod<INT>(sxq - syq, f[6]);
+        k4Pre = k4Pre + prod<INT>(sxm - syq, f[7]);
+        k4Pre = k4Pre + prod<INT>(sxq - sym, f[8]);
+        k5Pre = prod<INT, kZeroAny>(prod<INT>(ux, f[0]), uy);
+        k5Pre = k5Pre - prod<INT>(uy, prod<INT, kNonZero>(xm, f[1]));
+        k5Pre = k5Pre + prod<INT>(uy, prod<INT, kNonZero>(xq, f[2]));
+        k5Pre = k5Pre - prod<INT>(prod<INT>(ux, f[3]), ym);
+        k5Pre = k5Pre + prod<INT>(prod<INT>(ux, f[4]), yq);
+        k5Pre = k5Pre + prod<INT, kNonZero>(ym, prod<INT, kNonZero>(xm, f[5]));
+        k5Pre = k5Pre + prod<INT, kNonZero>(yq, prod<INT, kNonZero>(xq, f[6]));
+        k5Pre = k5Pre - prod<INT, kNonZero>(yq, prod<INT, kNonZero>(xm, f[7]));
+        k5Pre = k5Pre - prod<INT, kNonZero>(ym, prod<INT, kNonZero>(xq, f[8]));
     }
-    const double k4 = mul_int<kZeroAny>(om, pos_zero(k4Pre)), k5 = mul_int<kZeroAny>(om, pos_zero(k5Pre));
-    const double k3 = scale2_nz(mul_int<kNonZero>(rho, cs2), 1), k8 = mul_int<kNonZero>(rho, cs4);
-    const double XY = mul_int<kZeroAny>(ux, uy), W = scale2(XY, 1);
-    const double X2Y2 = mul_int<kZeroAny>(X2, Y2), uxY2 = mul_int<kZeroAny>(ux, Y2);
-    const double X2uy = mul_int<kZeroAny>(X2, uy);
+    const double k4 = prod<INT, kZeroAny>(om, pos_zero(k4Pre)), k5 = prod<INT, kZeroAny>(om, pos_zero(k5Pre));
+    const double k3 = scale2_nz(prod<INT, kNonZero>(rho, cs2), 1), k8 = prod<INT, kNonZero>(rho, cs4);
+    const double XY = prod<INT, kZeroAny>(ux, uy), W = scale2(XY, 1);
+    const double X2Y2 = prod<INT, kZeroAny>(X2, Y2), uxY2 = prod<INT, kZeroAny>(ux, Y2);
+    const double X2uy = prod<INT, kZeroAny>(X2, uy);
     const double A = X2 - X2Y2, Bq = X2uy - X2Y2, Sp = X2Y2 + X2uy;
     const double S = X2 + Y2, Qp = X2 + ux, Qm = X2 - ux, QpY = Qp + Y2, QmY = Qm + Y2, Rp = Qp - Y2, Rm = Qm - Y2;
     const double uyW = uy - W, dxy = ux - uy;
     // population: (((p0 k0 + p3 k3) + p4 k4) + p5 k5) +- k8, the moments scaled
     // by the powers of two of its class (Z3: whether p3 may be zero)
 #define LIFE_CM_POP(v, Z3, p0, p3, p4, p5, K0, K3, K4, K5, K8) \
-    fs[v] = (((mul_int(p0, K0) + mul_int<Z3>(p3, K3)) + mul_int<kZeroAny>(p4, K4)) + mul_int<kZeroAny>(p5, K5)) + (K8)
-    LIFE_CM_POP(0, kNonZero, add_pow2_int<0>(-A - Y2), -add_pow2_int<1>(-S), Y2 - X2, XY, rho, scale2_nz(k3, -1), scale2(k4, -1), scale2(k5, 2), k8);
+    fs[v] = (((prod<INT>(p0, K0) + prod<INT, Z3>(p3, K3)) + prod<INT, kZeroAny>(p4, K4)) + prod<INT, kZeroAny>(p5, K5)) + (K8)
+    LIFE_CM_POP(0, kNonZero, one_plus<INT>(-A - Y2), -two_plus<INT>(-S), Y2 - X2, XY, rho, scale2_nz(k3, -1), scale2(k4, -1), scale2(k5, 2), k8);
     {
         const double K0 = scale2_nz(rho, -1), K3 = scale2_nz(k3, -2), K4 = scale2(k4, -2), K8 = -scale2_nz(k8, -1);
-        LIFE_CM_POP(1, kNonZero, (A - uxY2) + ux, add_pow2_int<0>(-QpY), add_pow2_int<0>(Rp), -(uy + W), K0, K3, K4, k5, K8);
-        LIFE_CM_POP(2, kNonZero, (A + uxY2) - ux, add_pow2_int<0>(-QmY), add_pow2_int<0>(Rm), uyW, K0, K3, K4, k5, K8);
-        LIFE_CM_POP(3, kNonZero, ((Y2 - X2uy) - X2Y2) + uy, add_pow2_int<0>(-(S + uy)), -add_pow2_int<0>(uy - D), -(ux + W), K0, K3, K4, k5, K8);
-        LIFE_CM_POP(4, kNonZero, (Bq + Y2) - uy, add_pow2_int<0>(-(S - uy)), -add_pow2_int<0>(-(D + uy)), ux - W, K0, K3, K4, k5, K8);
+        LIFE_CM_POP(1, kNonZero, (A - uxY2) + ux, one_plus<INT>(-QpY), one_plus<INT>(Rp), -(uy + W), K0, K3, K4, k5, K8);
+        LIFE_CM_POP(2, kNonZero, (A + uxY2) - ux, one_plus<INT>(-QmY), one_plus<INT>(Rm), uyW, K0, K3, K4, k5, K8);
+        LIFE_CM_POP(3, kNonZero, ((Y2 - X2uy) - X2Y2) + uy, one_plus<INT>(-(S + uy)), -one_plus<INT>(uy - D), -(ux + W), K0, K3, K4, k5, K8);
+        LIFE_CM_POP(4, kNonZero, (Bq + Y2) - uy, one_plus<INT>(-(S - uy)), -one_plus<INT>(-(D + uy)), ux - W, K0, K3, K4, k5, K8);
     }
     {
         const double K0 = scale2_nz(rho, -2), K3 = scale2_nz(k3, -3), K4 = scale2(k4, -3), K5 = scale2(k5, -1);
         const double K8 = scale2_nz(k8, -2);
-        LIFE_CM_POP(5, kZeroA, (Sp + uxY2) + XY, QpY + uy, uy - Rp, add_pow2_int<-1>((ux + uy) + W), K0, K3, K4, K5, K8);
-        LIFE_CM_POP(6, kZeroA, XY - (Bq + uxY2), QmY - uy, -(Rm + uy), add_pow2_int<-1>(-(uyW + ux)), K0, K3, K4, K5, K8);
-        LIFE_CM_POP(7, kZeroA, (uxY2 - Bq) - XY, QpY - uy, -(Rp + uy), -add_pow2_int<-1>(dxy - W), K0, K3, K4, K5, K8);
-        LIFE_CM_POP(8, kZeroA, (Sp - uxY2) - XY, QmY + uy, uy - Rm, -add_pow2_int<-1>(-(dxy + W)), K0, K3, K4, K5, K8);
+        LIFE_CM_POP(5, kZeroA, (Sp + uxY2) + XY, QpY + uy, uy - Rp, half_plus<INT>((ux + uy) + W), K0, K3, K4, K5, K8);
+        LIFE_CM_POP(6, kZeroA, XY - (Bq + uxY2), QmY - uy, -(Rm + uy), half_plus<INT>(-(uyW + ux)), K0, K3, K4, K5, K8);
+        LIFE_CM_POP(7, kZeroA, (uxY2 - Bq) - XY, QpY - uy, -(Rp + uy), -half_plus<INT>(dxy - W), K0, K3, K4, K5, K8);
+        LIFE_CM_POP(8, kZeroA, (Sp - uxY2) - XY, QmY + uy, uy - Rm, -half_plus<INT>(-(dxy + W)), K0, K3, K4, K5, K8);
     }
 #undef LIFE_CM_POP
 }

@@ -623,10 +623,22 @@ __device__ __forceinline__ void store_history(const LatDev& L, int type, int i, 
     }
 }
 
-// Boundary-condition site q of the perimeter, enumerated bottom row, top row,
-// left column, right column: its step-t state by site_state() (regularised /
-// convective conditions applied), the outlet side outputs, and the collision
-// of the next step into B. FP64 arithmetic for every storage form.
+// One boundary-condition site (perimeter_site: number q of the perimeter,
+// enumerated bottom row, top row, left column, right column): its step-t state
+// by site_state() (regularised / convective conditions applied), the outlet
+// side outputs, and the collision of the next step into B. FP64 arithmetic for
+// every storage form.
+template <bool CM, class S>
+__device__ __forceinline__ void boundary_site(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
+                                              const LatDev& L, int t, int i, int j, const double* dU = nullptr) {
+    const int type = site_type(L, i, j);
+    if (type == LIFE_FLUID) return;
+    double f[9], rho, ux, uy;
+    site_state<CM, S>(A, L, t, i, j, f, rho, ux, uy, dU);
+    outlet_outputs(L, i, j, f, ux, uy);
+    store_history(L, type, i, j, rho, ux, uy);
+    store_collided<CM, S>(B, L, t + 1, i, j, f, rho, ux, uy, 0.0, 0.0);
+}
 template <bool CM, class S>
 __device__ __forceinline__ void perimeter_site(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
                                                const LatDev& L, int t, int q) {
@@ -637,13 +649,7 @@ __device__ __forceinline__ void perimeter_site(const typename S::T* __restrict__
     else if (q < 2 * Nx + (Ny - 2)) { i = 0; j = q - 2 * Nx + 1; }
     else if (q < 2 * Nx + 2 * (Ny - 2)) { i = Nx - 1; j = q - 2 * Nx - (Ny - 2) + 1; }
     else return;
-    const int type = site_type(L, i, j);
-    if (type == LIFE_FLUID) return;
-    double f[9], rho, ux, uy;
-    site_state<CM, S>(A, L, t, i, j, f, rho, ux, uy);
-    outlet_outputs(L, i, j, f, ux, uy);
-    store_history(L, type, i, j, rho, ux, uy);
-    store_collided<CM, S>(B, L, t + 1, i, j, f, rho, ux, uy, 0.0, 0.0);
+    boundary_site<CM, S>(A, B, L, t, i, j);
 }
 
 }  // namespace life

@@ -22,6 +22,7 @@
 #include "lbm_device.cuh"
 #include "lbm_kernels.h"
 #include "lbm_lanes.cuh"
+#include "lbm_walls.cuh"
 
 namespace life {
 
@@ -98,16 +99,6 @@ static __device__ __noinline__ void interior_site_general(const double* __restri
     const size_t s = (size_t)j * L.pitch + i;
 #pragma unroll
     for (int v = 0; v < 9; v++) B[(size_t)v * L.S + s] = fs[v];
-}
-
-// div_rn_recip for a zero numerator or operands within its window.
-__device__ __forceinline__ double quotient_in_range(double a, double b, double y) {
-    const double q0 = mul_int<kZeroAny>(a, y);
-    const double r0 = fma(-b, q0, a);
-    const double q1 = fma(r0, y, q0);
-    const double r1 = fma(-b, q1, a);
-    const double q = fma(r1, y, q1);
-    return (div_bits(a) << 1) == 0ull ? q0 : q;
 }
 
 template <bool CM, bool SITE>
@@ -204,14 +195,6 @@ __global__ void __launch_bounds__(256) k_interior_batch_f64(const BatchLatCase* 
             }
         }
     }
-}
-
-// Boundary-condition sites of one step, FP64 storage, three per warp
-// (lbm_lanes.cuh); the reduced-precision forms have theirs in lbm_lowp.cu.
-template <bool CM, class S>
-__global__ void __launch_bounds__(32) k_perimeter(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
-                                                  LatDev L, int t) {
-    lanes_perimeter<CM, S>(A, B, L, step_t(L, t), kLaneSites * (int)blockIdx.x);
 }
 
 // GridClass::convectiveSpeed (src/Grid.cpp:477-495): the mean outlet speed is
@@ -575,11 +558,7 @@ int batch_blocks_per_sm_f64(int tile_w) {
 
 cudaError_t launch_perimeter(const void* A, void* B, const LatDev& L, int t, cudaStream_t s) {
     if (L.prec != LIFE_PREC_F64) return launch_perimeter_lowp(A, B, L, t, s);
-    // one warp per block, spread over the SMs' FP64 units (as the
-    // reduced-precision perimeter)
-    const int n = 2 * L.Nx + 2 * (L.Ny - 2), g = (n + kLaneSites - 1) / kLaneSites;
-    if (L.cm) k_perimeter<true, StoreF64><<<g, 32, 0, s>>>((const double*)A, (double*)B, L, t);
-    else k_perimeter<false, StoreF64><<<g, 32, 0, s>>>((const double*)A, (double*)B, L, t);
+    launch_walls<StoreF64>(A, B, L, t, s);
     return cudaGetLastError();
 }
 

@@ -332,13 +332,11 @@ __device__ __forceinline__ bool perimeter_ij(const LatDev& L, int q, int& i, int
     return true;
 }
 
-// perimeter_site() for the three sites q0..q0+2 of a warp.
+// boundary_site() for the warp's three sites (`site`: whether this lane's is one).
 template <bool CM, class S>
-__device__ __forceinline__ void lanes_perimeter(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
-                                                const LatDev& L, int t, int q0) {
+__device__ __forceinline__ void lanes_boundary(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
+                                               const LatDev& L, int t, bool site, int i, int j) {
     const SiteLane g = site_lane();
-    int i = 0, j = 0;
-    const bool site = perimeter_ij(L, q0 + g.slot, i, j);
     const int type = site ? site_type(L, i, j) : LIFE_FLUID;
     if (!__any_sync(kAllLanes, type != LIFE_FLUID)) return;
     const bool store = g.store && type != LIFE_FLUID;

@@ -36,7 +36,7 @@
 #include <type_traits>
 
 #include "lbm_kernels.h"
-#include "lbm_lanes.cuh"
+#include "lbm_walls.cuh"
 #include "tma.cuh"
 
 namespace life {
@@ -402,27 +402,9 @@ cudaError_t launch_interior_lowp(const void* A, void* B, const LatDev& L, int t,
     return cudaGetLastError();
 }
 
-// Boundary-condition sites, reduced-precision storage, three per warp
-// (lbm_lanes.cuh; FP64 arithmetic, rounded as in lbm_f64.cu).
-template <bool CM, class S>
-__global__ void __launch_bounds__(32) k_perimeter_lowp(const typename S::T* __restrict__ A,
-                                                       typename S::T* __restrict__ B, LatDev L, int t) {
-    lanes_perimeter<CM, S>(A, B, L, step_t(L, t), kLaneSites * (int)blockIdx.x);
-}
-
-// One warp per block: a boundary site is a long FP64 chain, and an SM's FP64
-// unit is narrow, so the sites are spread over as many SMs as possible
-// rather than packed four warps to an SM.
 cudaError_t launch_perimeter_lowp(const void* A, void* B, const LatDev& L, int t, cudaStream_t s) {
-    const int n = 2 * L.Nx + 2 * (L.Ny - 2);
-    const int g = (n + kLaneSites - 1) / kLaneSites;
-    if (L.prec == LIFE_PREC_F32) {
-        if (L.cm) k_perimeter_lowp<true, StoreF32><<<g, 32, 0, s>>>((const float*)A, (float*)B, L, t);
-        else k_perimeter_lowp<false, StoreF32><<<g, 32, 0, s>>>((const float*)A, (float*)B, L, t);
-    } else {
-        if (L.cm) k_perimeter_lowp<true, StoreF16><<<g, 32, 0, s>>>((const __half*)A, (__half*)B, L, t);
-        else k_perimeter_lowp<false, StoreF16><<<g, 32, 0, s>>>((const __half*)A, (__half*)B, L, t);
-    }
+    if (L.prec == LIFE_PREC_F32) launch_walls<StoreF32>(A, B, L, t, s);
+    else launch_walls<StoreF16>(A, B, L, t, s);
     return cudaGetLastError();
 }
 
