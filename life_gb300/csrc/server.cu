@@ -86,7 +86,14 @@ struct LifeServer {
 
     double now() const { return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count(); }
     void loop();
+    bool can_admit();
 };
+
+// Whether the queue's first request could be admitted beside the active ones.
+bool LifeServer::can_admit() {
+    if (queue.empty() || (cfg.max_active > 0 && (int)active.size() >= cfg.max_active)) return false;
+    return st.bytes_in_use + reqs[queue.front()].estimate <= cfg.hbm_budget;
+}
 
 void LifeServer::loop() {
     cudaSetDevice(device);
@@ -219,9 +226,21 @@ void LifeServer::loop() {
         bool all_failed = false;
         std::string all_msg;
         int all_code = 0;
-        if (chunk > 0) {
+        // With the default round length the round is taken in slices that double
+        // from 8 steps, and ends between two of them when a request could join:
+        // requests that arrive together run together, where the first used to
+        // run its whole round alone (six 100-step canopies: 102 -> 83 ms).
+        int done = 0, slice = cfg.steps_per_round > 0 ? chunk : 8;
+        while (done < chunk && failed.empty() && !all_failed) {
+            if (done > 0) {
+                std::lock_guard<std::mutex> lk(mu);
+                if (stop || can_admit()) break;
+            }
+            const int n = std::min(slice, chunk - done);
+            done += n;
+            slice *= 2;
             for (auto& g : groups) {
-                int rc = batch_steps(g.second, chunk);
+                int rc = batch_steps(g.second, n);
                 if (!rc) continue;
                 int code = 0;
                 const int k = batch_failed_case(g.second, &code);
@@ -239,6 +258,7 @@ void LifeServer::loop() {
                 }
             }
         }
+        if (chunk > 0) chunk = done;
         {
             std::lock_guard<std::mutex> lk(mu);
             st.rounds++;
