@@ -51,9 +51,10 @@ namespace life {
 // lane's multiply and add into an fma (with the __fmul2_rn / __fadd2_rn
 // intrinsics and with this inline PTX alike; measured as one unit in the
 // last place on ~1 site in 10^6 per step), which the one-site path, compiled
-// without contraction, does not do. The BGK collision below is therefore
-// written so that no product feeds an addition, and the packed form is used
-// for BGK only.
+// without contraction, does not do. The collisions below are therefore
+// written so that no packed product feeds an addition, unless it is exact (by
+// a power of two) and fusing it changes nothing; mul_alone forms the two
+// products of the central moments that do, one lane at a time.
 struct V2 {
     unsigned long long b;  // lane x in the low 32 bits, lane y in the high 32 bits
     __device__ __forceinline__ float x() const {
@@ -114,16 +115,23 @@ template <class T> __device__ __forceinline__ T zero_of();
 template <> __device__ __forceinline__ float zero_of<float>() { return 0.0f; }
 template <> __device__ __forceinline__ V2 zero_of<V2>() { return v2(0.0f); }
 
+// A product that an addition takes, rounded by itself (see V2).
+__device__ __forceinline__ float mul_alone(float a, float b) { return a * b; }
+__device__ __forceinline__ V2 mul_alone(V2 a, V2 b) {
+    return v2(__fmul_rn(a.x(), b.x()), __fmul_rn(a.y(), b.y()));
+}
+
+// One axis of the rest part: u2 = u^2 rounded.
 template <class T>
-__device__ __forceinline__ void e1d(T u, T e[3], float w[3], T d[3]) {
+__device__ __forceinline__ void e1d(T u, T u2, T e[3], float w[3], T d[3]) {
     // index 0: c = 0, 1: c = +1, 2: c = -1
-    const T u2 = u * u;
     w[0] = 2.0f / 3.0f;
     w[1] = w[2] = 1.0f / 6.0f;
-    d[0] = -u2;
-    d[1] = fmaf(0.5f, u, 0.5f * u2);
-    d[2] = fmaf(-0.5f, u, 0.5f * u2);
-    e[0] = w[0] + d[0];
+    const T h2 = 0.5f * u2;
+    d[0] = (-1.0f) * u2;
+    d[1] = fmaf(0.5f, u, h2);
+    d[2] = fmaf(-0.5f, u, h2);
+    e[0] = w[0] - u2;
     e[1] = w[1] + d[1];
     e[2] = w[2] + d[2];
 }
@@ -144,7 +152,7 @@ __device__ __forceinline__ T cdot(int v, T a, T b) {
 // FORCED = false: the force of this step is zero everywhere (no gravity, no
 // Womersley term), so every forcing term is an exact zero and is not formed.
 // px, py: the momentum with the half force term, inv = 1/rho (ux = px inv,
-// uy = py inv). In BGK no product feeds an addition: c.u of a diagonal
+// uy = py inv). No packed product feeds an addition: in BGK c.u of a diagonal
 // direction is (px +- py) inv, and w (rho inner + dr) - g is one fused
 // multiply-add. A compiler that fuses a product into a following addition
 // (as one did for the packed two-site form) then has nothing to fuse, so the
@@ -208,60 +216,81 @@ __device__ __forceinline__ void collide_dev32(const T g[9], const T r[9], T dr, 
         const T dxxyy = (g[1] + g[2]) - (g[3] + g[4]);
         const T gxy = (g[5] + g[6]) - (g[7] + g[8]);
         const float om1 = 1.0f - omega;
-        const T k4 = om1 * fmaf(ux * ux - uy * uy, rho, fmaf(2.0f * uy, my, fmaf(-2.0f * ux, mx, dxxyy)));
-        const T k5 = om1 * fmaf(ux * uy, rho, fmaf(-ux, my, fmaf(-uy, mx, gxy)));
+        // Bound by instruction issue (297 warp instructions a site with every
+        // column entry formed as written and one site a thread: 74 % of issue
+        // slots, 76.6 us for 3001 x 2203 FP16 sites). The entries of the inverse
+        // transform share factors up to a sign or a power of two, so each is
+        // formed once and its sign and power sit in a multiple of the moment:
+        // exact, so every population is the one of the plain form. Packed for
+        // two sites that is about 160 operations: 68.1 us, and with a force
+        // 94.2 -> 79.4 us (3000 x 2200; FP32 98.8 -> 86.0 us).
+        // The only inexact products that feed additions are the two squares:
+        // mul_alone keeps them apart.
+        const T X2 = mul_alone(ux, ux), Y2 = mul_alone(uy, uy), XY = ux * uy;
+        const T XmY = X2 - Y2, nux = (-1.0f) * ux, nuy = (-1.0f) * uy;
+        const T k4 = om1 * fmaf(XmY, rho, fmaf(2.0f * uy, my, fmaf(2.0f * nux, mx, dxxyy)));
+        const T k5 = om1 * fmaf(XY, rho, fmaf(nux, my, fmaf(nuy, mx, gxy)));
         // force moments (exact zeros, and unused, when not FORCED)
         const float k1 = FORCED ? 0.5f * Gx : 0.0f, k2 = FORCED ? 0.5f * Gy : 0.0f;
         const float k7 = FORCED ? Gx * (1.0f / 6.0f) : 0.0f, k6 = FORCED ? Gy * (1.0f / 6.0f) : 0.0f;
         T ex[3], dx[3], ey[3], dy[3];
-        float wx[3], wy[3];
-        e1d(ux, ex, wx, dx);
-        e1d(uy, ey, wy, dy);
-        const T X2 = ux * ux, Y2 = uy * uy, XY = ux * uy;
-        // T_v1..T_v7 (force/stress columns of the inverse transform)
-        T T1[9], T2[9], T4[9], T5[9], T6[9], T7[9];
-        T1[0] = 2.0f * ux * (Y2 - 1.0f);          T2[0] = 2.0f * uy * (X2 - 1.0f);
-        T4[0] = -0.5f * (X2 - Y2);                T5[0] = 4.0f * XY;
-        T6[0] = 2.0f * uy;                        T7[0] = 2.0f * ux;
-        T1[1] = -0.5f * (2.0f * ux + 1.0f) * (Y2 - 1.0f);  T2[1] = -XY * (ux + 1.0f);
-        T4[1] = 0.25f * (X2 + ux - Y2 + 1.0f);    T5[1] = -uy * (2.0f * ux + 1.0f);
-        T6[1] = -uy;                              T7[1] = -0.5f * (2.0f * ux + 1.0f);
-        T1[2] = -0.5f * (2.0f * ux - 1.0f) * (Y2 - 1.0f);  T2[2] = -XY * (ux - 1.0f);
-        T4[2] = 0.25f * (X2 - ux - Y2 + 1.0f);    T5[2] = -uy * (2.0f * ux - 1.0f);
-        T6[2] = -uy;                              T7[2] = -0.5f * (2.0f * ux - 1.0f);
-        T1[3] = -XY * (uy + 1.0f);                T2[3] = -0.5f * (X2 - 1.0f) * (2.0f * uy + 1.0f);
-        T4[3] = 0.25f * (X2 - Y2 - uy - 1.0f);    T5[3] = -ux * (2.0f * uy + 1.0f);
-        T6[3] = -0.5f * (2.0f * uy + 1.0f);       T7[3] = -ux;
-        T1[4] = -XY * (uy - 1.0f);                T2[4] = -0.5f * (X2 - 1.0f) * (2.0f * uy - 1.0f);
-        T4[4] = 0.25f * (X2 - Y2 + uy - 1.0f);    T5[4] = -ux * (2.0f * uy - 1.0f);
-        T6[4] = -0.5f * (2.0f * uy - 1.0f);       T7[4] = -ux;
-        T1[5] = 0.25f * uy * (2.0f * ux + 1.0f) * (uy + 1.0f);  T2[5] = 0.25f * ux * (ux + 1.0f) * (2.0f * uy + 1.0f);
-        T4[5] = -0.125f * (ux - uy) * (ux + uy + 1.0f);          T5[5] = 0.25f * (2.0f * ux + 1.0f) * (2.0f * uy + 1.0f);
-        T6[5] = 0.25f * (2.0f * uy + 1.0f);                      T7[5] = 0.25f * (2.0f * ux + 1.0f);
-        T1[6] = 0.25f * uy * (2.0f * ux - 1.0f) * (uy - 1.0f);  T2[6] = 0.25f * ux * (ux - 1.0f) * (2.0f * uy - 1.0f);
-        T4[6] = -0.125f * (ux - uy) * (ux + uy - 1.0f);          T5[6] = 0.25f * (2.0f * ux - 1.0f) * (2.0f * uy - 1.0f);
-        T6[6] = 0.25f * (2.0f * uy - 1.0f);                      T7[6] = 0.25f * (2.0f * ux - 1.0f);
-        T1[7] = 0.25f * uy * (2.0f * ux + 1.0f) * (uy - 1.0f);  T2[7] = 0.25f * ux * (ux + 1.0f) * (2.0f * uy - 1.0f);
-        T4[7] = -0.125f * (ux + uy) * (ux - uy + 1.0f);          T5[7] = 0.25f * (2.0f * ux + 1.0f) * (2.0f * uy - 1.0f);
-        T6[7] = 0.25f * (2.0f * uy - 1.0f);                      T7[7] = 0.25f * (2.0f * ux + 1.0f);
-        T1[8] = 0.25f * uy * (2.0f * ux - 1.0f) * (uy + 1.0f);  T2[8] = 0.25f * ux * (ux - 1.0f) * (2.0f * uy + 1.0f);
-        T4[8] = -0.125f * (ux + uy) * (ux - uy - 1.0f);          T5[8] = 0.25f * (2.0f * ux - 1.0f) * (2.0f * uy + 1.0f);
-        T6[8] = 0.25f * (2.0f * uy + 1.0f);                      T7[8] = 0.25f * (2.0f * ux - 1.0f);
+        float w[3];
+        e1d(ux, X2, ex, w, dx);
+        e1d(uy, Y2, ey, w, dy);
+        // Columns of the inverse transform, as (factor, multiple of the moment):
+        // powers of two and signs sit in the multiples (exact), so each is formed
+        // once. Stress k4: (X2 - Y2) / -2; ((X2 +- ux) - Y2 + 1) / 4;
+        // ((X2 - Y2) -+ uy - 1) / 4; (ux - uy)(ux + uy +- 1) / -8,
+        // (ux + uy)(ux - uy +- 1) / -8. Stress k5: 4 XY; -uy (2 ux +- 1);
+        // -ux (2 uy +- 1); (2 ux +- 1)(2 uy +- 1) / 4.
+        const T xp = fmaf(2.0f, ux, 1.0f), xm = fmaf(2.0f, ux, -1.0f);
+        const T yp = fmaf(2.0f, uy, 1.0f), ym = fmaf(2.0f, uy, -1.0f);
+        const T su = ux + uy, di = ux - uy;
+        const T q4 = 0.25f * k4, e4 = -0.125f * k4, n5 = (-1.0f) * k5, q5 = 0.25f * k5;
 #pragma unroll
         for (int v = 0; v < 9; v++) {
             const int a = ax(cx_of(v)), b = ax(cy_of(v));
-            const T E = ex[a] * ey[b];
-            const T D = fmaf(dx[a], dy[b], fmaf(wx[a], dy[b], dx[a] * wy[b]));
-            T acc = fmaf(dr, E, D);
+            const T D = fmaf(dx[a], dy[b], fmaf(w[a], dy[b], w[b] * dx[a]));
+            T acc = fmaf(dr, ex[a] * ey[b], D);
+            const T x = a == 1 ? xp : xm, y = b == 1 ? yp : ym;  // 2 u + c
             if (FORCED) {
-                acc = fmaf(T1[v], k1, acc);
-                acc = fmaf(T2[v], k2, acc);
+                T T1, T2;
+                if (v == 0) {
+                    T1 = 2.0f * ux * (Y2 - 1.0f);
+                    T2 = 2.0f * uy * (X2 - 1.0f);
+                } else if (b == 0) {
+                    T1 = -0.5f * x * (Y2 - 1.0f);
+                    T2 = (-1.0f) * XY * (a == 1 ? ux + 1.0f : ux - 1.0f);
+                } else if (a == 0) {
+                    T1 = (-1.0f) * XY * (b == 1 ? uy + 1.0f : uy - 1.0f);
+                    T2 = -0.5f * (X2 - 1.0f) * y;
+                } else {
+                    T1 = 0.25f * uy * x * (b == 1 ? uy + 1.0f : uy - 1.0f);
+                    T2 = 0.25f * ux * (a == 1 ? ux + 1.0f : ux - 1.0f) * y;
+                }
+                acc = fmaf(T1, k1, acc);
+                acc = fmaf(T2, k2, acc);
             }
-            acc = fmaf(T4[v], k4, acc);
-            acc = fmaf(T5[v], k5, acc);
+            if (v == 0) {
+                acc = fmaf(XmY, -0.5f * k4, acc);
+                acc = fmaf(XY, 4.0f * k5, acc);
+            } else if (b == 0) {
+                acc = fmaf(((a == 1 ? X2 + ux : X2 - ux) - Y2) + 1.0f, q4, acc);
+                acc = fmaf(uy * x, n5, acc);
+            } else if (a == 0) {
+                acc = fmaf((b == 1 ? XmY - uy : XmY + uy) - 1.0f, q4, acc);
+                acc = fmaf(ux * y, n5, acc);
+            } else {
+                const T one = a == b ? di * (a == 1 ? su + 1.0f : su - 1.0f)
+                                     : su * (a == 1 ? di + 1.0f : di - 1.0f);
+                acc = fmaf(one, e4, acc);
+                acc = fmaf(x * y, q5, acc);
+            }
             if (FORCED) {
-                acc = fmaf(T6[v], k6, acc);
-                acc = fmaf(T7[v], k7, acc);
+                const T T6 = v == 0 ? 2.0f * uy : (b == 0 ? nuy : (a == 0 ? -0.5f * y : 0.25f * y));
+                const T T7 = v == 0 ? 2.0f * ux : (b == 0 ? -0.5f * x : (a == 0 ? nux : 0.25f * x));
+                acc = fmaf(T6, k6, acc);
+                acc = fmaf(T7, k7, acc);
             }
             gs[v] = acc;
         }
@@ -451,8 +480,8 @@ __global__ void __launch_bounds__(256, 6) k_step_lowp(const typename S::T* __res
 // all nine population planes, into one of the shared-memory stages, while the
 // CTA computes an earlier tile; the copy's completion is counted on the
 // stage's mbarrier. The sites then read their nine pulled populations from
-// shared memory and finish exactly as in the one-site path
-// (finish_site_lowp), so the results are the same bits. The first blocks of
+// shared memory, two per thread, and finish with the arithmetic of the one-site
+// path (finish_site_lowp), so the results are the same bits. The first blocks of
 // the grid take the boundary-condition sites and the periodic edge sites, as
 // in k_step_lowp.
 template <class S>
@@ -501,27 +530,6 @@ struct TmaShape {
 // LIFE_ERR_TIMEOUT).
 __device__ int g_tma_timeouts;
 
-template <bool CM, bool FORCED, class S>
-__device__ __forceinline__ void tma_tile_sites(const unsigned char* stage, typename S::T* __restrict__ B,
-                                               const LatDev& L, int t, int i0, int j0) {
-    using TT = TmaTile<S>;
-    using SH = TmaShape<S>;
-    const int ii = (int)threadIdx.x % TT::W;
-    const int i = i0 + ii;
-    if (i < 1 || i > L.Nx - 2) return;
-    for (int jj = (int)threadIdx.x / TT::W; jj < TT::H; jj += (int)blockDim.x / TT::W) {
-        const int j = j0 + jj;
-        if (j > L.Ny - 2) break;
-        float r[9];
-#pragma unroll
-        for (int v = 0; v < 9; v++) {
-            const typename S::T* plane = reinterpret_cast<const typename S::T*>(stage + v * SH::PLANE);
-            r[v] = S::raw(plane[(jj + 1 - cy_of(v)) * SH::Wb + (ii + TT::HALO - cx_of(v))]);
-        }
-        finish_site_lowp<CM, FORCED, S>(r, B, L, t, i, j);
-    }
-}
-
 // Two adjacent stored values as floats (S::raw of each), and back (S::put_raw).
 template <class S>
 struct PairIO;
@@ -550,7 +558,7 @@ struct PairIO<StoreF32> {
     }
 };
 
-// BGK tiles with two x-adjacent sites per thread (an even column and the
+// Tiles with two x-adjacent sites per thread (an even column and the
 // next): paired loads where the pulled pair is aligned (directions with no x
 // component), the collision in packed FP32x2 (V2), and one paired store per
 // direction. Each lane computes exactly what finish_site_lowp computes for
@@ -559,7 +567,7 @@ struct PairIO<StoreF32> {
 // convective outlet's last three columns (which also write side outputs),
 // take the one-site path.
 // The pair of columns (ii, ii+1) of tile row jj.
-template <bool FORCED, class S>
+template <bool CM, bool FORCED, class S>
 __device__ __forceinline__ void tma_pair(const unsigned char* stage, typename S::T* __restrict__ B, const LatDev& L,
                                          int t, int i0, int j0, int jj, int ii) {
     using T = typename S::T;
@@ -579,7 +587,7 @@ __device__ __forceinline__ void tma_pair(const unsigned char* stage, typename S:
                 const T* plane = reinterpret_cast<const T*>(stage + v * SH::PLANE);
                 r[v] = S::raw(plane[(jj + 1 - cy_of(v)) * SH::Wb + (ii + q + TT::HALO - cx_of(v))]);
             }
-            finish_site_lowp<false, FORCED, S>(r, B, L, t, iq, j);
+            finish_site_lowp<CM, FORCED, S>(r, B, L, t, iq, j);
         }
         return;
     }
@@ -607,10 +615,11 @@ __device__ __forceinline__ void tma_pair(const unsigned char* stage, typename S:
     const V2 px = FORCED ? fmaf(0.5f, Fxd, mx) : mx, py = FORCED ? fmaf(0.5f, Fyd, my) : my;
     const V2 ux = px * inv, uy = py * inv;
     V2 gs[9];
-    collide_dev32<false, FORCED, S::SCALED>(g, r, dr, rho, mx, my, ux, uy, px, py, inv, Gxd, Gyd, L.omega_f, gs);
+    collide_dev32<CM, FORCED, S::SCALED && !CM>(g, r, dr, rho, mx, my, ux, uy, px, py, inv, Gxd, Gyd, L.omega_f, gs);
     T* out = B + (size_t)j * L.pitch + i;
 #pragma unroll
-    for (int v = 0; v < 9; v++) PairIO<S>::store2(out + (size_t)v * L.S, gs[v]);
+    for (int v = 0; v < 9; v++)
+        PairIO<S>::store2(out + (size_t)v * L.S, S::SCALED && CM ? gs[v] * h16_inv(v) : gs[v]);
 }
 
 // The last CTA of a launch to finish clears the tile counters for the next
@@ -627,7 +636,7 @@ __device__ __forceinline__ void step_tma_done(int* ctr, int ncta) {
     }
 }
 
-// BGK tiles with a pipeline per warp instead of CTA barriers: the warps
+// Tiles with a pipeline per warp instead of CTA barriers: the warps
 // share each tile's site pairs (two sites per lane per pass). Stage s has a
 // "full" mbarrier (the producer's arrival with the copies' byte count, or a
 // plain arrival with tile -1 when the counter is exhausted) and an "empty"
@@ -636,7 +645,7 @@ __device__ __forceinline__ void step_tma_done(int* ctr, int ncta) {
 // k-1 with tile k+NST-1 once all warps have released it. A warp therefore
 // waits only for its own data and, through the producer, for the slowest
 // warp two tiles back, not for every warp at every tile.
-template <class S>
+template <bool CM, class S>
 __device__ __forceinline__ void tma_tiles_by_warp(const CUtensorMap& tm, typename S::T* __restrict__ B,
                                                   const LatDev& L, int t, int tiles_x, int ntiles,
                                                   unsigned char* smem) {
@@ -700,8 +709,8 @@ __device__ __forceinline__ void tma_tiles_by_warp(const CUtensorMap& tm, typenam
         const int i0 = (tile % tiles_x) * TT::W, j0 = 1 + (tile / tiles_x) * TT::H;
         // pair p of the tile: row p / 64, columns 2 (p % 64) and the next
         for (int p = warp * 32 + lane; p < TT::H * (TT::W / 2); p += NW * 32) {
-            if (forced) tma_pair<true, S>(smem + st * SH::STAGE, B, L, t, i0, j0, p / (TT::W / 2), 2 * (p % (TT::W / 2)));
-            else tma_pair<false, S>(smem + st * SH::STAGE, B, L, t, i0, j0, p / (TT::W / 2), 2 * (p % (TT::W / 2)));
+            if (forced) tma_pair<CM, true, S>(smem + st * SH::STAGE, B, L, t, i0, j0, p / (TT::W / 2), 2 * (p % (TT::W / 2)));
+            else tma_pair<CM, false, S>(smem + st * SH::STAGE, B, L, t, i0, j0, p / (TT::W / 2), 2 * (p % (TT::W / 2)));
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[st]);
@@ -719,7 +728,6 @@ __global__ void __launch_bounds__(256, TmaTile<S>::CTAS) k_step_tma(const __grid
                                                   LatDev L, int t, int pb, int tiles_x, int ntiles) {
     using TT = TmaTile<S>;
     using SH = TmaShape<S>;
-    constexpr int NST = SH::NST;
     t = step_t(L, t);
     if ((int)blockIdx.x < pb) {
         // boundary-condition sites; an edge site of a periodic wall is an
@@ -733,63 +741,8 @@ __global__ void __launch_bounds__(256, TmaTile<S>::CTAS) k_step_tma(const __grid
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) &
                                                            ~static_cast<uintptr_t>(127));
-    const int ncta = (int)gridDim.x - pb;
-    int* ctr = L.tile_ctr;  // [0]: tiles handed out, [1]: CTAs finished
-    if constexpr (!CM) {
-        tma_tiles_by_warp<S>(tm, B, L, t, tiles_x, ntiles, smem);
-        step_tma_done(ctr, ncta);
-        return;
-    }
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + NST * SH::STAGE);
-    int* s_tile = reinterpret_cast<int*>(smem + NST * SH::STAGE + 8 * NST);  // tile held by each stage, or -1
-    int& s_ok = s_tile[NST];
-    if (threadIdx.x == 0) {
-        for (int q = 0; q < NST; q++) mbar_init(&bar[q], 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    auto issue = [&](int tile, int st) {
-        const int i0 = (tile % tiles_x) * TT::W, j0 = 1 + (tile / tiles_x) * TT::H;
-        mbar_arrive_expect_tx(&bar[st], 9u * SH::BOX);
-        tma_load_3d(smem + st * SH::STAGE, &tm, i0 - TT::HALO, j0 - 1, 0, &bar[st]);
-    };
-    // Tiles are handed out by a counter, so CTAs that start late (behind the
-    // boundary blocks) take fewer tiles and the step ends evenly. The stage of
-    // tile k+NST-1 is filled while tile k is computed; it is the stage tile
-    // k-1 used. The results do not depend on which CTA takes which tile.
-    auto grab = [&](int st) {
-        const int tile = atomicAdd(&ctr[0], 1);
-        s_tile[st] = tile < ntiles ? tile : -1;
-        if (tile < ntiles) issue(tile, st);
-    };
-    if (threadIdx.x == 0)
-        for (int q = 0; q < NST - 1; q++) grab(q);
-    const bool forced = lattice_forced(L);
-    for (int k = 0;; k++) {
-        const int st = k % NST;
-        if (threadIdx.x == 0) {
-            fence_proxy_async_smem();
-            grab((k + NST - 1) % NST);
-            s_ok = 1;
-            if (s_tile[st] >= 0 && !mbar_wait_bounded(&bar[st], (unsigned)(k / NST) & 1u, 1u << 22)) {
-                // give the copies in flight into the other stages time to land
-                // before the CTA (and its shared memory) goes away
-                for (int q = 1; q < NST; q++)
-                    if (s_tile[(k + q) % NST] >= 0)
-                        mbar_wait_bounded(&bar[(k + q) % NST], (unsigned)((k + q) / NST) & 1u, 1u << 22);
-                atomicAdd(&g_tma_timeouts, 1);
-                s_ok = 0;
-            }
-        }
-        __syncthreads();
-        const int tile = s_tile[st];
-        if (tile < 0 || !s_ok) break;
-        const int i0 = (tile % tiles_x) * TT::W, j0 = 1 + (tile / tiles_x) * TT::H;
-        if (forced) tma_tile_sites<CM, true, S>(smem + st * SH::STAGE, B, L, t, i0, j0);
-        else tma_tile_sites<CM, false, S>(smem + st * SH::STAGE, B, L, t, i0, j0);
-        __syncthreads();
-    }
-    step_tma_done(ctr, ncta);
+    tma_tiles_by_warp<CM, S>(tm, B, L, t, tiles_x, ntiles, smem);
+    step_tma_done(L.tile_ctr, (int)gridDim.x - pb);
 }
 
 // The tensor map of one population buffer: dims (pitch, Ny, 9 planes), box
@@ -854,7 +807,9 @@ int tma_timeouts() {
 // Which step kernel a reduced-precision case uses: the TMA-staged tiles
 // (k_step_tma) for both storage forms; the one-site kernel (k_step_lowp) is
 // kept for comparison. Measured at 4096^2: FP16 95.6-99.6k (one-site) against
-// 159k MLUPS (staged), FP32 85.8-86.3k against 90.2-90.9k.
+// 159k MLUPS (staged), FP32 85.8-86.3k against 90.2-90.9k; with central moments
+// and FP16 at 3001 x 2203 the staged form takes 68.1 us a step (76.6 with one
+// site a thread in the staged form).
 // LIFE_STEP_KERNEL=site|tma overrides, for measurements and for the tests
 // that compare the two bit for bit.
 enum { STEP_SITE = 1, STEP_TMA = 3 };
