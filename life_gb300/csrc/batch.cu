@@ -6,8 +6,8 @@
 //     (k_interior_batch_*): the batch is cut into tiles of tile_w x tile_h
 //     sites, case k owning tiles [tile0_k, tile0_k + tiles_k), and each CTA
 //     walks the tile list with a grid-stride loop;
-//   * the rest of a step (convective outlet, boundary perimeter, IBM interp /
-//     FSI subiteration loop / spread) runs per case on the case's own stream,
+//   * the rest of a step (boundary sites, IBM interp / FSI subiteration loop /
+//     spread) runs per case on the case's own stream,
 //     so the cases overlap on the device;
 //   * one whole batch step is captured into a CUDA graph, once per step
 //     parity (the ping-pong buffers and outlet buffers alternate), and
@@ -375,10 +375,10 @@ static int check_status(LifeBatch* b) {
 
 // Steps the next graph launch may take: kChain for a single case without
 // flexible bodies on a lattice below 2^22 sites, whose steps are so short that
-// the launch of each step's graph and its step-counter kernel show: 16 steps
-// in one graph against one took a 256^2 FP64 cavity from 28.9 to 24.0 us and a
-// 1501 x 703 FP32 channel from 28.3 to 23.9 us per step.
-// Larger lattices and flexible bodies step in 0.1 ms and more, and a batch of
+// the launch of each step's graph and its step-counter kernel show: a
+// 1501 x 703 FP32 channel takes 17.3 us a step with 16 steps in one graph and
+// 23.1 with two.
+// Larger lattices and flexible bodies step in 0.07 ms and more, and a batch of
 // several cases in about 1 ms. The chain is captured when a run is long enough
 // to repay it.
 static int chain_steps(LifeBatch* b, int left, int ph) {

@@ -10,7 +10,8 @@
 //   k_perimeter     the same for boundary-condition sites, with the
 //                   regularised / convective conditions applied
 //   k_outlet_f64    convective outlet speed (sequential mean, as the reference;
-//                   a fixed-order tree sum for the reduced-precision forms)
+//                   a fixed-order tree sum for the reduced-precision forms), for
+//                   the one-launch step kernels; other steps form it in place
 //   k_state         collision from an explicit state (restart read)
 //   k_export        reference-layout fields of the current step
 //   k_maxvel        max |u| and NaN scan
@@ -160,8 +161,8 @@ __device__ __forceinline__ void interior_site_f64(const double* __restrict__ A, 
     }
 }
 
-// (Five blocks of 96 registers an SM: 0.717 ms against 0.737 with 106
-// registers and four, 0.741 with seven, 1536 x 1536 central moments.)
+// (Five blocks of 96 registers an SM: 0.672 ms a step against 0.701 with four
+// and 0.689 with six, 1536 x 1536 central moments.)
 template <bool CM, bool SITE>
 __global__ void __launch_bounds__(128, 5) k_interior_f64(const double* __restrict__ A, double* __restrict__ B, LatDev L,
                                                       int t) {

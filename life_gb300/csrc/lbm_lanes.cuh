@@ -12,8 +12,9 @@
 // 1000 x 400 channel went from 30.0 to 17.4 us (central moments, FP32 storage),
 // that of a 256^2 FP64 cavity from 28 to 10.8 us (cold, under ncu). Per site
 // the FP64 unit is busy as long as before (three sites share 95 instructions,
-// where 32 shared 800), so there is no size at which the one-thread form is
-// the better one as a kernel of its own. Every value is formed with
+// where 32 shared 800); where many sites step together, straight walls take one
+// thread a site with the shared products formed once (lbm_walls.cuh, 200 for
+// 32 sites). Every value is formed with
 // the operations and in the order of site_state() / collide() in
 // lbm_device.cuh, so the results are the same bits.
 //
