@@ -73,6 +73,7 @@ int push_markers(LifeCase* c) {
     const int n = (int)m.size();
     std::vector<double> pos(2 * n), vel(2 * n), force(2 * n), eps(n), ds(n), sd(9 * n);
     std::vector<int> ns(n), si(9 * n), sj(9 * n), body(n);
+    bool edge = c->obj.hasFlex;
     for (int k = 0; k < n; k++) {
         for (int d = 0; d < 2; d++) {
             pos[2 * k + d] = m[k].pos[d];
@@ -83,12 +84,16 @@ int push_markers(LifeCase* c) {
         ds[k] = m[k].ds;
         ns[k] = m[k].nsupp;
         body[k] = m[k].body;
+        for (int s = 0; s < m[k].nsupp; s++)
+            edge = edge || m[k].si[s] <= 0 || m[k].si[s] >= c->Nx - 1 || m[k].sj[s] <= 0 || m[k].sj[s] >= c->Ny - 1;
         for (int s = 0; s < 9; s++) {
             si[9 * k + s] = m[k].si[s];
             sj[9 * k + s] = m[k].sj[s];
             sd[9 * k + s] = m[k].sd[s];
         }
     }
+    if (edge != c->spread_on_edge) c->rec_gen++;
+    c->spread_on_edge = edge;
     MarkerDev& M = c->M;
     cudaStream_t s = c->stream;
     CK(cudaMemcpyAsync(M.pos, pos.data(), 16 * n, cudaMemcpyHostToDevice, s));

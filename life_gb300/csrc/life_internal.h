@@ -108,8 +108,13 @@ struct LifeCase {
     const int* t_dev = nullptr;
     int t_off = 0;
     int loop_body_kernels = 0;  // kernels in one pass of a captured FSI loop body
+    // Whether the markers' support may reach an edge of the lattice: the spread
+    // then writes sites that the boundary kernel writes too, and follows it.
+    // Flexible bodies move, so theirs always may.
+    bool spread_on_edge = true;
     // observables recorder (life_case_record); rec_gen changes whenever the
-    // recorder is set up or removed, so captured step graphs are rebuilt
+    // recorder is set up or removed or spread_on_edge changes, so captured step
+    // graphs are rebuilt
     life::RecorderDev rec{};
     int rec_gen = 0;
 };
