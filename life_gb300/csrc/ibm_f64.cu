@@ -1,6 +1,6 @@
 // Immersed-boundary kernels (FP64), rigid and flexible markers.
 //
-//   k_ibm_interp    one thread per marker: rho and rho*u at the marker's
+//   k_ibm_interp    one warp per marker: rho and rho*u at the marker's
 //                   support sites (reconstructed from P_t exactly as the step
 //                   kernel computed them), then the direct force
 //                   (IBMNodeClass::interpolate + forceCalc,
@@ -49,33 +49,41 @@ __device__ __forceinline__ void mark_site(const IbmScratch& W, const LatDev& L, 
     }
 }
 
-// One warp per marker: lane s reconstructs support site s, and every lane
-// then adds the nsupp terms in support order (the reference's loop), so the
-// sums are formed exactly as in a sequential loop while the nine site states
-// are computed side by side. MARK: also the work of k_ibm_mark (the markers do
-// not move before the spread).
+// One warp per marker: lane s reconstructs support site s, and lanes 0, 1 and 2
+// add the nsupp terms of rho, rho ux and rho uy in support order (the
+// reference's loop), so the sums are formed exactly as in a sequential loop while
+// the nine site states are computed side by side. (A lane past nsupp holds +0,
+// which changes no sum that starts at +0.) MARK: also the work of k_ibm_mark (the
+// markers do not move before the spread), by a second warp per marker: its
+// atomics, each waiting for the one before, used to stand in front of the sums.
+// A block per marker, so that a body's markers do not share an SM's FP64 unit: the
+// kernel is bound by the chain of one warp (126 markers of the 1000 x 400 cylinder:
+// 11.0 -> 8.8 us cold).
 template <bool CM, class S, bool MARK>
-__global__ void __launch_bounds__(128) k_ibm_interp(const typename S::T* __restrict__ P, LatDev L, int t, MarkerDev M,
-                                                    IbmScratch W, double velScale, const int* __restrict__ t_dev) {
-    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__global__ void __launch_bounds__(MARK ? 64 : 32) k_ibm_interp(const typename S::T* __restrict__ P, LatDev L, int t,
+                                                               MarkerDev M, IbmScratch W, double velScale,
+                                                               const int* __restrict__ t_dev) {
+    const int k = blockIdx.x;
     const int lane = threadIdx.x & 31;
-    if (MARK) clear_force(W, L, (int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(gridDim.x * blockDim.x));
-    if (k >= M.n) return;  // uniform per warp
-    t = t_dev ? *t_dev : step_t(L, t);  // inside a replayed graph the step comes from the device
+    const int e = k * 9 + (lane < 9 ? lane : 0);
     const int ns = M.nsupp[k];
     const bool act = lane < ns;
-    int i = 0, j = 0;
-    if (act) {
-        i = M.si[k * 9 + lane];
-        j = M.sj[k * 9 + lane];
+    const int i = M.si[e], j = M.sj[e];
+    const double d = M.sd[e], vel = lane == 1 || lane == 2 ? M.vel[k * 2 + lane - 1] : 0.0;
+    const int imin = __reduce_min_sync(kAllLanes, act ? i : (1 << 30));
+    const int imax = __reduce_max_sync(kAllLanes, act ? i : -(1 << 30));
+    if (!MARK || threadIdx.x >= 32) {
+        const int jmin = __reduce_min_sync(kAllLanes, act ? j : (1 << 30));
+        const int jmax = __reduce_max_sync(kAllLanes, act ? j : -(1 << 30));
+        const int4 bb = make_int4(imin, imax, jmin, jmax);
+        if (lane == 0) M.bbox[k] = bb;
+        if (MARK) {
+            clear_force(W, L, k * 32 + lane, (int)gridDim.x * 32);
+            if (act) mark_site(W, L, k, i, j, lane == 0, bb);
+            return;
+        }
     }
-    const int imin = __reduce_min_sync(0xffffffffu, act ? i : (1 << 30));
-    const int imax = __reduce_max_sync(0xffffffffu, act ? i : -(1 << 30));
-    const int jmin = __reduce_min_sync(0xffffffffu, act ? j : (1 << 30));
-    const int jmax = __reduce_max_sync(0xffffffffu, act ? j : -(1 << 30));
-    const int4 bb = make_int4(imin, imax, jmin, jmax);
-    if (lane == 0) M.bbox[k] = bb;
-    if (MARK && act) mark_site(W, L, k, i, j, lane == 0, bb);
+    t = t_dev ? *t_dev : step_t(L, t);  // inside a replayed graph the step comes from the device
     // support sites on a convective outlet: its speed term, formed here too
     // (nothing of this step has to be finished before the interpolation)
     double dU[2] = {0.0, 0.0};
@@ -86,24 +94,21 @@ __global__ void __launch_bounds__(128) k_ibm_interp(const typename S::T* __restr
     }
     double tr = 0.0, tx = 0.0, ty = 0.0;
     if (act) {
-        const double d = M.sd[k * 9 + lane];
         double f[9], rho, ux, uy;
         site_state<CM, S>(P, L, t, i, j, f, rho, ux, uy, form ? dU : nullptr);
         tr = rho * d * 1.0 * 1.0;
         tx = rho * ux * d * 1.0 * 1.0;
         ty = rho * uy * d * 1.0 * 1.0;
     }
-    double iRho = 0.0, iMx = 0.0, iMy = 0.0;
-    for (int q = 0; q < ns; q++) {
-        iRho += __shfl_sync(0xffffffffu, tr, q);
-        iMx += __shfl_sync(0xffffffffu, tx, q);
-        iMy += __shfl_sync(0xffffffffu, ty, q);
+    double acc = 0.0;
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+        const double r = lane_get(tr, q), x = lane_get(tx, q), y = lane_get(ty, q);
+        acc += lane == 0 ? r : (lane == 1 ? x : y);
     }
-    if (lane == 0) {
-        const double sc = velScale * iRho;
-        M.force[k * 2 + 0] = 2.0 * (sc * M.vel[k * 2 + 0] - iMx);
-        M.force[k * 2 + 1] = 2.0 * (sc * M.vel[k * 2 + 1] - iMy);
-    }
+    const double sc = velScale * lane_get(acc, 0);
+    const double force = 2.0 * (sc * vel - acc);
+    if (lane == 1 || lane == 2) M.force[k * 2 + lane - 1] = force;
 }
 
 // One thread per support entry: the first to set a site's bit lists the site.
@@ -124,8 +129,8 @@ __global__ void k_ibm_mark(MarkerDev M, IbmScratch W, LatDev L) {
 // that own their tiles: with one CTA per touched 16 x 16 tile and one thread
 // per site (a chain of 700-900 FP64 instructions of 64 cycles) the kernel took
 // 44 us for the 126 markers of the 1000 x 400 cylinder (central moments, FP32
-// storage), 26 us now; 41 us for a circle and its tail of 132 markers (BGK,
-// FP64), 13 us now.
+// storage), 16 us now; 41 us for a circle and its tail of 132 markers (BGK,
+// FP64), 12 us now.
 __device__ __forceinline__ bool box_has(const int4& b, int i, int j) {
     return i >= b.x && i <= b.y && j >= b.z && j <= b.w;
 }
@@ -168,17 +173,26 @@ __global__ void __launch_bounds__(32) k_ibm_spread(const typename S::T* __restri
             while (bodies) {
                 const int b = b0 + __ffs(bodies) - 1;
                 bodies &= bodies - 1;
-                const int kend = W.body_start[b + 1];
-                for (int k0 = W.body_start[b]; k0 < kend; k0 += 32) {
+                const int kbeg = W.body_start[b], kend = W.body_start[b + 1];
+                // the support box of the next chunk's marker comes while this
+                // chunk's is looked at, and what a hit needs with its entries
+                int4 next = kbeg + lane < kend ? M.bbox[kbeg + lane] : make_int4(0, -1, 0, -1);
+                for (int k0 = kbeg; k0 < kend; k0 += 32) {
                     const int k = k0 + lane;
+                    const int4 bb = next;
+                    next = k + 32 < kend ? M.bbox[k + 32] : make_int4(0, -1, 0, -1);
                     int at[kLaneSites];  // this marker's support entry at each site
                     bool any = false;
+                    double mx = 0.0, my = 0.0, me = 0.0, ds = 0.0;
 #pragma unroll
                     for (int c = 0; c < kLaneSites; c++) at[c] = -1;
                     if (k < kend) {
-                        const int4 bb = M.bbox[k];
                         if (box_has(bb, is[0], js[0]) || box_has(bb, is[1], js[1]) || box_has(bb, is[2], js[2])) {
                             const int ns = M.nsupp[k];
+                            mx = M.force[k * 2];
+                            my = M.force[k * 2 + 1];
+                            me = M.eps[k];
+                            ds = M.ds[k];
 #pragma unroll
                             for (int e = 8; e >= 0; e--) {
                                 const int ei = M.si[k * 9 + e], ej = M.sj[k * 9 + e];
@@ -192,9 +206,8 @@ __global__ void __launch_bounds__(32) k_ibm_spread(const typename S::T* __restri
                     if (!__any_sync(kAllLanes, any)) continue;
                     double gx = 0.0, gy = 0.0;
                     if (any) {
-                        const double e = M.eps[k], ds = M.ds[k];
-                        gx = M.force[k * 2] * e * ds * 1.0;
-                        gy = M.force[k * 2 + 1] * e * ds * 1.0;
+                        gx = mx * me * ds * 1.0;
+                        gy = my * me * ds * 1.0;
                     }
                     unsigned hits = 0;
 #pragma unroll
@@ -301,12 +314,11 @@ struct TypedPtr {
 cudaError_t launch_ibm_interp(const void* P, const LatDev& L, int t, const MarkerDev& M, const IbmScratch* mark,
                               double velScale, cudaStream_t s, const int* t_dev) {
     if (M.n == 0) return cudaSuccess;
-    const int nb = (M.n + 3) / 4;  // one warp per marker
     TypedPtr<void> Pp{P};
 #define LIFE_INTERP(CM, S)                                                                              \
     do {                                                                                                \
-        if (mark) k_ibm_interp<CM, S, true><<<nb, 128, 0, s>>>(Pp, L, t, M, *mark, velScale, t_dev);     \
-        else k_ibm_interp<CM, S, false><<<nb, 128, 0, s>>>(Pp, L, t, M, IbmScratch{}, velScale, t_dev);  \
+        if (mark) k_ibm_interp<CM, S, true><<<M.n, 64, 0, s>>>(Pp, L, t, M, *mark, velScale, t_dev);     \
+        else k_ibm_interp<CM, S, false><<<M.n, 32, 0, s>>>(Pp, L, t, M, IbmScratch{}, velScale, t_dev);  \
     } while (0)
     if (L.prec == LIFE_PREC_F64) {
         if (L.cm) LIFE_INTERP(true, StoreF64);
