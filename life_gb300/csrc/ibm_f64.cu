@@ -129,22 +129,26 @@ __global__ void k_ibm_mark(MarkerDev M, IbmScratch W, LatDev L) {
 // that own their tiles: with one CTA per touched 16 x 16 tile and one thread
 // per site (a chain of 700-900 FP64 instructions of 64 cycles) the kernel took
 // 44 us for the 126 markers of the 1000 x 400 cylinder (central moments, FP32
-// storage), 16 us now; 41 us for a circle and its tail of 132 markers (BGK,
-// FP64), 12 us now.
+// storage), 14.5 us now; 41 us for a circle and its tail of 132 markers (BGK,
+// FP64), 12 us now. Bound by the latency of one chain: a second warp of the block
+// forms the site's populations, their sums and the reciprocal of the density while
+// the first scans the markers (15.9 us with one warp for both).
 __device__ __forceinline__ bool box_has(const int4& b, int i, int j) {
     return i >= b.x && i <= b.y && j >= b.z && j <= b.w;
 }
 
 template <bool CM, class S>
-__global__ void __launch_bounds__(32) k_ibm_spread(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
+__global__ void __launch_bounds__(64) k_ibm_spread(const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
                                                    LatDev L, int t, MarkerDev M, IbmScratch W) {
     __shared__ double s_c[kLaneSites][2][32];
-    const int lane = threadIdx.x;
+    __shared__ double s_a[kLaneSites][2];
+    const int lane = threadIdx.x & 31;
+    const bool scans = threadIdx.x < 32;
     const SiteLane g = site_lane();
     t = step_t(L, t);
     const int nsites = *W.nsites;
     // the next step's list starts empty
-    if (blockIdx.x == 0) {
+    if (blockIdx.x == 0 && scans) {
         if (lane == 0) *W.nsites_prev = 0;
         for (int b = lane; b < W.nbodies; b += 32)
             W.body_box_next[b] = make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff);
@@ -154,91 +158,104 @@ __global__ void __launch_bounds__(32) k_ibm_spread(const typename S::T* __restri
         const bool on = q0 + g.slot < nsites;
         const long long s = W.sites[on ? q0 + g.slot : q0];
         const int j = (int)(s / L.pitch), i = (int)(s - (long long)j * L.pitch);
-        int is[kLaneSites], js[kLaneSites];
+        const bool store = on && g.store;
+        double Fx = 0.0, Fy = 0.0, f = 0.0, m = 0.0, rho = 0.0, y = 0.0;
+        if (!scans) {
+            f = lanes_populations<CM, S>(A, L, t, g, i, j, Fx, Fy);
+            m = lanes_sums(g, f);
+            rho = lane_get(m, g.base);
+            y = __drcp_rn(rho);
+        } else {
+            int is[kLaneSites], js[kLaneSites];
 #pragma unroll
-        for (int c = 0; c < kLaneSites; c++) {
-            is[c] = __shfl_sync(kAllLanes, i, 9 * c);
-            js[c] = __shfl_sync(kAllLanes, j, 9 * c);
-        }
-        // lanes 0 and 1 of a site sum the x and the y force
-        const int comp = g.v == 1 ? 1 : 0;
-        double acc = 0.0;
-        for (int b0 = 0; b0 < W.nbodies; b0 += 32) {
-            bool near = false;
-            if (b0 + lane < W.nbodies) {
-                const int4 box = W.body_box[b0 + lane];
-                near = box_has(box, is[0], js[0]) || box_has(box, is[1], js[1]) || box_has(box, is[2], js[2]);
+            for (int c = 0; c < kLaneSites; c++) {
+                is[c] = __shfl_sync(kAllLanes, i, 9 * c);
+                js[c] = __shfl_sync(kAllLanes, j, 9 * c);
             }
-            unsigned bodies = __ballot_sync(kAllLanes, near);
-            while (bodies) {
-                const int b = b0 + __ffs(bodies) - 1;
-                bodies &= bodies - 1;
-                const int kbeg = W.body_start[b], kend = W.body_start[b + 1];
-                // the support box of the next chunk's marker comes while this
-                // chunk's is looked at, and what a hit needs with its entries
-                int4 next = kbeg + lane < kend ? M.bbox[kbeg + lane] : make_int4(0, -1, 0, -1);
-                for (int k0 = kbeg; k0 < kend; k0 += 32) {
-                    const int k = k0 + lane;
-                    const int4 bb = next;
-                    next = k + 32 < kend ? M.bbox[k + 32] : make_int4(0, -1, 0, -1);
-                    int at[kLaneSites];  // this marker's support entry at each site
-                    bool any = false;
-                    double mx = 0.0, my = 0.0, me = 0.0, ds = 0.0;
+            // lanes 0 and 1 of a site sum the x and the y force
+            const int comp = g.v == 1 ? 1 : 0;
+            double acc = 0.0;
+            for (int b0 = 0; b0 < W.nbodies; b0 += 32) {
+                bool near = false;
+                if (b0 + lane < W.nbodies) {
+                    const int4 box = W.body_box[b0 + lane];
+                    near = box_has(box, is[0], js[0]) || box_has(box, is[1], js[1]) || box_has(box, is[2], js[2]);
+                }
+                unsigned bodies = __ballot_sync(kAllLanes, near);
+                while (bodies) {
+                    const int b = b0 + __ffs(bodies) - 1;
+                    bodies &= bodies - 1;
+                    const int kbeg = W.body_start[b], kend = W.body_start[b + 1];
+                    // the support box of the next chunk's marker comes while this
+                    // chunk's is looked at, and what a hit needs with its entries
+                    int4 next = kbeg + lane < kend ? M.bbox[kbeg + lane] : make_int4(0, -1, 0, -1);
+                    for (int k0 = kbeg; k0 < kend; k0 += 32) {
+                        const int k = k0 + lane;
+                        const int4 bb = next;
+                        next = k + 32 < kend ? M.bbox[k + 32] : make_int4(0, -1, 0, -1);
+                        int at[kLaneSites];  // this marker's support entry at each site
+                        bool any = false;
+                        double mx = 0.0, my = 0.0, me = 0.0, ds = 0.0;
 #pragma unroll
-                    for (int c = 0; c < kLaneSites; c++) at[c] = -1;
-                    if (k < kend) {
-                        if (box_has(bb, is[0], js[0]) || box_has(bb, is[1], js[1]) || box_has(bb, is[2], js[2])) {
-                            const int ns = M.nsupp[k];
-                            mx = M.force[k * 2];
-                            my = M.force[k * 2 + 1];
-                            me = M.eps[k];
-                            ds = M.ds[k];
+                        for (int c = 0; c < kLaneSites; c++) at[c] = -1;
+                        if (k < kend) {
+                            if (box_has(bb, is[0], js[0]) || box_has(bb, is[1], js[1]) || box_has(bb, is[2], js[2])) {
+                                const int ns = M.nsupp[k];
+                                mx = M.force[k * 2];
+                                my = M.force[k * 2 + 1];
+                                me = M.eps[k];
+                                ds = M.ds[k];
 #pragma unroll
-                            for (int e = 8; e >= 0; e--) {
-                                const int ei = M.si[k * 9 + e], ej = M.sj[k * 9 + e];
+                                for (int e = 8; e >= 0; e--) {
+                                    const int ei = M.si[k * 9 + e], ej = M.sj[k * 9 + e];
 #pragma unroll
-                                for (int c = 0; c < kLaneSites; c++)
-                                    if (e < ns && ei == is[c] && ej == js[c]) at[c] = e;
+                                    for (int c = 0; c < kLaneSites; c++)
+                                        if (e < ns && ei == is[c] && ej == js[c]) at[c] = e;
+                                }
+                                any = at[0] >= 0 || at[1] >= 0 || at[2] >= 0;
                             }
-                            any = at[0] >= 0 || at[1] >= 0 || at[2] >= 0;
                         }
-                    }
-                    if (!__any_sync(kAllLanes, any)) continue;
-                    double gx = 0.0, gy = 0.0;
-                    if (any) {
-                        gx = mx * me * ds * 1.0;
-                        gy = my * me * ds * 1.0;
-                    }
-                    unsigned hits = 0;
+                        if (!__any_sync(kAllLanes, any)) continue;
+                        double gx = 0.0, gy = 0.0;
+                        if (any) {
+                            gx = mx * me * ds * 1.0;
+                            gy = my * me * ds * 1.0;
+                        }
+                        unsigned hits = 0;
 #pragma unroll
-                    for (int c = 0; c < kLaneSites; c++) {
-                        const unsigned h = __ballot_sync(kAllLanes, at[c] >= 0);
-                        if (c == g.slot) hits = h;
-                        if (at[c] >= 0) {
-                            const double d = M.sd[k * 9 + at[c]];
-                            s_c[c][0][lane] = gx * d;
-                            s_c[c][1][lane] = gy * d;
+                        for (int c = 0; c < kLaneSites; c++) {
+                            const unsigned h = __ballot_sync(kAllLanes, at[c] >= 0);
+                            if (c == g.slot) hits = h;
+                            if (at[c] >= 0) {
+                                const double d = M.sd[k * 9 + at[c]];
+                                s_c[c][0][lane] = gx * d;
+                                s_c[c][1][lane] = gy * d;
+                            }
                         }
+                        __syncwarp();
+                        while (hits) {
+                            acc = acc + s_c[g.slot][comp][__ffs(hits) - 1];
+                            hits &= hits - 1;
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
-                    while (hits) {
-                        acc = acc + s_c[g.slot][comp][__ffs(hits) - 1];
-                        hits &= hits - 1;
-                    }
-                    __syncwarp();
                 }
             }
+            if (g.store && g.v < 2) s_a[g.slot][g.v] = acc;
         }
-        const double ax = lane_get(acc, g.base), ay = lane_get(acc, g.base + 1);
-        const bool store = on && g.store;
-        if (store && g.v == 0) {
-            W.force_ibm[s] = ax;
-            W.force_ibm[L.S + s] = ay;
-            atomicAnd(&W.site_flag[s >> 5], ~(1u << (s & 31)));
+        __syncthreads();
+        const double ax = s_a[g.slot][0], ay = s_a[g.slot][1];
+        __syncthreads();  // (the next three sites' sums may come)
+        if (scans) {
+            if (store && g.v == 0) {
+                W.force_ibm[s] = ax;
+                W.force_ibm[L.S + s] = ay;
+                atomicAnd(&W.site_flag[s >> 5], ~(1u << (s & 31)));
+            }
+            continue;
         }
-        double Fx, Fy, rho, ux, uy;
-        const double f = lanes_populations<CM, S>(A, L, t, g, i, j, Fx, Fy);
-        lanes_macroscopic(g, f, Fx + ax, Fy + ay, rho, ux, uy);
+        double ux, uy;
+        lanes_velocity(g, m, rho, y, Fx + ax, Fy + ay, ux, uy);
         if (store && g.v == 0) {
             store_history(L, site_type(L, i, j), i, j, rho, ux, uy);
             if (L.convective && i >= L.Nx - 3) {
@@ -347,7 +364,7 @@ cudaError_t launch_ibm_spread(const void* A, void* B, const LatDev& L, int t, co
     // blocks (about 27 per SM) a block takes further sites in turn
     const int grid = 3 * M.n < 4096 ? 3 * M.n : 4096;
     TypedPtr<void> Ap{A}, Bp{B};
-    IBM_DISPATCH(k_ibm_spread, grid, 32, Ap, Bp, L, t, M, W);
+    IBM_DISPATCH(k_ibm_spread, grid, 64, Ap, Bp, L, t, M, W);
     return cudaGetLastError();
 }
 

@@ -84,15 +84,20 @@ __device__ __forceinline__ double lanes_sums(const SiteLane& g, double f) {
     return pos_zero(acc);
 }
 
+// The velocity of macroscopic() from this lane's sum m, given y = RN(1/rho).
+__device__ __forceinline__ void lanes_velocity(const SiteLane& g, double m, double rho, double y, double Fx, double Fy,
+                                               double& ux, double& uy) {
+    const double q = div_rn_recip(m + 0.5 * (g.role == 2 ? Fy : Fx), rho, y);
+    ux = lane_get(q, g.base + 1);
+    uy = lane_get(q, g.base + 2);
+}
+
 // macroscopic() / macroscopic_ibm(): F is the force in the half term.
 __device__ __forceinline__ void lanes_macroscopic(const SiteLane& g, double f, double Fx, double Fy, double& rho,
                                                   double& ux, double& uy) {
     const double m = lanes_sums(g, f);
     rho = lane_get(m, g.base);
-    const double y = __drcp_rn(rho);
-    const double q = div_rn_recip(m + 0.5 * (g.role == 2 ? Fy : Fx), rho, y);
-    ux = lane_get(q, g.base + 1);
-    uy = lane_get(q, g.base + 2);
+    lanes_velocity(g, m, rho, __drcp_rn(rho), Fx, Fy, ux, uy);
 }
 
 // equilibrium<CM>() of this lane's direction
