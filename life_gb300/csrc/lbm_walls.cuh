@@ -7,7 +7,8 @@
 // cases with a force take nine lanes a site (lbm_lanes.cuh: 95 to 130 FP64
 // instructions for three sites, 38 a site, a shorter chain). A case alone with
 // few boundary sites takes nine lanes for all of them: 14.2 us a step against
-// 15.6 (256 x 256, 1020 sites); at 2800 sites the two are even (35.6 and 35.8),
+// 15.6 (256 x 256, 1020 sites); at 2800 sites the two were even (35.6 and 35.8,
+// measured where a body's spread waited for the walls),
 // at 4400 the threads are ahead (17.2 against 19.4 us, 1501 x 703 FP32), and 64
 // lattices in a batch step in 573 us against 976. (Products from the integer
 // units, as in the interior, make the warp's chain longer: 15.6 -> 18.4 us at
