@@ -311,11 +311,7 @@ static void rewind_host_view(LifeBatch* b) {
         const int adv = c->t - b->t_base[k];
         c->t = b->t_base[k];
         c->cur = b->cur_base[k];
-        if (adv & 1) {
-            std::swap(c->W.sites, c->W.sites_prev);
-            std::swap(c->W.nsites, c->W.nsites_prev);
-            std::swap(c->W.body_box, c->W.body_box_next);
-        }
+        if (adv & 1) swap_site_lists(c->W);
     }
 }
 
@@ -425,11 +421,7 @@ static int run_batch(LifeBatch* b, int nsteps, cudaEvent_t start, cudaEvent_t st
         for (LifeCase* c : b->cases) {
             c->t += m;
             c->cur ^= m & 1;
-            if (c->obj.hasIBM && (m & 1)) {
-                std::swap(c->W.sites, c->W.sites_prev);
-                std::swap(c->W.nsites, c->W.nsites_prev);
-                std::swap(c->W.body_box, c->W.body_box_next);
-            }
+            if (m & 1) swap_site_lists(c->W);
         }
         s += m;
     }

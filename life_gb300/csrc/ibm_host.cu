@@ -110,6 +110,28 @@ int push_markers(LifeCase* c) {
     return LIFE_OK;
 }
 
+static size_t flag_words(const LifeCase* c) { return ((size_t)c->S + 31) / 32; }
+
+// The lists of support sites as they are before a case's first step, for a
+// state that no step of this case has left behind (at creation, and when a
+// state is loaded): both empty, no site flagged, no force on the lattice, and
+// the list that the next step fills the one that goes with P[0].
+int life::reset_site_lists(LifeCase* c) {
+    IbmScratch& W = c->W;
+    if (!c->obj.hasIBM) return LIFE_OK;
+    if (c->cur) swap_site_lists(W);
+    cudaStream_t s = c->stream;
+    CK(cudaMemsetAsync(W.force_ibm, 0, sizeof(double) * 2 * c->S, s));
+    CK(cudaMemsetAsync(W.nsites, 0, sizeof(int), s));
+    CK(cudaMemsetAsync(W.nsites_prev, 0, sizeof(int), s));
+    CK(cudaMemsetAsync(W.site_flag, 0, sizeof(unsigned) * flag_words(c), s));
+    const std::vector<int4> empty((size_t)W.nbodies, make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff));
+    CK(cudaMemcpyAsync(W.body_box, empty.data(), sizeof(int4) * empty.size(), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(W.body_box_next, empty.data(), sizeof(int4) * empty.size(), cudaMemcpyHostToDevice, s));
+    CK(cudaStreamSynchronize(s));
+    return LIFE_OK;
+}
+
 int upload_markers(LifeCase* c) {
     const int n = (int)c->obj.m.size();
     MarkerDev& M = c->M;
@@ -122,15 +144,10 @@ int upload_markers(LifeCase* c) {
         return rc;
     if ((rc = push_markers(c))) return rc;
     IbmScratch& W = c->W;
-    const size_t flag_words = ((size_t)c->S + 31) / 32;
     if ((rc = alloc_t(c, &W.force_ibm, (size_t)2 * c->S)) || (rc = alloc_t(c, &W.sites, (size_t)9 * n + 1)) ||
         (rc = alloc_t(c, &W.sites_prev, (size_t)9 * n + 1)) || (rc = alloc_t(c, &W.nsites, 1)) ||
-        (rc = alloc_t(c, &W.nsites_prev, 1)) || (rc = alloc_t(c, &W.site_flag, flag_words)))
+        (rc = alloc_t(c, &W.nsites_prev, 1)) || (rc = alloc_t(c, &W.site_flag, flag_words(c))))
         return rc;
-    CK(cudaMemsetAsync(W.force_ibm, 0, sizeof(double) * 2 * c->S, c->stream));
-    CK(cudaMemsetAsync(W.nsites, 0, sizeof(int), c->stream));
-    CK(cudaMemsetAsync(W.nsites_prev, 0, sizeof(int), c->stream));
-    CK(cudaMemsetAsync(W.site_flag, 0, sizeof(unsigned) * flag_words, c->stream));
     // bodies as contiguous marker ranges (markers are stored body by body);
     // one range over all markers if that ever does not hold
     std::vector<int> start(1, 0);
@@ -152,13 +169,12 @@ int upload_markers(LifeCase* c) {
     if ((rc = alloc_t(c, &d_start, start.size())) || (rc = alloc_t(c, &d_box_of, box_of.size())) ||
         (rc = alloc_t(c, &W.body_box, (size_t)W.nbodies)) || (rc = alloc_t(c, &W.body_box_next, (size_t)W.nbodies)))
         return rc;
-    const std::vector<int4> empty((size_t)W.nbodies, make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff));
-    CK(cudaMemcpyAsync(W.body_box, empty.data(), sizeof(int4) * empty.size(), cudaMemcpyHostToDevice, c->stream));
     W.body_start = d_start;
     W.box_of = d_box_of;
     CK(cudaMemcpyAsync(d_start, start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(d_box_of, box_of.data(), sizeof(int) * box_of.size(), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if ((rc = reset_site_lists(c))) return rc;
     if ((rc = alloc_t(c, &c->d_fsi, 1)) || (rc = alloc_t(c, &c->d_status, 4))) return rc;
     FsiScalars f{};
     f.relax = c->p.relaxMax;
@@ -196,9 +212,7 @@ int ibm_apply(LifeCase* c, int t, const void* A, void* B, cudaStream_t s) {
     e = launch_ibm_spread(A, B, L, t, c->M, c->W, s);
     if (e != cudaSuccess) return cuda_fail(e, "ibm_spread");
     c->ibm_launches += 1;
-    std::swap(c->W.sites, c->W.sites_prev);
-    std::swap(c->W.nsites, c->W.nsites_prev);
-    std::swap(c->W.body_box, c->W.body_box_next);
+    swap_site_lists(c->W);
     return LIFE_OK;
 }
 

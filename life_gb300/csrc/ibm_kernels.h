@@ -40,6 +40,22 @@ struct IbmScratch {
     int4* body_box_next;      // [nbodies] the other of two, reset by this step's spread
 };
 
+// The two lists of support sites (and the boxes of each) change roles every
+// step, as the two population buffers do: the step that reads P[0] fills one
+// list, the step that reads P[1] the other, also in step graphs captured long
+// before.
+inline void swap_site_lists(IbmScratch& W) {
+    long long* const s = W.sites;
+    int* const n = W.nsites;
+    int4* const b = W.body_box;
+    W.sites = W.sites_prev;
+    W.nsites = W.nsites_prev;
+    W.body_box = W.body_box_next;
+    W.sites_prev = s;
+    W.nsites_prev = n;
+    W.body_box_next = b;
+}
+
 // Close marker pairs of removeOverlapMarkers (appended unordered, see
 // k_overlap_pairs).
 cudaError_t launch_overlap_pairs(const double* pos, int nm, double Dx, int* count, int2* out, int cap,

@@ -848,6 +848,7 @@ extern "C" int life_case_set_fields(LifeCase* c, int32_t t, const double* rho, c
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     cleanup();
     if (e != cudaSuccess) return cuda_fail(e, "set_fields");
+    if ((rc = reset_site_lists(c))) return rc;
     c->cur = 0;
     return LIFE_OK;
 }

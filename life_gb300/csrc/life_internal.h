@@ -139,6 +139,9 @@ void free_fem(LifeCase* c);
 // inside a capture the step is read from c->t_dev.
 cudaError_t launch_record(const LifeCase* c, int t, cudaStream_t s);
 void free_recorder(LifeCase* c);
+// The lists of support sites as before a case's first step (ibm_host.cu); sets
+// them up for c->cur = 0.
+int reset_site_lists(LifeCase* c);
 int ensure_steps(LifeCase* c, int t0, int n);
 // removeOverlapMarkers' pair test on the device (an OverlapScan, objects.h).
 int device_overlap_scan(const double* pos, int nm, double Dx, std::vector<std::pair<int, int>>* pairs,
