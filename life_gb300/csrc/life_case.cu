@@ -5,6 +5,8 @@
 // order. The state after step t is kept as P_{t+1} (post-collision
 // populations, structure of arrays) plus the small side buffers the next step
 // reads; see lbm_device.cuh.
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -16,6 +18,7 @@
 #include <vector>
 
 #include "../../include/life_gb300.h"
+#include "host_array.h"
 #include "ibm_kernels.h"
 #include "lbm_kernels.h"
 #include "life_internal.h"
@@ -653,6 +656,36 @@ extern "C" int life_case_status(LifeCase* c, LifeStatus* st) {
     return LIFE_OK;
 }
 
+// What the driver knows of a host pointer (nothing of ordinary memory).
+static HostRange host_range(const void* p) {
+    HostRange r;
+    cudaPointerAttributes host{};
+    if (cudaPointerGetAttributes(&host, p) != cudaSuccess || host.type != cudaMemoryTypeHost) {
+        cudaGetLastError();
+        return r;
+    }
+    static const PFN_cuPointerGetAttribute_v4000 query = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 4000, cudaEnableDefault, &q);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<PFN_cuPointerGetAttribute_v4000>(fn)
+                                                                    : nullptr;
+    }();
+    const CUdeviceptr a = reinterpret_cast<CUdeviceptr>(p);
+    CUdeviceptr start = 0;
+    unsigned access = 0;
+    if (!query || query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, a) != CUDA_SUCCESS ||
+        query(&r.size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, a) != CUDA_SUCCESS)
+        return r;
+    r.locked = true;
+    r.start = static_cast<std::uintptr_t>(start);
+    r.device = reinterpret_cast<std::uintptr_t>(host.devicePointer);
+    r.writable = query(&access, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS, a) == CUDA_SUCCESS &&
+                 access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE;
+    return r;
+}
+
 extern "C" int life_case_get_fields(LifeCase* c, double* rho, double* u, double* f, double* force_ibm) {
     if (!c) return set_error(LIFE_ERR_INVALID, "case is NULL");
     const size_t n = (size_t)c->Nx * c->Ny;
@@ -663,8 +696,8 @@ extern "C" int life_case_get_fields(LifeCase* c, double* rho, double* u, double*
         if (force_ibm) std::memcpy(force_ibm, c->h_fibm.data(), n * 2 * sizeof(double));
         return LIFE_OK;
     }
-    // Page-locked host arrays that the device can address take rho, u and
-    // force_ibm straight from the export kernel, which writes whole runs of
+    // Host arrays that are page-locked from end to end and that the device can
+    // write take rho, u and force_ibm straight from the export kernel, which writes whole runs of
     // them: no staging buffers and no copies. (The populations are written
     // per site, so a call that wants them goes through the device.) Staged,
     // the 64 cases of an ensemble took 0.4-1.3 ms each to read, most of it in
@@ -674,14 +707,16 @@ extern "C" int life_case_get_fields(LifeCase* c, double* rho, double* u, double*
     double* dev_p[3] = {nullptr, nullptr, nullptr};
     {
         double* const host[4] = {rho, u, force_ibm, f};
+        const int doubles[4] = {1, 2, 2, 9};
         for (int k = 0; k < 4; k++) {
             if (!host[k]) continue;
-            cudaPointerAttributes a{};
-            if (cudaPointerGetAttributes(&a, host[k]) != cudaSuccess || a.type != cudaMemoryTypeHost) locked = false;
-            else if (k < 3) dev_p[k] = static_cast<double*>(a.devicePointer);
-            if (k < 3 && (!dev_p[k] || (reinterpret_cast<uintptr_t>(dev_p[k]) & (k == 0 ? 7 : 15)))) mapped = false;
+            const HostRange r = host_range(host[k]);
+            const size_t bytes = n * doubles[k] * sizeof(double);
+            locked = locked && host_range_covers(r, host[k], bytes);
+            if (k == 3) continue;
+            dev_p[k] = reinterpret_cast<double*>(kernel_target(r, host[k], bytes, k == 0 ? 8 : 16));
+            mapped = mapped && dev_p[k];
         }
-        cudaGetLastError();
     }
     if (locked && mapped && c->t != c->t_set) {
         const cudaError_t e = launch_export(c->P[c->cur ^ 1], lattice_view(c, c->t), c->t, false, dev_p[0], dev_p[1],
