@@ -306,9 +306,9 @@ __host__ __device__ __forceinline__ double cm_population(int cx, int cy, const C
 // the FP64 unit busy 82 % of the time and the integer unit 53 %; with the
 // products on the FP64 unit as well the shared sums alone would leave 240.
 
-// The populations are in [2^-8, 1) and each velocity component is zero or in
-// [2^-60, 2^-3): then every product of the two collisions is zero or in the
-// normal range (cm_factored_ok's bounds), and what 1/2, 1 and 2 are added to
+// The populations are in [2^-8, 1), so the density is in [2^-5, 9), and each
+// velocity component is zero or in [2^-60, 2^-3): then every product of the two
+// collisions is zero or in the normal range (cm_factored_ok's bounds), and what 1/2, 1 and 2 are added to
 // is smaller than they are (3 |ux + uy| < 3/4, |ux + uy + 2 ux uy| < 1/2).
 __host__ __device__ __forceinline__ bool populations_in_range(const double f[9]) {
     unsigned worst = 0;
@@ -350,7 +350,7 @@ __host__ __device__ __forceinline__ double two_plus(double x) {
 }
 
 // equilibrium<false>() and equilibrium<true>() of all nine directions (rho in
-// [2^-5, 2^3), velocity_in_range), the products that directions share formed
+// [2^-5, 9), velocity_in_range), the products that directions share formed
 // once.
 template <bool INT = true>
 __host__ __device__ __forceinline__ void equilibria_bgk_int(double rho, double ux, double uy, double feq[9]) {

@@ -133,7 +133,8 @@ __host__ __device__ __forceinline__ double add_pow2_int(double x) {
 // The density and momentum sums of moment_sums() for populations in [2^-8, 1):
 // every population is a multiple of 2^-60, so the running sums are 64-bit
 // integers in that unit, rounded to 53 significant bits after each addition.
-// About 25 issue cycles an addition.
+// The density may reach 9, which needs all 64 bits, unsigned; the momenta stay
+// below 3 in magnitude. About 25 issue cycles an addition.
 __host__ __device__ __forceinline__ long long round53(long long s) {
     const unsigned long long z = (unsigned long long)(s ^ (s >> 63));
     int p = 11 - leading_zeros(z);  // bits below the 53 significant ones
@@ -142,12 +143,13 @@ __host__ __device__ __forceinline__ long long round53(long long s) {
     s += (below >> 1) + ((lo >> p) & (p > 0 ? 1u : 0u));
     return s & ~(long long)below;
 }
+__host__ __device__ __forceinline__ unsigned long long unit60_bits(unsigned long long a) {  // a 2^-60, a of 53 bits, not 0
+    const int lz = leading_zeros(a);
+    return (shift_left(a, (unsigned)lz) >> 11) + ((unsigned long long)(unsigned)(1025 - lz) << 52);
+}
 __host__ __device__ __forceinline__ double unit60(long long s) {  // s 2^-60, |s| of 53 bits at most
     const unsigned long long a = s < 0 ? 0ull - (unsigned long long)s : (unsigned long long)s;
-    const int lz = leading_zeros(a);
-    const unsigned long long m = shift_left(a, (unsigned)lz) >> 11;
-    const unsigned long long r = m + ((unsigned long long)(unsigned)(1025 - lz) << 52);
-    return bits_double(a == 0 ? 0ull : r | ((unsigned long long)s & 0x8000000000000000ull));
+    return bits_double(a == 0 ? 0ull : unit60_bits(a) | ((unsigned long long)s & 0x8000000000000000ull));
 }
 __host__ __device__ __forceinline__ void moment_sums_int(const double f[9], double& r, double& mx, double& my) {
     long long x[9];
@@ -158,16 +160,16 @@ __host__ __device__ __forceinline__ void moment_sums_int(const double f[9], doub
         const unsigned long long m = ((unsigned long long)((h & 0xfffffu) | 0x100000u) << 32) | (unsigned)u;
         x[v] = (long long)(m << ((h >> 20) - 1015u));
     }
-    long long s = x[0];
+    unsigned long long s = (unsigned long long)x[0];
 #pragma unroll
     for (int v = 1; v < 9; v++) {
-        s += x[v];  // at least 2^53: something to round every time
-        const int p = 11 - leading_zeros((unsigned long long)s);
+        s += (unsigned long long)x[v];  // at least 2^53: something to round every time
+        const int p = 11 - leading_zeros(s);
         const unsigned below = (1u << p) - 1u;
         s += (below >> 1) + (((unsigned)s >> p) & 1u);
-        s &= ~(long long)below;
+        s &= ~(unsigned long long)below;
     }
-    r = unit60(s);
+    r = bits_double(unit60_bits(s));
     mx = unit60(round53(round53(round53(round53(round53(x[1] - x[2]) + x[5]) - x[6]) + x[7]) - x[8]));
     my = unit60(round53(round53(round53(round53(round53(x[3] - x[4]) + x[5]) - x[6]) - x[7]) + x[8]));
 }
