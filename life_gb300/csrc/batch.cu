@@ -76,6 +76,7 @@ struct LifeBatch {
     // kChain steps from an even parity in one graph (single small cases)
     cudaGraphExec_t chain = nullptr;
     int chain_nodes = 0;
+    bool no_chain = false;   // its capture failed
     long long launched = 0;  // kernel nodes launched so far
     std::vector<int> t_base, cur_base, rec_gen;
     std::vector<int> ring_end;  // step tables are valid for t < ring_end[k]
@@ -94,6 +95,7 @@ static void drop_graphs(LifeBatch* b) {
         }
     if (b->chain) cudaGraphExecDestroy(b->chain);
     b->chain = nullptr;
+    b->no_chain = false;
 }
 
 static void free_batch(LifeBatch* b) {
@@ -203,6 +205,20 @@ static int refill_steps(LifeBatch* b, int n, int ahead = 1) {
     return LIFE_OK;
 }
 
+// What steps change in the host's view of a case. A capture goes through the
+// steps without running any, so the view is put back after it, also after one
+// that failed halfway through a step.
+struct HostView {
+    int t, cur;
+    IbmScratch W;
+};
+static HostView host_view(const LifeCase* c) { return {c->t, c->cur, c->W}; }
+static void set_host_view(LifeCase* c, const HostView& v) {
+    c->t = v.t;
+    c->cur = v.cur;
+    c->W = v.W;
+}
+
 // Captures batch steps from the cases' current state and advances the host
 // view of every case by them (t, buffer parity, IBM scratch parity).
 // Per case, the boundary perimeter runs on the case's side stream beside the
@@ -304,17 +320,6 @@ static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* o
     return LIFE_OK;
 }
 
-// Undoes what captures did to the host view since the graphs' base state.
-static void rewind_host_view(LifeBatch* b) {
-    for (size_t k = 0; k < b->cases.size(); k++) {
-        LifeCase* c = b->cases[k];
-        const int adv = c->t - b->t_base[k];
-        c->t = b->t_base[k];
-        c->cur = b->cur_base[k];
-        if (adv & 1) swap_site_lists(c->W);
-    }
-}
-
 static int build_graphs(LifeBatch* b) {
     drop_graphs(b);
     for (LifeCase* c : b->cases) CK(cudaStreamSynchronize(c->stream));
@@ -329,9 +334,11 @@ static int build_graphs(LifeBatch* b) {
         b->cur_base[k] = b->cases[k]->cur;
         b->rec_gen[k] = b->cases[k]->rec_gen;
     }
+    std::vector<HostView> now;
+    for (const LifeCase* c : b->cases) now.push_back(host_view(c));
     int rc = LIFE_OK;
     for (int p = 0; p < 2 && rc == LIFE_OK; p++) rc = capture_steps(b, p, 1, &b->exec[p], &b->kernel_nodes[p]);
-    rewind_host_view(b);
+    for (int k = 0; k < n; k++) set_host_view(b->cases[k], now[k]);
     if (rc != LIFE_OK) drop_graphs(b);
     return rc;
 }
@@ -380,22 +387,26 @@ static int check_status(LifeBatch* b) {
 // 23.1 with two.
 // Larger lattices and flexible bodies step in 0.07 ms and more, and a batch of
 // several cases in about 1 ms. The chain is captured when a run is long enough
-// to repay it.
+// to repay it; where it cannot be captured the steps go one by one.
 static int chain_steps(LifeBatch* b, int left, int ph) {
-    if (b->cases.size() != 1 || left < kChain || ph != 0) return 1;
-    const LifeCase* c = b->cases[0];
+    if (b->cases.size() != 1 || left < kChain || ph != 0 || b->no_chain) return 1;
+    LifeCase* c = b->cases[0];
     if (c->obj.hasFlex || (long long)c->Nx * c->Ny >= (1LL << 22)) return 1;
     if (!b->chain) {
         if (left < 2 * kChain) return 1;
-        // captured from the base state, as the step graphs were
-        LifeCase* m = b->cases[0];
-        const int t = m->t, cur = m->cur;
-        m->t = b->t_base[0];
-        m->cur = b->cur_base[0];
+        // captured from the base state, as the step graphs were (the site lists
+        // are those of the base state: phase 0)
+        const HostView now = host_view(c);
+        c->t = b->t_base[0];
+        c->cur = b->cur_base[0];
         const int rc = capture_steps(b, 0, kChain, &b->chain, &b->chain_nodes);
-        m->t = t;
-        m->cur = cur;
-        if (rc != LIFE_OK) return -rc;
+        set_host_view(c, now);
+        if (rc != LIFE_OK) {
+            cudaGetLastError();
+            b->chain = nullptr;
+            b->no_chain = true;
+            return 1;
+        }
     }
     return kChain;
 }
@@ -414,7 +425,6 @@ static int run_batch(LifeBatch* b, int nsteps, cudaEvent_t start, cudaEvent_t st
     for (int s = 0; s < nsteps;) {
         const int ph = graph_phase(b);
         const int m = chain_steps(b, nsteps - s, ph);
-        if (m < 0) return -m;
         if (int rc = refill_steps(b, std::min(nsteps - s, kStepChunk), m)) return rc;
         CK(cudaGraphLaunch(m > 1 ? b->chain : b->exec[ph], b->stream));
         b->launched += m > 1 ? b->chain_nodes : b->kernel_nodes[ph];
