@@ -49,6 +49,10 @@ __global__ void k_batch_advance(int* __restrict__ tnow, int n, int steps) {
     if (k < n) tnow[k] += steps;
 }
 
+// The first node of a step graph of one case whose boundary sites run beside the
+// interior (see capture_steps).
+__global__ void k_graph_root() {}
+
 // Steps per graph launch of a small single case (see chain_steps).
 constexpr int kChain = 16;
 
@@ -230,6 +234,14 @@ static void set_host_view(LifeCase* c, const HostView& v) {
 // made a step of the 1000 x 400 FP32 cylinder 35.3 us, beside them 25.2. Where a
 // kernel forms the convective outlet's speed term, it comes before whatever reads
 // it (LatDev::outlet_form).
+// A graph of one case whose step forks starts from one empty kernel: started from
+// two nodes, the boundary sites and the interior, a graph of one step takes longer
+// and the boundary sites start behind the interior's blocks (runs of eight steps,
+// 4000 x 400 FP32 channel: 38.7 us a step, 26.9 with the root; FP64 1501 x 703:
+// 142 and 129; with 16 steps a graph 22.3 and 20.7). A step that is one launch does
+// without (it would be 1.5 us longer), so does one with a subiteration loop (which
+// the rest waits for anyway), and batches, where the root gained up to 6 us at 3
+// cases and lost up to 7 at 24.
 static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* out, int* kernels) {
     cudaStream_t bs = b->stream;
     const int n = (int)b->cases.size();
@@ -238,7 +250,11 @@ static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* o
     cudaError_t e = cudaSuccess;
     for (int s = 0; s < steps && e == cudaSuccess && rc == LIFE_OK; s++) {
         const int phase = (phase0 + s) & 1;
-        e = cudaEventRecord(b->ev_fork, bs);
+        if (s == 0 && n == 1 && !b->cases[0]->obj.hasFlex && (!fused_step(b) || b->cases[0]->obj.hasIBM)) {
+            k_graph_root<<<1, 1, 0, bs>>>();
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(b->ev_fork, bs);
         for (int k = 0; k < n && e == cudaSuccess && rc == LIFE_OK; k++) {
             LifeCase* c = b->cases[k];
             c->t_dev = b->d_tnow + k;
