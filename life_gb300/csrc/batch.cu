@@ -30,6 +30,7 @@
 #include "../../include/life_gb300.h"
 #include "lbm_kernels.h"
 #include "life_internal.h"
+#include "wall_plan.h"
 
 using namespace life;
 
@@ -245,6 +246,12 @@ static void set_host_view(LifeCase* c, const HostView& v) {
 static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* out, int* kernels) {
     cudaStream_t bs = b->stream;
     const int n = (int)b->cases.size();
+    long long sites = 0;
+    int slow = 0;
+    for (const LifeCase* c : b->cases) {
+        sites += (long long)c->Nx * c->Ny;
+        slow += slow_wall_sites(lattice_view(c, c->t + 1));
+    }
     CK(cudaStreamBeginCapture(bs, cudaStreamCaptureModeThreadLocal));
     int rc = LIFE_OK;
     cudaError_t e = cudaSuccess;
@@ -261,7 +268,8 @@ static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* o
             c->t_off = 1 + s;
             const int tt = c->t + 1;
             LatDev L = lattice_view(c, tt);
-            L.crowded = n > 1;
+            L.others_sites = sites - (long long)c->Nx * c->Ny;
+            L.others_slow = slow - slow_wall_sites(L);
             e = cudaStreamWaitEvent(c->side, b->ev_fork, 0);
             const bool fused = fused_step(b);  // perimeter inside the interior launch
             if (L.convective && L.outlet_form == kOutletKernel) {

@@ -5,12 +5,9 @@
 // share formed once: about 200 FP64 instructions of the warp (BGK), 6 a site.
 // Corners, pressure and free-slip walls, which extrapolate from the fluid, and
 // cases with a force take nine lanes a site (lbm_lanes.cuh: 95 to 130 FP64
-// instructions for three sites, 38 a site, a shorter chain). A case alone with
-// few boundary sites takes nine lanes for all of them: 14.2 us a step against
-// 15.6 (256 x 256, 1020 sites); at 2800 sites the two were even (35.6 and 35.8,
-// measured where a body's spread waited for the walls),
-// at 4400 the threads are ahead (17.2 against 19.4 us, 1501 x 703 FP32), and 64
-// lattices in a batch step in 573 us against 976. (Products from the integer
+// instructions for three sites, 38 a site, a shorter chain), and with many such
+// sites one thread a site, every direction written out (boundary_site: 700 to 900
+// for 32 sites). wall_plan.h has the lines between them. (Products from the integer
 // units, as in the interior, make the warp's chain longer: 15.6 -> 18.4 us at
 // 256 x 256, no gain in a batch.) A thread whose values leave the range that
 // moment_sums_int takes runs the general code of boundary_site(). All of them
@@ -18,8 +15,11 @@
 // collide().
 #pragma once
 #include "lbm_lanes.cuh"
+#include "wall_plan.h"
 
 namespace life {
+
+static_assert(kLaneSites == 3, "wall_plan.h counts three sites a warp");
 
 // div_rn_recip for a zero numerator or operands within its window.
 __device__ __forceinline__ double quotient_in_range(double a, double b, double y) {
@@ -136,36 +136,6 @@ __device__ __forceinline__ bool wall_site(const typename S::T* __restrict__ A, t
     return true;
 }
 
-// Which warps take what: first the sites for nine lanes (the four corners, then
-// the edges of `lanes`: bottom, top, left, right as bits 0..3), three a warp,
-// then the other edges, 32 sites a warp. Edges do not hold the corners.
-constexpr int kFewWallSites = 2048;
-struct WallPlan {
-    int lane_sites, lane_warps, lanes, straight;
-    int warps;
-};
-__host__ __device__ inline int edge_sites(const LatDev& L, int e) { return (e < 2 ? L.Nx : L.Ny) - 2; }
-inline WallPlan wall_plan(const LatDev& L) {
-    const bool forced = L.womersley || L.Fx0 != 0.0 || L.Fy0 != 0.0 || L.site_force;
-    const bool few = !L.crowded && 2 * (L.Nx + L.Ny) < kFewWallSites;
-    WallPlan p{};
-    p.lane_sites = 4;
-    for (int e = 0; e < 4; e++) {
-        const int type = L.wall[(e + 2) & 3];  // (walls: left, right, bottom, top)
-        if (type == LIFE_FLUID) continue;
-        const bool formed = type != LIFE_CONVECTIVE || L.outlet_form == kOutletSites;
-        if (!few && !forced && formed && (type == LIFE_WALL || type == LIFE_VELOCITY || type == LIFE_CONVECTIVE)) {
-            p.straight |= 1 << e;
-            p.warps += (edge_sites(L, e) + 31) / 32;
-        } else {
-            p.lanes |= 1 << e;
-            p.lane_sites += edge_sites(L, e);
-        }
-    }
-    p.lane_warps = (p.lane_sites + kLaneSites - 1) / kLaneSites;
-    p.warps += p.lane_warps;
-    return p;
-}
 __device__ __forceinline__ void edge_ij(const LatDev& L, int e, int q, int& i, int& j) {
     if (e < 2) {
         i = 1 + q;
@@ -208,7 +178,7 @@ __device__ __forceinline__ void walls_warp(const typename S::T* __restrict__ A, 
             q -= padded;
             continue;
         }
-        const int type = L.wall[(e + 2) & 3];
+        const int type = edge_type(L, e);
         int i, j;
         edge_ij(L, e, q, i, j);
         double dU0 = 0.0, dU1 = 0.0;
@@ -234,11 +204,38 @@ __global__ void __launch_bounds__(32) k_perimeter(const typename S::T* __restric
     walls_warp<CM, S>(A, B, L, step_t(L, t), plan, blockIdx.x);
 }
 
+// One thread a site, every direction written out, around the whole perimeter
+// (perimeter_ij's order). The outlet's mean is formed by the warps that hold outlet
+// sites.
+template <bool CM, class S>
+__global__ void __launch_bounds__(32) k_perimeter_general(const typename S::T* __restrict__ A,
+                                                          typename S::T* __restrict__ B, LatDev L, int t) {
+    int i = 0, j = 0;
+    const bool on = perimeter_ij(L, 32 * (int)blockIdx.x + (int)threadIdx.x, i, j);
+    const int type = on ? site_type(L, i, j) : LIFE_FLUID;
+    const bool form = L.convective && L.outlet_form == kOutletSites;
+    double dU[2] = {0.0, 0.0};
+    if (form && __any_sync(kAllLanes, type == LIFE_CONVECTIVE)) {
+        const double uOut = lanes_outlet_mean<S::prec == LIFE_PREC_F64>(L);
+        if (type == LIFE_CONVECTIVE) {
+            outlet_term(L, uOut, j, dU[0], dU[1]);
+            L.delU[j * 2 + 0] = dU[0];
+            L.delU[j * 2 + 1] = dU[1];
+        }
+    }
+    if (type != LIFE_FLUID) boundary_site<CM, S>(A, B, L, step_t(L, t), i, j, form ? dU : nullptr);
+}
+
 template <class S>
 static void launch_walls(const void* A, void* B, const LatDev& L, int t, cudaStream_t s) {
     const WallPlan plan = wall_plan(L);
     const typename S::T* a = (const typename S::T*)A;
     typename S::T* b = (typename S::T*)B;
+    if (plan.general) {
+        if (L.cm) k_perimeter_general<true, S><<<plan.warps, 32, 0, s>>>(a, b, L, t);
+        else k_perimeter_general<false, S><<<plan.warps, 32, 0, s>>>(a, b, L, t);
+        return;
+    }
     if (L.cm) k_perimeter<true, S><<<plan.warps, 32, 0, s>>>(a, b, L, t, plan);
     else k_perimeter<false, S><<<plan.warps, 32, 0, s>>>(a, b, L, t, plan);
 }

@@ -53,7 +53,10 @@ struct LatDev {
     const double* outlet_f_prev;// [Ny][3] post-BC f[2,6,8] at Nx-1 of the previous step
     double* outlet_f_next;      // [Ny][3] written by the current step
     double* delU;               // [Ny][2] convective speed term of the current step
-    int crowded;                // stepped together with other cases (a batch)
+    // the other cases of a batch that are stepped together with this one: their
+    // lattice sites, and their boundary sites that nine lanes would take
+    long long others_sites;
+    int others_slow;
     int outlet_form;            // who forms delU before the outlet column is stepped (kOutlet*)
     const double* force_ibm;    // [2][S] dense IBM force of the current step, or null
     // Inside a replayed graph the step index comes from device memory: when
