@@ -50,9 +50,8 @@ __global__ void k_batch_advance(int* __restrict__ tnow, int n, int steps) {
     if (k < n) tnow[k] += steps;
 }
 
-// The first node of a step graph of one case whose boundary sites run beside the
-// interior (see capture_steps).
-__global__ void k_graph_root() {}
+// An empty kernel: a node that others of a step graph wait for (see capture_steps).
+__global__ void k_graph_node() {}
 
 // Steps per graph launch of a small single case (see chain_steps).
 constexpr int kChain = 16;
@@ -241,14 +240,23 @@ static void set_host_view(LifeCase* c, const HostView& v) {
 // 4000 x 400 FP32 channel: 38.7 us a step, 26.9 with the root; FP64 1501 x 703:
 // 142 and 129; with 16 steps a graph 22.3 and 20.7). A step that is one launch does
 // without (it would be 1.5 us longer), so does one with a subiteration loop (which
-// the rest waits for anyway), and batches, where the root gained up to 6 us at 3
-// cases and lost up to 7 at 24.
+// the rest waits for anyway).
+// In a batch of reduced precision the interior also waits for a second empty
+// kernel behind the root: its persistent blocks fill the chip until the step ends,
+// and boundary sites that start after them run after them (24 FP32 channels 70.5 ->
+// 57.8 us a step, free-slip 94.4 -> 64.9, with central moments 101.7 -> 65.5; 48
+// channels 108.5 -> 104.6). With FP64 storage the two share the FP64 unit all the
+// same (3 channels 29.2 -> 25.1 us, 6 under gravity with central moments 212 ->
+// 219), and with subiteration loops the step waits for those (the 64 cases of an
+// ensemble 1140 -> 1164).
 static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* out, int* kernels) {
     cudaStream_t bs = b->stream;
     const int n = (int)b->cases.size();
+    bool interior_behind = n > 1 && b->prec != LIFE_PREC_F64;
     long long sites = 0;
     int slow = 0;
     for (const LifeCase* c : b->cases) {
+        interior_behind = interior_behind && !c->obj.hasFlex;
         sites += (long long)c->Nx * c->Ny;
         slow += slow_wall_sites(lattice_view(c, c->t + 1));
     }
@@ -257,8 +265,9 @@ static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* o
     cudaError_t e = cudaSuccess;
     for (int s = 0; s < steps && e == cudaSuccess && rc == LIFE_OK; s++) {
         const int phase = (phase0 + s) & 1;
-        if (s == 0 && n == 1 && !b->cases[0]->obj.hasFlex && (!fused_step(b) || b->cases[0]->obj.hasIBM)) {
-            k_graph_root<<<1, 1, 0, bs>>>();
+        if (s == 0 && (n > 1 ? interior_behind
+                             : !b->cases[0]->obj.hasFlex && (!fused_step(b) || b->cases[0]->obj.hasIBM))) {
+            k_graph_node<<<1, 1, 0, bs>>>();
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaEventRecord(b->ev_fork, bs);
@@ -284,6 +293,10 @@ static int capture_steps(LifeBatch* b, int phase0, int steps, cudaGraphExec_t* o
                 if (e == cudaSuccess) rc = ibm_forces(c, tt, c->P[c->cur], c->aux);
                 if (e == cudaSuccess && rc == LIFE_OK) e = cudaEventRecord(c->ev_aux, c->aux);
             }
+        }
+        if (e == cudaSuccess && rc == LIFE_OK && interior_behind) {
+            k_graph_node<<<1, 1, 0, bs>>>();
+            e = cudaGetLastError();
         }
         if (e == cudaSuccess && rc == LIFE_OK) e = launch_batch_interior(b, phase, bs, nullptr, nullptr, 1 + s);
         if (e == cudaSuccess) e = cudaEventRecord(b->ev_int, bs);

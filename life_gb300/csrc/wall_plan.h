@@ -52,8 +52,10 @@ constexpr int kFewWallSites = 2048;
 // (free-slip channels 64 high, us a step, lanes and threads: FP32 BGK 2000 wide
 // 19.8 and 22.9, 3000 25.1 and 23.4, 8000 59.8 and 27.3; central moments 2000 26.9
 // and 29.1, 3000 35.5 and 30.5, 8000 83.7 and 37.3). In a batch the cases' walls
-// fill the chip together.
-constexpr int kManySlowBgk = 6400, kManySlowCm = 4800, kManySlowBatch = 10000;
+// fill the chip together (free-slip FP32 channels: 6 of them, 2856 sites, 27.5 and
+// 31.6 us, 12, 6864 sites, 42.8 and 33.9; pressure outlets 12, 1640 sites, 28.5 and
+// 33.0, 24, 4330 sites, 69.8 and 63.1).
+constexpr int kManySlowBgk = 6400, kManySlowCm = 4800, kManySlowBatch = 4000;
 // FP64 storage: the interior needs the same unit. Under a force, whose interior is
 // all FP64, the threads are ahead once the lattice takes longer than their chain
 // (1000 x 64 under gravity 36.1 and 33.0 us, 500 x 64 20.4 and 21.6; central moments

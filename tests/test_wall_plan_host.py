@@ -79,7 +79,7 @@ PERIODIC = (FLUID, FLUID, WALL, WALL)
     (499, 100, PERIODIC, dict(force=1, prec=F64), "lanes"), (500, 100, PERIODIC, dict(force=1, prec=F64), "general"),
     (299, 100, PERIODIC, dict(force=1, prec=F64, cm=1), "lanes"),
     (300, 100, PERIODIC, dict(force=1, prec=F64, cm=1), "general"),
-    (502, 100, SLIP, dict(others=(10 ** 6, 8999)), "both"), (502, 100, SLIP, dict(others=(10 ** 6, 9000)), "general"),
+    (502, 100, SLIP, dict(others=(10 ** 6, 2999)), "both"), (502, 100, SLIP, dict(others=(10 ** 6, 3000)), "general"),
     (502, 100, CHANNEL, dict(others=(10 ** 6, 10 ** 6)), "straight"),  # nothing slow of its own
 ])
 def test_form(driver, nx, ny, walls, kw, form):
