@@ -89,6 +89,25 @@ __global__ void k_init_fill(typename S::T* __restrict__ B, const InitRow<S>* __r
 // lie in an ordinary range takes its products from the integer units
 // (collide_bgk_int, collide_cm_int): the kernel is bound by the FP64 unit and
 // has issue slots to spare. Any other site runs the general code.
+//
+// A site that is only too fast (1/8 a component and more) has its sums and
+// quotients already: with KEEP it takes them along and the general code begins at
+// the collision. A batch of 24 channels at a velocity of 0.15 takes 404 us a step so,
+// 529 with the sums formed again, 498 with every product in FP64 (central moments
+// 1106, 1226 and 1195). Not for central moments in the kernel of one case: 1024 x 1024
+// sites at 0.15 take 639 us without (all in FP64 657), and ordinary sites would lose
+// 0.7 % to the call (1536 x 1536: 668.7 -> 673.4).
+template <bool CM>
+static __device__ __noinline__ void collide_site_general(const double* __restrict__ A, double* __restrict__ B,
+                                                         const LatDev& L, int i, int j, double rho, double ux, double uy) {
+    double f[9], fs[9];
+    gather<StoreF64>(A, L, i, j, f);
+    outlet_outputs(L, i, j, f, ux, uy);
+    collide<CM, true>(f, rho, ux, uy, 0.0, 0.0, L.omega, L.cs, fs);
+    const size_t s = (size_t)j * L.pitch + i;
+#pragma unroll
+    for (int v = 0; v < 9; v++) B[(size_t)v * L.S + s] = fs[v];
+}
 template <bool CM>
 static __device__ __noinline__ void interior_site_general(const double* __restrict__ A, double* __restrict__ B,
                                                           const LatDev& L, int i, int j) {
@@ -102,7 +121,7 @@ static __device__ __noinline__ void interior_site_general(const double* __restri
     for (int v = 0; v < 9; v++) B[(size_t)v * L.S + s] = fs[v];
 }
 
-template <bool CM, bool SITE>
+template <bool CM, bool SITE, bool KEEP>
 __device__ __forceinline__ void interior_site_f64(const double* __restrict__ A, double* __restrict__ B,
                                                   const LatDev& L, int t, int i, int j) {
     if (site_type(L, i, j) != LIFE_FLUID) return;
@@ -138,8 +157,9 @@ __device__ __forceinline__ void interior_site_f64(const double* __restrict__ A, 
     } else {
         // zero force at every step: the velocity without the force half-term
         // (the same value) and no forcing terms in the collision
-        bool ok = populations_in_range(f);
-        if (ok) {
+        const bool sums = populations_in_range(f);
+        bool ok = sums;
+        if (sums) {
             double mx, my;
             moment_sums_int(f, rho, mx, my);
             const double y = __drcp_rn(rho);
@@ -148,7 +168,8 @@ __device__ __forceinline__ void interior_site_f64(const double* __restrict__ A, 
             ok = site_range_ok(ux, uy, L.omega);
         }
         if (!ok) {
-            interior_site_general<CM>(A, B, L, i, j);
+            if (KEEP && sums) collide_site_general<CM>(A, B, L, i, j, rho, ux, uy);
+            else interior_site_general<CM>(A, B, L, i, j);
             return;
         }
         outlet_outputs(L, i, j, f, ux, uy);
@@ -168,7 +189,7 @@ __global__ void __launch_bounds__(128, 5) k_interior_f64(const double* __restric
                                                       int t) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
     if (i >= L.Nx) return;
-    interior_site_f64<CM, SITE>(A, B, L, step_t(L, t), i, j);
+    interior_site_f64<CM, SITE, !CM>(A, B, L, step_t(L, t), i, j);
 }
 
 // All cases of a batch in one persistent launch (see k_interior_batch_lowp).
@@ -188,11 +209,11 @@ __global__ void __launch_bounds__(256) k_interior_batch_f64(const BatchLatCase* 
         const int j1 = (ty + 1) * tile_h < L.Ny ? (ty + 1) * tile_h : L.Ny;
         for (int j = ty * tile_h; j < j1; j++) {
             if (L.site_force) {
-                if (L.cm) interior_site_f64<true, true>(A, B, L, t, i, j);
-                else interior_site_f64<false, true>(A, B, L, t, i, j);
+                if (L.cm) interior_site_f64<true, true, true>(A, B, L, t, i, j);
+                else interior_site_f64<false, true, true>(A, B, L, t, i, j);
             } else {
-                if (L.cm) interior_site_f64<true, false>(A, B, L, t, i, j);
-                else interior_site_f64<false, false>(A, B, L, t, i, j);
+                if (L.cm) interior_site_f64<true, false, true>(A, B, L, t, i, j);
+                else interior_site_f64<false, false, true>(A, B, L, t, i, j);
             }
         }
     }
