@@ -33,7 +33,7 @@ __device__ __forceinline__ void clear_force(const IbmScratch& W, const LatDev& L
     }
 }
 
-// List the support site (i, j), if no other entry has, and widen the body's
+// List the support site (i, j), if no other entry has, and widen its range's
 // support box by the marker's (once per marker: `first`).
 __device__ __forceinline__ void mark_site(const IbmScratch& W, const LatDev& L, int k, int i, int j, bool first,
                                           const int4& bb) {
@@ -41,7 +41,7 @@ __device__ __forceinline__ void mark_site(const IbmScratch& W, const LatDev& L, 
     const unsigned bit = 1u << (s & 31);
     if (!(atomicOr(&W.site_flag[s >> 5], bit) & bit)) W.sites[atomicAdd(W.nsites, 1)] = s;
     if (first) {
-        int4* box = W.body_box + W.box_of[k];
+        int4* box = W.range_box + W.range_of[k];
         atomicMin(&box->x, bb.x);
         atomicMax(&box->y, bb.y);
         atomicMin(&box->z, bb.z);
@@ -121,7 +121,7 @@ __global__ void k_ibm_mark(MarkerDev M, IbmScratch W, LatDev L) {
 }
 
 // One warp takes three listed sites, nine lanes each (lbm_lanes.cuh). The
-// lanes scan the bodies whose support box reaches one of the sites (in body
+// lanes scan the ranges of markers whose support box reaches one of the sites (in
 // order) 32 markers at a time for all three sites; a marker that reaches a
 // site leaves its contribution in shared memory, and one lane per site and
 // component adds the chunk's contributions in marker order. The few hundred
@@ -150,8 +150,8 @@ __global__ void __launch_bounds__(64) k_ibm_spread(const typename S::T* __restri
     // the next step's list starts empty
     if (blockIdx.x == 0 && scans) {
         if (lane == 0) *W.nsites_prev = 0;
-        for (int b = lane; b < W.nbodies; b += 32)
-            W.body_box_next[b] = make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff);
+        for (int b = lane; b < W.nranges; b += 32)
+            W.range_box_next[b] = make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff);
     }
     for (int q0 = kLaneSites * (int)blockIdx.x; q0 < nsites; q0 += kLaneSites * (int)gridDim.x) {
         // this lane's site; a missing one repeats the first and is not stored
@@ -175,17 +175,17 @@ __global__ void __launch_bounds__(64) k_ibm_spread(const typename S::T* __restri
             // lanes 0 and 1 of a site sum the x and the y force
             const int comp = g.v == 1 ? 1 : 0;
             double acc = 0.0;
-            for (int b0 = 0; b0 < W.nbodies; b0 += 32) {
+            for (int b0 = 0; b0 < W.nranges; b0 += 32) {
                 bool near = false;
-                if (b0 + lane < W.nbodies) {
-                    const int4 box = W.body_box[b0 + lane];
+                if (b0 + lane < W.nranges) {
+                    const int4 box = W.range_box[b0 + lane];
                     near = box_has(box, is[0], js[0]) || box_has(box, is[1], js[1]) || box_has(box, is[2], js[2]);
                 }
-                unsigned bodies = __ballot_sync(kAllLanes, near);
-                while (bodies) {
-                    const int b = b0 + __ffs(bodies) - 1;
-                    bodies &= bodies - 1;
-                    const int kbeg = W.body_start[b], kend = W.body_start[b + 1];
+                unsigned ranges = __ballot_sync(kAllLanes, near);
+                while (ranges) {
+                    const int b = b0 + __ffs(ranges) - 1;
+                    ranges &= ranges - 1;
+                    const int kbeg = W.range_start[b], kend = W.range_start[b + 1];
                     // the support box of the next chunk's marker comes while this
                     // chunk's is looked at, and what a hit needs with its entries
                     int4 next = kbeg + lane < kend ? M.bbox[kbeg + lane] : make_int4(0, -1, 0, -1);

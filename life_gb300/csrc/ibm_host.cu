@@ -125,9 +125,9 @@ int life::reset_site_lists(LifeCase* c) {
     CK(cudaMemsetAsync(W.nsites, 0, sizeof(int), s));
     CK(cudaMemsetAsync(W.nsites_prev, 0, sizeof(int), s));
     CK(cudaMemsetAsync(W.site_flag, 0, sizeof(unsigned) * flag_words(c), s));
-    const std::vector<int4> empty((size_t)W.nbodies, make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff));
-    CK(cudaMemcpyAsync(W.body_box, empty.data(), sizeof(int4) * empty.size(), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(W.body_box_next, empty.data(), sizeof(int4) * empty.size(), cudaMemcpyHostToDevice, s));
+    const std::vector<int4> empty((size_t)W.nranges, make_int4(0x7fffffff, -0x7fffffff, 0x7fffffff, -0x7fffffff));
+    CK(cudaMemcpyAsync(W.range_box, empty.data(), sizeof(int4) * empty.size(), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(W.range_box_next, empty.data(), sizeof(int4) * empty.size(), cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));
     return LIFE_OK;
 }
@@ -148,31 +148,24 @@ int upload_markers(LifeCase* c) {
         (rc = alloc_t(c, &W.sites_prev, (size_t)9 * n + 1)) || (rc = alloc_t(c, &W.nsites, 1)) ||
         (rc = alloc_t(c, &W.nsites_prev, 1)) || (rc = alloc_t(c, &W.site_flag, flag_words(c))))
         return rc;
-    // bodies as contiguous marker ranges (markers are stored body by body);
-    // one range over all markers if that ever does not hold
+    // ranges of markers whose support boxes the spread looks at: one per body
+    // (markers are stored body by body), a long body in several
     std::vector<int> start(1, 0);
-    bool contiguous = true;
-    for (int k = 1; k < n; k++) {
-        const int b0 = c->obj.m[k - 1].body, b1 = c->obj.m[k].body;
-        if (b1 != b0) {
-            if (b1 < b0) contiguous = false;
-            start.push_back(k);
-        }
-    }
+    for (int k = 1; k < n; k++)
+        if (c->obj.m[k].body != c->obj.m[k - 1].body || k - start.back() == kRangeMarkers) start.push_back(k);
     start.push_back(n);
-    if (!contiguous || n == 0) start = {0, n};
-    W.nbodies = (int)start.size() - 1;
-    std::vector<int> box_of((size_t)std::max(n, 1), 0);
-    for (int r = 0; r < W.nbodies; r++)
-        for (int k = start[r]; k < start[r + 1]; k++) box_of[k] = r;
-    int *d_start = nullptr, *d_box_of = nullptr;
-    if ((rc = alloc_t(c, &d_start, start.size())) || (rc = alloc_t(c, &d_box_of, box_of.size())) ||
-        (rc = alloc_t(c, &W.body_box, (size_t)W.nbodies)) || (rc = alloc_t(c, &W.body_box_next, (size_t)W.nbodies)))
+    W.nranges = (int)start.size() - 1;
+    std::vector<int> range_of((size_t)std::max(n, 1), 0);
+    for (int r = 0; r < W.nranges; r++)
+        for (int k = start[r]; k < start[r + 1]; k++) range_of[k] = r;
+    int *d_start = nullptr, *d_range_of = nullptr;
+    if ((rc = alloc_t(c, &d_start, start.size())) || (rc = alloc_t(c, &d_range_of, range_of.size())) ||
+        (rc = alloc_t(c, &W.range_box, (size_t)W.nranges)) || (rc = alloc_t(c, &W.range_box_next, (size_t)W.nranges)))
         return rc;
-    W.body_start = d_start;
-    W.box_of = d_box_of;
+    W.range_start = d_start;
+    W.range_of = d_range_of;
     CK(cudaMemcpyAsync(d_start, start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(d_box_of, box_of.data(), sizeof(int) * box_of.size(), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(d_range_of, range_of.data(), sizeof(int) * range_of.size(), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     if ((rc = reset_site_lists(c))) return rc;
     if ((rc = alloc_t(c, &c->d_fsi, 1)) || (rc = alloc_t(c, &c->d_status, 4))) return rc;
