@@ -731,9 +731,13 @@ __global__ void __launch_bounds__(256, TmaTile<S>::CTAS) k_step_tma(const __grid
     t = step_t(L, t);
     if ((int)blockIdx.x < pb) {
         // boundary-condition sites; an edge site of a periodic wall is an
-        // interior site with wrapped neighbours (each call skips the other kind)
+        // interior site with wrapped neighbours (each call skips the other kind).
+        // Inlined: in a function of its own it reads L through its address, by
+        // loads that wait behind the tiles' (FP32 central moments, two sites a
+        // thread: 2048 x 2048 cavity 79.1 -> 67.3 us a step, free-slip channel 114 ->
+        // 87; FP16 BGK 2048 x 2048 cavity 53.4 -> 45.0; 4096 x 4096 unchanged).
         const int q = blockIdx.x * blockDim.x + threadIdx.x;
-        perimeter_site_call<CM, S>(A, B, L, t, q);
+        perimeter_site<CM, S>(A, B, L, t, q);
         int i, j;
         if (perimeter_ij(L, q, i, j)) interior_site_lowp<CM, S, false>(A, B, L, t, i, j);
         return;
