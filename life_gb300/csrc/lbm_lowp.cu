@@ -53,8 +53,8 @@ namespace life {
 // last place on ~1 site in 10^6 per step), which the one-site path, compiled
 // without contraction, does not do. The collisions below are therefore
 // written so that no packed product feeds an addition, unless it is exact (by
-// a power of two) and fusing it changes nothing; mul_alone forms the two
-// products of the central moments that do, one lane at a time.
+// a power of two) and fusing it changes nothing; mul_alone forms the products of
+// the central moments that do (the squares, the velocity), one lane at a time.
 struct V2 {
     unsigned long long b;  // lane x in the low 32 bits, lane y in the high 32 bits
     __device__ __forceinline__ float x() const {
@@ -224,8 +224,8 @@ __device__ __forceinline__ void collide_dev32(const T g[9], const T r[9], T dr, 
         // exact, so every population is the one of the plain form. Packed for
         // two sites that is about 160 operations: 68.1 us, and with a force
         // 94.2 -> 79.4 us (3000 x 2200; FP32 98.8 -> 86.0 us).
-        // The only inexact products that feed additions are the two squares:
-        // mul_alone keeps them apart.
+        // The only inexact products that feed additions are the two squares and the
+        // velocity itself: mul_alone keeps them apart, here and in tma_pair.
         const T X2 = mul_alone(ux, ux), Y2 = mul_alone(uy, uy), XY = ux * uy;
         const T XmY = X2 - Y2, nux = (-1.0f) * ux, nuy = (-1.0f) * uy;
         const T k4 = om1 * fmaf(XmY, rho, fmaf(2.0f * uy, my, fmaf(2.0f * nux, mx, dxxyy)));
@@ -613,7 +613,8 @@ __device__ __forceinline__ void tma_pair(const unsigned char* stage, typename S:
     const V2 y0 = v2(rcp_approx(rho.x()), rcp_approx(rho.y()));
     const V2 inv = fmaf(y0, fmaf((-1.0f) - dr, y0, 1.0f), y0);
     const V2 px = FORCED ? fmaf(0.5f, Fxd, mx) : mx, py = FORCED ? fmaf(0.5f, Fyd, my) : my;
-    const V2 ux = px * inv, uy = py * inv;
+    // (the central moments add to the velocity, BGK does not)
+    const V2 ux = CM ? mul_alone(px, inv) : px * inv, uy = CM ? mul_alone(py, inv) : py * inv;
     V2 gs[9];
     collide_dev32<CM, FORCED, S::SCALED && !CM>(g, r, dr, rho, mx, my, ux, uy, px, py, inv, Gxd, Gyd, L.omega_f, gs);
     T* out = B + (size_t)j * L.pitch + i;
