@@ -457,12 +457,12 @@ __device__ __forceinline__ void regularised(double f[9], int type, int nx, int n
     }
 }
 
-constexpr int kOutletThreads = 256;  // of k_outlet_f64
+constexpr int kOutletThreads = 256;  // of k_outlet_lowp
 
-// The mean outlet speed of k_outlet_f64, formed by one warp with the same
-// additions in the same order: sequential over j for FP64 storage (32 values
-// loaded at a time), for the others the strided partial sums of its threads,
-// each warp's tree, and the warp sums in order.
+// The mean outlet speed, formed by one warp: sequential over j for FP64 storage, as
+// the reference's sum (32 values loaded at a time); for the others with the
+// additions of k_outlet_lowp in their order, the strided partial sums of its
+// threads, each warp's tree, and the warp sums in order.
 template <bool F64>
 __device__ __forceinline__ double lanes_outlet_mean(const LatDev& L) {
     const int lane = (int)threadIdx.x & 31, Ny = L.Ny;

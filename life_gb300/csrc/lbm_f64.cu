@@ -9,9 +9,9 @@
 //                   populations per site)
 //   k_perimeter     the same for boundary-condition sites, with the
 //                   regularised / convective conditions applied
-//   k_outlet_f64    convective outlet speed (sequential mean, as the reference;
-//                   a fixed-order tree sum for the reduced-precision forms), for
-//                   the one-launch step kernels; other steps form it in place
+//   k_outlet_lowp   convective outlet speed (a fixed-order tree sum) before the
+//                   one-launch steps of the reduced-precision forms; other steps
+//                   form it in place
 //   k_state         collision from an explicit state (restart read)
 //   k_export        reference-layout fields of the current step
 //   k_maxvel        max |u| and NaN scan
@@ -219,47 +219,27 @@ __global__ void __launch_bounds__(256) k_interior_batch_f64(const BatchLatCase* 
     }
 }
 
-// GridClass::convectiveSpeed (src/Grid.cpp:477-495): the mean outlet speed is
-// a sequential sum over j, as in the reference.
-__global__ void __launch_bounds__(kOutletThreads) k_outlet_f64(LatDev L, double* __restrict__ delU) {
+// GridClass::convectiveSpeed (src/Grid.cpp:477-495) before a one-launch step of
+// the reduced-precision forms, whose state is not the reference's bits: the mean
+// outlet speed is a tree sum in a fixed order (strided per thread, then the warps,
+// then the warp sums in order), the same on every run; a chain of ~15 dependent
+// FP64 additions instead of Ny. (Other steps form it in place, lanes_outlet_mean.)
+__global__ void __launch_bounds__(kOutletThreads) k_outlet_lowp(LatDev L, double* __restrict__ delU) {
+    __shared__ double wsum[kOutletThreads / 32];
     __shared__ double uOut_s;
-    __shared__ double col[1024];
     const int Ny = L.Ny;
     const double* u1 = L.outlet_u_prev + (size_t)2 * Ny * 2;  // column Nx-1
     const double* u2 = L.outlet_u_prev + (size_t)1 * Ny * 2;  // column Nx-2
     const double* u3 = L.outlet_u_prev;                       // column Nx-3
-    if (L.prec != LIFE_PREC_F64) {
-        // Reduced-precision forms (whose state is not the reference's bits):
-        // a tree sum in a fixed order (strided per thread, then the warps,
-        // then the warp sums in order), the same on every run; a chain of
-        // ~15 dependent FP64 additions instead of Ny.
-        __shared__ double wsum[32];
-        double part = 0.0;
-        for (int j = threadIdx.x; j < Ny; j += blockDim.x) part += u1[j * 2];
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-        if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = part;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0.0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) a += wsum[w];
-            uOut_s = a / (double)Ny;
-        }
-    } else {
-        // All threads stage the outlet column through shared memory; one
-        // thread then adds it up in j order, as the reference does.
-        double acc = 0.0;
-        for (int j0 = 0; j0 < Ny; j0 += 1024) {
-            const int m = Ny - j0 < 1024 ? Ny - j0 : 1024;
-            __syncthreads();
-            for (int j = threadIdx.x; j < m; j += blockDim.x) col[j] = u1[(j0 + j) * 2];
-            __syncthreads();
-            if (threadIdx.x == 0)
-                for (int j = 0; j < m; j++) acc += col[j];
-        }
-        if (threadIdx.x == 0) {
-            acc /= (double)Ny;
-            uOut_s = acc;
-        }
+    double part = 0.0;
+    for (int j = threadIdx.x; j < Ny; j += blockDim.x) part += u1[j * 2];
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
+    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = part;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) a += wsum[w];
+        uOut_s = a / (double)Ny;
     }
     __syncthreads();
     const double uOut = uOut_s;
@@ -585,7 +565,8 @@ cudaError_t launch_perimeter(const void* A, void* B, const LatDev& L, int t, cud
 }
 
 cudaError_t launch_outlet(const LatDev& L, double* delU, cudaStream_t s) {
-    k_outlet_f64<<<1, kOutletThreads, 0, s>>>(L, delU);
+    if (L.prec == LIFE_PREC_F64) return cudaErrorInvalidValue;  // (its mean is sequential, formed in place)
+    k_outlet_lowp<<<1, kOutletThreads, 0, s>>>(L, delU);
     return cudaGetLastError();
 }
 

@@ -85,7 +85,7 @@ struct LatDev {
     int* tile_ctr;
 };
 
-// LatDev::outlet_form: a kernel before the step (k_outlet_f64), or the warps
+// LatDev::outlet_form: a kernel before the step (k_outlet_lowp), or the warps
 // that hold outlet sites (the perimeter's also store it).
 enum { kOutletKernel, kOutletSites };
 
