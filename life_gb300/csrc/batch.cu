@@ -83,7 +83,6 @@ struct LifeBatch {
     bool no_chain = false;   // its capture failed
     long long launched = 0;  // kernel nodes launched so far
     std::vector<int> t_base, cur_base, rec_gen;
-    std::vector<int> ring_end;  // step tables are valid for t < ring_end[k]
     std::string status_msg;
     int status_code = 0;
     bool owns_cases = true;
@@ -198,13 +197,11 @@ static cudaError_t launch_batch_interior(LifeBatch* b, int phase, cudaStream_t s
 // when they do not, they are refilled for the next `n` steps (at most
 // kStepChunk, at least `ahead`).
 static int refill_steps(LifeBatch* b, int n, int ahead = 1) {
-    for (size_t k = 0; k < b->cases.size(); k++) {
-        LifeCase* c = b->cases[k];
-        if (c->t + 2 + ahead <= b->ring_end[k]) continue;
+    for (LifeCase* c : b->cases) {
+        if (c->steps_t0 <= c->t && c->t + 2 + ahead <= c->steps_t0 + c->steps_n) continue;
         const int m = std::min(std::max(n, 1), kStepChunk) + 2;
         CK(cudaStreamSynchronize(b->stream));
         if (int rc = ensure_steps(c, c->t, m)) return rc;
-        b->ring_end[k] = c->t + m;
     }
     return LIFE_OK;
 }
@@ -517,7 +514,6 @@ int batch_wrap(const std::vector<LifeCase*>& cases, LifeBatch** out) {
         return rc;
     }
     b->cases = cases;
-    b->ring_end.assign(cases.size(), 0);
     *out = b;
     return LIFE_OK;
 }
@@ -534,7 +530,6 @@ static int self_batch(LifeCase* c) {
         return rc;
     }
     b->cases = {c};
-    b->ring_end.assign(1, 0);
     c->self_batch = b;
     return LIFE_OK;
 }
@@ -602,7 +597,6 @@ extern "C" int life_batch_create(const LifeCaseParams* params, const LifeBodyDes
         b->sites += (long long)c->Nx * c->Ny;
         off += n_bodies[k];
     }
-    b->ring_end.assign(n_cases, 2);
     *out = b;
     return LIFE_OK;
 }

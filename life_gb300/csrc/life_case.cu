@@ -178,6 +178,7 @@ int life::ensure_steps(LifeCase* c, int t0, int n) {
         CK(cudaMemcpyAsync(c->d_steps, h.data() + n1, sizeof(StepScalars) * (n - n1), cudaMemcpyHostToDevice,
                            c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    c->steps_t0 = t0;
     c->steps_n = n;
     return LIFE_OK;
 }

@@ -69,7 +69,7 @@ struct LifeCase {
     double* d_u_in = nullptr;
     double* d_rho_in = nullptr;
     life::StepScalars* d_steps = nullptr;
-    int steps_cap = 0, steps_n = 0;
+    int steps_cap = 0, steps_t0 = 0, steps_n = 0;  // the table holds steps_t0 <= t < steps_t0 + steps_n
     double* d_outlet_u[2] = {nullptr, nullptr};
     double* d_outlet_f[2] = {nullptr, nullptr};
     double* d_delU = nullptr;
