@@ -222,8 +222,9 @@ __device__ __forceinline__ void collide_dev32(const T g[9], const T r[9], T dr, 
         // transform share factors up to a sign or a power of two, so each is
         // formed once and its sign and power sit in a multiple of the moment:
         // exact, so every population is the one of the plain form. Packed for
-        // two sites that is about 160 operations: 68.1 us, and with a force
-        // 94.2 -> 79.4 us (3000 x 2200; FP32 98.8 -> 86.0 us).
+        // two sites that is about 160 operations: 68.1 us (62.2 since the boundary
+        // blocks beside it are inlined), and with a force 94.2 -> 79.4 us (3000 x
+        // 2200; FP32 98.8 -> 86.0 us).
         // The only inexact products that feed additions are the two squares and the
         // velocity itself: mul_alone keeps them apart, here and in tma_pair.
         const T X2 = mul_alone(ux, ux), Y2 = mul_alone(uy, uy), XY = ux * uy;
@@ -733,10 +734,10 @@ __global__ void __launch_bounds__(256, TmaTile<S>::CTAS) k_step_tma(const __grid
     if ((int)blockIdx.x < pb) {
         // boundary-condition sites; an edge site of a periodic wall is an
         // interior site with wrapped neighbours (each call skips the other kind).
-        // Inlined: in a function of its own it reads L through its address, by
-        // loads that wait behind the tiles' (FP32 central moments, two sites a
-        // thread: 2048 x 2048 cavity 79.1 -> 67.3 us a step, free-slip channel 114 ->
-        // 87; FP16 BGK 2048 x 2048 cavity 53.4 -> 45.0; 4096 x 4096 unchanged).
+        // Inlined: as a function of its own, which takes L by address, its chain
+        // is slower beside the tiles (FP32 central moments, two sites a thread:
+        // 2048 x 2048 cavity 79.1 -> 67.3 us a step, free-slip channel 114 -> 87;
+        // FP16 BGK 2048 x 2048 cavity 53.4 -> 45.0; 4096 x 4096 unchanged).
         const int q = blockIdx.x * blockDim.x + threadIdx.x;
         perimeter_site<CM, S>(A, B, L, t, q);
         int i, j;
@@ -813,8 +814,8 @@ int tma_timeouts() {
 // (k_step_tma) for both storage forms; the one-site kernel (k_step_lowp) is
 // kept for comparison. Measured at 4096^2: FP16 95.6-99.6k (one-site) against
 // 159k MLUPS (staged), FP32 85.8-86.3k against 90.2-90.9k; with central moments
-// and FP16 at 3001 x 2203 the staged form takes 68.1 us a step (76.6 with one
-// site a thread in the staged form).
+// and FP16 at 3001 x 2203 the staged form takes 62.2 us a step (76.6 with one
+// site a thread in the staged form and the boundary sites in a called function).
 // LIFE_STEP_KERNEL=site|tma overrides, for measurements and for the tests
 // that compare the two bit for bit.
 enum { STEP_SITE = 1, STEP_TMA = 3 };
