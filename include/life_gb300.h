@@ -340,7 +340,7 @@ typedef struct LifeServer LifeServer;
 typedef struct LifeServerConfig {
     size_t hbm_budget;         /* bytes the admitted requests may hold */
     int32_t max_active;        /* requests stepped together at most (0: no limit) */
-    int32_t steps_per_round;   /* steps per scheduling round (0: 200) */
+    int32_t steps_per_round;   /* steps per scheduling round (0: 200, fewer when a waiting request could join) */
 } LifeServerConfig;
 
 enum { LIFE_REQ_QUEUED = 0, LIFE_REQ_RUNNING = 1, LIFE_REQ_DONE = 2, LIFE_REQ_FAILED = 3 };
