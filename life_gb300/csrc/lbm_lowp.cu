@@ -727,7 +727,7 @@ __device__ __forceinline__ void tma_tiles_by_warp(const CUtensorMap& tm, typenam
 template <bool CM, class S>
 __global__ void __launch_bounds__(256, TmaTile<S>::CTAS) k_step_tma(const __grid_constant__ CUtensorMap tm,
                                                   const typename S::T* __restrict__ A, typename S::T* __restrict__ B,
-                                                  LatDev L, int t, int pb, int tiles_x, int ntiles) {
+                                                  LatDev L, int t, int pb, int pt, int tiles_x, int ntiles) {
     using TT = TmaTile<S>;
     using SH = TmaShape<S>;
     t = step_t(L, t);
@@ -738,7 +738,8 @@ __global__ void __launch_bounds__(256, TmaTile<S>::CTAS) k_step_tma(const __grid
         // is slower beside the tiles (FP32 central moments, two sites a thread:
         // 2048 x 2048 cavity 79.1 -> 67.3 us a step, free-slip channel 114 -> 87;
         // FP16 BGK 2048 x 2048 cavity 53.4 -> 45.0; 4096 x 4096 unchanged).
-        const int q = blockIdx.x * blockDim.x + threadIdx.x;
+        if ((int)threadIdx.x >= pt) return;
+        const int q = blockIdx.x * pt + threadIdx.x;
         perimeter_site<CM, S>(A, B, L, t, q);
         int i, j;
         if (perimeter_ij(L, q, i, j)) interior_site_lowp<CM, S, false>(A, B, L, t, i, j);
@@ -795,12 +796,20 @@ static cudaError_t launch_step_tma_t(const void* A, void* B, const LatDev& L, in
     CUtensorMap tm;
     if ((e = plane_tensor_map<S>(&tm, A, L)) != cudaSuccess) return e;
     const int n = 2 * L.Nx + 2 * (L.Ny - 2);
-    const int pb = (n + 255) / 256;
+    // Boundary sites a block: 256, or 128 where their chain is longer than the
+    // tiles' time (one warp a sub-partition has the FP64 unit to itself, but a
+    // block holds its place among the tiles' all the same). FP32 central moments,
+    // us a step with 256 and 128: 2048 x 2048 cavity 68.2 and 58.3, under gravity
+    // between walls 73.0 and 62.1, 2500 x 2000 67.2 and 67.8, 73.8 and 70.5; 3001 x
+    // 2203 82.6 and 85.1, 85.3 and 87.3, 4096 x 4096 189.0 and 192.6.
+    const bool long_chain = CM && !S::SCALED && (long long)L.Nx * L.Ny < 5500000;
+    const int pt = long_chain ? 128 : 256;
+    const int pb = (n + pt - 1) / pt;
     const int tiles_x = (L.Nx - 1 + TT::W - 1) / TT::W, tiles_y = (L.Ny - 2 + TT::H - 1) / TT::H;
     const int ntiles = tiles_x * tiles_y;
     const int persistent = std::min(ntiles, sms[dev] * per_sm[dev]);
     k_step_tma<CM, S><<<pb + std::max(persistent, 1), 256, SH::SMEM, s>>>(
-        tm, (const typename S::T*)A, (typename S::T*)B, L, t, pb, tiles_x, ntiles);
+        tm, (const typename S::T*)A, (typename S::T*)B, L, t, pb, pt, tiles_x, ntiles);
     return cudaGetLastError();
 }
 
